@@ -33,6 +33,11 @@ void launch_snap_copy(const Snap &dst, const Snap &src, int nv, int nl, int nr, 
     if (n) k_snap_copy<<<(n + 255) / 256, 256, 0, st>>>(dst, src, nv, nl, nr);
 }
 
+static int adj_grid(int n) {
+    const int t = fp64_threads(n, 128);
+    return (n + t - 1) / t;
+}
+
 __global__ void __launch_bounds__(128) k_adj_slots(Dev d, Snap s, AdjBufs a) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l < d.nl) adj::adj_link_slots(d, s, a, l);
@@ -64,18 +69,18 @@ __global__ void __launch_bounds__(128) k_adj_seed(Dev d, AdjBufs a) {
 }
 
 void launch_adj_slots(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st) {
-    if (d.nl) k_adj_slots<<<(d.nl + 127) / 128, 128, 0, st>>>(d, s, a);
+    if (d.nl) k_adj_slots<<<adj_grid(d.nl), fp64_threads(d.nl, 128), 0, st>>>(d, s, a);
 }
 void launch_adj_voxel_link(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st) {
-    if (d.nv) k_adj_voxel<<<(d.nv + 127) / 128, 128, 0, st>>>(d, s, a);
-    if (d.nl) k_adj_link<<<(d.nl + 127) / 128, 128, 0, st>>>(d, s, a);
+    if (d.nv) k_adj_voxel<<<adj_grid(d.nv), fp64_threads(d.nv, 128), 0, st>>>(d, s, a);
+    if (d.nl) k_adj_link<<<adj_grid(d.nl), fp64_threads(d.nl, 128), 0, st>>>(d, s, a);
 }
 void launch_adj_gather_slots(const Dev &d, const Snap &sg, const Snap *ss, const AdjBufs &a, cudaStream_t st) {
     const int n = d.nv > d.nl ? d.nv : d.nl;
     if (!ss) {
-        if (d.nv) k_adj_gather<<<(d.nv + 127) / 128, 128, 0, st>>>(d, sg, a);
+        if (d.nv) k_adj_gather<<<adj_grid(d.nv), fp64_threads(d.nv, 128), 0, st>>>(d, sg, a);
     } else if (n) {
-        k_adj_gather_slots<<<(n + 127) / 128, 128, 0, st>>>(d, sg, *ss, a);
+        k_adj_gather_slots<<<adj_grid(n), fp64_threads(n, 128), 0, st>>>(d, sg, *ss, a);
     }
 }
 
@@ -85,12 +90,12 @@ __global__ void __launch_bounds__(128) k_adj_contact(Dev d, Snap s, AdjBufs a) {
 }
 
 void launch_adj_contact(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st) {
-    if (d.ns) k_adj_contact<<<(d.ns + 127) / 128, 128, 0, st>>>(d, s, a);
+    if (d.ns) k_adj_contact<<<adj_grid(d.ns), fp64_threads(d.ns, 128), 0, st>>>(d, s, a);
 }
 
 void launch_adj_seed(const Dev &d, const AdjBufs &a, cudaStream_t st) {
     const int n = d.nv > d.nl ? d.nv : d.nl;
-    if (n) k_adj_seed<<<(n + 127) / 128, 128, 0, st>>>(d, a);
+    if (n) k_adj_seed<<<adj_grid(n), fp64_threads(n, 128), 0, st>>>(d, a);
 }
 
 }  // namespace vx3g

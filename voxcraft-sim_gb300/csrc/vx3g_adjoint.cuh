@@ -238,7 +238,7 @@ __device__ __forceinline__ void link_forward(const Dev &d, const Snap &s, int l,
     if (small) {
         pos2.x -= restR;
     } else {
-        angle1 = from_angle_to_posx(angle1, pos2);
+        angle1 = from_angle_to_posx(angle1, pos2, len(pos2));
         angle2 = qmul(angle1, angle2);
         pos2 = V{len(pos2) - restR, 0, 0};
     }

@@ -1424,7 +1424,10 @@ cudaError_t launch_collision(const Dev &d, cudaStream_t s) {
 void launch_coll_eval(const Dev &d, cudaStream_t s) {
     if (!d.ns) return;
     if (d.mixed) launch_coll_eval_mixed(d, s);
-    else k_coll_eval<<<(d.ns + 255) / 256, 256, 0, s>>>(d);
+    else {
+        const int t = fp64_threads(d.ns, 256);
+        k_coll_eval<<<(d.ns + t - 1) / t, t, 0, s>>>(d);
+    }
 }
 
 // ---------------------------------------------------------------- host state exchange

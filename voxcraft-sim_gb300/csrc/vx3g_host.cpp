@@ -367,6 +367,8 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
 
     std::vector<VMat> vmats;
     std::vector<LMat> lmats;
+    std::vector<int> lrob;  // the robot of each link material
+    bool any_actuated = false;
     std::vector<RobotP> rps(c->nr);
     std::vector<double4> pos, quat;
     std::vector<float> tempe;
@@ -506,6 +508,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
             }
         }
         RobotP &rp = rps[r];
+        any_actuated |= R.vary_temp && R.temp_period > 0;
         rp.vox_size = R.vox_size;
         rp.temp_amp = R.temp_amplitude;
         rp.temp_period = R.temp_period;
@@ -715,6 +718,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
                 vnb_h[6 * (size_t)c->ends[l].y + 2 * a + 1] = c->ends[l].x;  // positive end: toward -axis
             }
         }
+        lrob.resize(lmats.size(), r);
         // lists in shared memory when the robot fits (lattice coordinates below 512, packed in 10 bits each)
         int cmax = 0;
         for (int k = 0; k < nvr; k++) {
@@ -805,6 +809,16 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     d.rp = drp;
     d.vmat = dvm;
     d.lmat = dlm;
+    d.lmatd = nullptr;
+    d.act = nullptr;
+    d.actv = nullptr;
+    LMatD *lmatd = nullptr;  // FP64: link constants and actuation phases (filled once the time step is known)
+    int *lrob_d = nullptr;
+    if (!d.mixed) {
+        if ((rc = c->alloc(&lmatd, lmats.size())) || (rc = c->upload(&lrob_d, lrob))) return rc;
+        d.lmatd = lmatd;
+        if (any_actuated && ((rc = c->alloc(&d.act, 2 * (size_t)d.nr)) || (rc = c->alloc(&d.actv, d.nv)))) return rc;
+    }
     MathTok *dft;
     if ((rc = c->upload(&dft, ftok))) return rc;
     d.ftok = dft;
@@ -906,6 +920,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
 
     launch_init_temperature(d, c->precision == VX3G_PRECISION_MIXED, c->stream);
     launch_dt(d, c->scratch, c->stream);
+    if (!d.mixed) launch_fp64_tables(d, lmatd, lrob_d, (int)lmats.size(), c->stream);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(c->stream));
     return VX3G_OK;
@@ -1871,11 +1886,13 @@ int vx3g_backward(vx3g_ctx *c, const double *dL_dcom, double *dL_dphase, double 
         const int len = std::min(k, n - j * k);
         const int p0 = (int)((c->rec_start + (int64_t)j * k) & 1);
         launch_snap_copy(live, c->rec_ck[j], d.nv, d.nl, d.nr, c->stream);
+        launch_actuation(d, p0, c->stream);
         cudaGraphExec_t g = nullptr;
         if ((rc = adj_segment_graph(c, a, len, p0, &g))) return rc;
         CU(cudaGraphLaunch(g, c->stream));
     }
     launch_snap_copy(live, c->rec_end, d.nv, d.nl, d.nr, c->stream);
+    launch_actuation(d, (int)(c->steps & 1), c->stream);
     CU(cudaMemcpyAsync(d.slots, c->rec_slots, 36 * nv * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     CU(cudaMemcpyAsync(d.contact, (double *)c->rec_slots + 36 * nv, nv * sizeof(double4), cudaMemcpyDeviceToDevice,
                        c->stream));

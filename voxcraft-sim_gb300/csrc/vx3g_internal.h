@@ -77,6 +77,12 @@ struct LMat {  // one link material (global index), oriented: (negative end, pos
     int ssn, sso;     // stress-strain points of a non-linear model: (0,0), then the model's from (0,0) on
 };
 
+struct LMatD {  // FP64 contexts: a link material's constants as the FP64 link pass multiplies by them
+    double b1, b2, b3, a2, sqA1, sqB1, sqA2, sqB2, sqB3;
+    double kN, kP, jN, jP;  // the ends' dampingMultiplier / 2 and / 4 at the robot's time step
+    int same, pad;          // kN == kP
+};
+
 struct RobotP {
     double vox_size, temp_amp, temp_period, inv_period, dt_frac;
     float cyc_rate, amp_f;  // mixed precision: actuation cycles per second (inv_period * kCycle), amplitude
@@ -174,6 +180,13 @@ struct Dev {
     // materials
     const VMat *vmat;
     const LMat *lmat;
+    // FP64 contexts (NULL in mixed ones): lmat in FP64; [2][NR] by parity, written with T, sine and
+    // cosine of a robot's actuation argument at the end of the step, the bound of the temperature
+    // formed from them, and that time; per voxel sine and cosine of its phase term (the last two
+    // NULL without actuated robots)
+    const LMatD *lmatd;
+    double4 *act;
+    double2 *actv;
     // collision
     int *csurf;     // collision surface list (global voxel index), NS entries
     int4 *ccell;    // x: the bucket of a collision-surface voxel in the large-robot grid (-1: not binned)
@@ -259,9 +272,24 @@ __device__ __forceinline__ double4 load_state(const Dev &d, const double4 *a, in
 }
 #endif
 
+// Threads per block of an FP64 pass over n elements.  An SM issues one FP64 warp instruction
+// about every 16-20 cycles, whichever of its warps it comes from, so these passes are bound by
+// the busiest SM's count of warps, not by occupancy: blocks of one warp spread a small batch over
+// all 152 SMs (a 10^3 block's link pass, 2,700 links: 31.2 us in 11 blocks of 256 threads, 7.4 us
+// in 85 of 32).  Once every SM has eight blocks, larger ones cost nothing and launch faster.
+inline int fp64_threads(int n, int most) {
+    int t = 32;
+    while (t < most && (n + t - 1) / t > 152 * 8) t *= 2;
+    return t;
+}
+
 // launchers (defined in the .cu files)
 void launch_links_fp64(const Dev &d, cudaStream_t s);
 void launch_voxels_fp64(const Dev &d, int parity, cudaStream_t s);
+// FP64 contexts: fills lmatd (lrob: the robot of each link material) and actv; and act for the
+// step of the given parity (again whenever T was written by anything but the voxel pass)
+void launch_fp64_tables(const Dev &d, LMatD *lmatd, const int *lrob, int n, cudaStream_t s);
+void launch_actuation(const Dev &d, int parity, cudaStream_t s);
 // launch shapes of the mixed-precision passes (vx3g_mixed.cu), chosen by vx3g_autotune
 struct LaunchShape { int threads, min_blocks; };
 constexpr int kMixedShapes = 6;

@@ -1,10 +1,6 @@
-// vx3g_step.cuh -- the two per-step passes, templated on the link-math type R.
-//
-//   R = double : the reference's arithmetic (FP64 vectors; float wherever the
-//                reference uses float).  Compiled with --fmad=false so that the
-//                rounding sequence matches the reference step op for op.
-//   R = float  : FP32 link forces/moments and FP32 force/moment sums; positions,
-//                momenta and quaternions stay FP64 and are advanced in FP64.
+// vx3g_step.cuh -- the two per-step passes in the reference's arithmetic (FP64 vectors; float
+// wherever the reference uses float) and the math they share with the other units.  Compiled
+// with --fmad=false so that the rounding sequence matches the reference step op for op.
 //
 // Link pass  : VX3_Link::orientLink + updateForces + updateStrain
 //              (src/VX3/VX3_Link.cu:90-260), one thread per link.
@@ -66,66 +62,133 @@ template <class R> __device__ __forceinline__ V3<R> qrotinv(Q4<R> q, V3<R> f) {
                  tw * q.z + tx * q.y - ty * q.x + tz * q.w};
 }
 
-// ToRotationVector (VX3_Quat3D.h:347-359).  The FP64 form is the reference's;
-// the FP32 form computes 1-w^2 as |xyz|^2 and acos(w) as atan2(|xyz|, w), the
-// same function without the cancellation that FP32 would suffer near w = 1.
-template <class R> __device__ __forceinline__ V3<R> to_rotvec(Q4<R> q) {
-    V3<R> v{q.x, q.y, q.z};
-    if constexpr (std::is_same<R, double>::value) {
-        if (q.w >= 1.0 || q.w <= -1.0) return V3<R>{0, 0, 0};
-        double sq = 1.0 - q.w * q.w;
-        if (sq < 2.4e-3) return scl(scl(v, 2.0), sqrt((2 - 2 * q.w) / sq));
-        return vdiv(scl(scl(v, 2.0), acos(q.w)), sqrt(sq));
-    } else {
-        const float s2 = q.x * q.x + q.y * q.y + q.z * q.z;
-        if (!(s2 > 0.0f)) return V3<R>{0, 0, 0};
-        const float s = sqrtf(s2);
-        return scl(v, 2.0f * atan2f(s, q.w) / s);
-    }
+// ------------------------------------------------------------- FP64 arithmetic that is not FP64
+// GB300 starts an FP64 warp instruction every 19 cycles per SM (64 cycles per warp, active lanes
+// or not, measured) and a float-to-double conversion every 16, against four FP32 or integer ones
+// per cycle: the FP64 passes are bound by the number of FP64 instructions.  What is only compared
+// is therefore compared as integers or in FP32 with a margin, falling back to the exact FP64
+// expression inside the margin, and FP32 constants come converted (LMatD) or are widened with
+// integer operations.  Values keep the reference's rounding, operation for operation.
+__device__ __forceinline__ int hi_word(double x) {
+#if defined(__CUDA_ARCH__)
+    return __double2hiint(x);
+#else
+    long long b;
+    __builtin_memcpy(&b, &x, 8);
+    return (int)(b >> 32);
+#endif
+}
+__device__ __forceinline__ int lo_word(double x) {
+#if defined(__CUDA_ARCH__)
+    return __double2loint(x);
+#else
+    long long b;
+    __builtin_memcpy(&b, &x, 8);
+    return (int)b;
+#endif
+}
+__device__ __forceinline__ double from_words(int hi, int lo) {
+#if defined(__CUDA_ARCH__)
+    return __hiloint2double(hi, lo);
+#else
+    const long long b = ((long long)hi << 32) | (unsigned)lo;
+    double x;
+    __builtin_memcpy(&x, &b, 8);
+    return x;
+#endif
+}
+__device__ __forceinline__ float int_float(int i) {
+#if defined(__CUDA_ARCH__)
+    return __int_as_float(i);
+#else
+    float f;
+    __builtin_memcpy(&f, &i, 4);
+    return f;
+#endif
+}
+__device__ __forceinline__ int float_int(float f) {
+#if defined(__CUDA_ARCH__)
+    return __float_as_int(f);
+#else
+    int i;
+    __builtin_memcpy(&i, &f, 4);
+    return i;
+#endif
+}
+// (double)f, exact
+__device__ __forceinline__ double widen(float f) {
+    const int b = float_int(f), e = b & 0x7f800000;
+    if (e == 0 || e == 0x7f800000) return (double)f;
+    return from_words((b & (int)0x80000000) | (((b & 0x7fffffff) >> 3) + 0x38000000), b << 29);
+}
+// |x| in FP32, truncated: at most 2^-20 relative below |x|; 0 below FP32's range, a huge value or
+// NaN above it.  For comparisons with a margin.
+__device__ __forceinline__ float mag(double x) {
+    const int h = (hi_word(x) & 0x7fffffff) - 0x38000000;
+    return int_float(h < 0 ? 0 : h >= 0x0ff00000 ? 0x7fc00000 : h << 3);
+}
+__device__ __forceinline__ float signed_mag(double x) {
+    return int_float(float_int(mag(x)) | (hi_word(x) & (int)0x80000000));
 }
 
-// FromRotationVector (VX3_Quat3D.h:363-377)
-template <class R> __device__ __forceinline__ Q4<R> from_rotvec(V3<R> in) {
-    V3<R> th = vdiv(in, (R)2);
-    R s, m2 = th.x * th.x + th.y * th.y + th.z * th.z;
-    Q4<R> q;
-    if (m2 * m2 < (R)5.328e-15) {
-        q.w = (R)1.0 - (R)0.5 * m2;
-        s = (R)1.0 - m2 / (R)6.0;
-    } else {
-        R m = sqrt(m2);
-        q.w = cos(m);
-        s = sin(m) / m;
+// ToRotationVector (VX3_Quat3D.h:347-359), its comparisons on the bits (|w| >= 1; 1 - w^2 >= 0)
+__device__ __forceinline__ V3<double> to_rotvec(Q4<double> q) {
+    if ((unsigned)((hi_word(q.w) & 0x7fffffff) - 0x3ff00000) <= 0x40000000u) return V3<double>{0, 0, 0};  // |w| >= 1
+    const V3<double> v{q.x, q.y, q.z};
+    const double sq = 1.0 - q.w * q.w;
+    if (mag(sq) < 2.399e-3f || sq < 2.4e-3) {
+        const double g = sqrt(fma(-2.0, q.w, 2.0) / sq);  // 1 to 1.0003
+        return scl(v, from_words(hi_word(g) + 0x100000, lo_word(g)));  // 2g
     }
-    q.x = th.x * s;
-    q.y = th.y * s;
-    q.z = th.z * s;
-    return q;
+    return vdiv(scl(scl(v, 2.0), acos(q.w)), sqrt(sq));
 }
 
-// FromAngleToPosX (VX3_Quat3D.h:384-432); q unchanged for a zero vector
-template <class R> __device__ __forceinline__ Q4<R> from_angle_to_posx(Q4<R> q, V3<R> r) {
+// FromRotationVector (VX3_Quat3D.h:363-377) of the rotation vector 2*th.  sincos gives the bits of
+// sin and cos for 27 FP64 instructions instead of 43.
+__device__ __forceinline__ Q4<double> from_half_rotvec(V3<double> th) {
+    const double m2 = th.x * th.x + th.y * th.y + th.z * th.z;
+    double w, s;
+    if (m2 * m2 < 5.328e-15) {
+        w = fma(-0.5, m2, 1.0);
+        s = 1.0 - m2 / 6.0;
+    } else {
+        const double m = sqrt(m2);
+        sincos(m, &s, &w);
+        s = s / m;
+    }
+    return Q4<double>{w, th.x * s, th.y * s, th.z * s};
+}
+__device__ __forceinline__ Q4<double> from_rotvec(V3<double> in) { return from_half_rotvec(scl(in, 0.5)); }
+
+// FromAngleToPosX (VX3_Quat3D.h:384-432); q unchanged for a zero vector.  l = |r|.
+__device__ __forceinline__ Q4<double> from_angle_to_posx(Q4<double> q, V3<double> r, double l) {
     if (r.x == 0 && r.y == 0 && r.z == 0) return q;
-    R yx = r.y / r.x, zx = r.z / r.x;
-    const R SA = (R)1.732e-2;
-    if (yx < SA && yx > -SA && zx < SA && zx > -SA) {
-        q.x = 0;
-        q.y = (R)0.5 * zx;
-        q.z = (R)-0.5 * yx;
-        q.w = 1 + (R)0.5 * (-q.y * q.y - q.z * q.z);
-        return q;
+    const float sx = 0.0174f * mag(r.x);
+    if (!(mag(r.y) > sx || mag(r.z) > sx)) {  // near the shortcut's bound: decide exactly
+        const double yx = r.y / r.x, zx = r.z / r.x, SA = 1.732e-2;
+        if (yx < SA && yx > -SA && zx < SA && zx > -SA) {
+            q.x = 0;
+            q.y = 0.5 * zx;
+            q.z = -0.5 * yx;
+            q.w = 1 + 0.5 * (-q.y * q.y - q.z * q.z);
+            return q;
+        }
     }
-    V3<R> n = r;
-    R l = sqrt(n.x * n.x + n.y * n.y + n.z * n.z);
+    V3<double> n = r;
     if (l > 0) {
-        R li = (R)1.0 / l;
+        const double li = 1.0 / l;
         n.x *= li; n.y *= li; n.z *= li;
     }
-    R theta = acos(n.x);
-    if (theta > (R)(3.14159265358979 - 1e-7)) return Q4<R>{0, 0, 1, 0};
-    R axis_inv = (R)1.0 / sqrt(n.z * n.z + n.y * n.y);
-    R a = (R)0.5 * theta, s = sin(a);
-    return Q4<R>{cos(a), 0, n.z * axis_inv * s, -n.y * axis_inv * s};
+    const double theta = acos(n.x);
+    if (theta > 3.14159265358979 - 1e-7) return Q4<double>{0, 0, 1, 0};
+    const double axis_inv = 1.0 / sqrt(n.z * n.z + n.y * n.y);
+    double s, c;
+    sincos(0.5 * theta, &s, &c);
+    return Q4<double>{c, 0, n.z * axis_inv * s, -n.y * axis_inv * s};
+}
+
+__device__ __forceinline__ bool is_zero(V3<double> a) {  // on the bits, either sign
+    return (((hi_word(a.x) | hi_word(a.y) | hi_word(a.z)) & 0x7fffffff) | lo_word(a.x) | lo_word(a.y) | lo_word(a.z)) == 0;
 }
 
 // VX3_Link.h:134-191 (bond-local +X frame and back)
@@ -344,7 +407,103 @@ __device__ __forceinline__ void new_link_scale_mx(const Dev &d, int l, int dneg,
     d.lnew[l] = n - 1;
 }
 
+// the constants of a link in FP64, from the damping numerators of its ends (VX3_Voxel::
+// dampingMultiplier, VX3_Voxel.h:206-208: previousDt is the robot's dt once a voxel has stepped,
+// 0 for fixed voxels, which never step)
+__device__ __forceinline__ LMatD make_lmatd(const LMat &m, float dmcN, float dmcP, bool fixN, bool fixP, float dtf) {
+    LMatD c;
+    c.b1 = widen(m.b1), c.b2 = widen(m.b2), c.b3 = widen(m.b3), c.a2 = widen(m.a2);
+    c.sqA1 = widen(m.sqA1), c.sqB1 = widen(m.sqB1), c.sqA2 = widen(m.sqA2xIp), c.sqB2 = widen(m.sqB2xFMp);
+    c.sqB3 = widen(m.sqB3xIp);
+    const float dmN = dmcN / (fixN ? 0.0f : dtf), dmP = dmcP / (fixP ? 0.0f : dtf);
+    c.kN = 0.5 * widen(dmN), c.kP = 0.5 * widen(dmP);
+    c.jN = 0.5 * c.kN, c.jP = 0.5 * c.kP;
+    c.same = dmN == dmP ? 1 : 0;
+    return c;
+}
+__device__ __forceinline__ LMatD link_consts(const Dev &d, uint32_t i, int2 e, float dtf) {
+    if (d.lmatd) return d.lmatd[i];
+    const uint32_t fn = d.vinfo[e.x].y, fp = d.vinfo[e.y].y;
+    return make_lmatd(d.lmat[i], d.vmat[fn >> 8].dmc, d.vmat[fp >> 8].dmc, fn & VF_FIXED, fp & VF_FIXED, dtf);
+}
+
+// the hysteresis of orientLink (VX3_Link.cu:107-125) on pos2 before the rest length is taken off:
+// SmallTurn = (|z| + |y|)/x, ExtendPerc = |1 - x/rest|.  Decided in FP32 on the truncated
+// magnitudes where they are clear of the thresholds by more than the truncation (2^-20), else
+// with the reference's divisions
+__device__ __forceinline__ void turn_state(V3<double> pos2, double rest, bool &small, bool &lvv) {
+    const float X = mag(pos2.x), T = mag(pos2.y) + mag(pos2.z), R = mag(rest);
+    const bool ahead = hi_word(pos2.x) > 0;
+    if (small) {
+        if (ahead && T < 0.05999f * X && X > 0.401f * R && X < 1.599f * R) return;  // stays small
+    } else if (ahead && T > 0.05001f * X) {
+        return;  // stays large
+    }
+    const float SmallTurn = (float)((fabs(pos2.z) + fabs(pos2.y)) / pos2.x);
+    const float ExtendPerc = (float)(fabs(1 - pos2.x / rest));
+    const float HF = 1.2f, BEND = 0.05f, EXT = 0.50f;
+    if (!small && SmallTurn < BEND && ExtendPerc < EXT) {
+        small = true;
+        lvv = false;
+    } else if (small && (SmallTurn > HF * BEND || ExtendPerc > HF * EXT)) {
+        small = false;
+        lvv = false;
+    }
+}
+
+// The elastic and damping forces and moments of a link in its own frame (VX3_Link::updateForces,
+// VX3_Link.cu:150-204).  Factors 1/2 and 2 are moved through products, which is exact; a link
+// that is and was in the small-angle branch (a1v and oldA1 zero) leaves out the terms that are zero;
+// ends with equal damping have opposite forces.
+struct LinkForces {
+    V3<double> fNeg, fPos, mNeg, mPos;
+};
+__device__ __forceinline__ LinkForces link_forces(const LMatD &c, float axial, bool lvv, bool bent, V3<double> pos2,
+                                                  V3<double> oldPos2, V3<double> a1v, V3<double> oldA1, V3<double> a2v,
+                                                  V3<double> oldA2) {
+    LinkForces o;
+    const double t1 = c.b2 * pos2.z, t3 = c.b2 * pos2.y;
+    const V3<double> D = sub(pos2, oldPos2), E2 = sub(a2v, oldA2);  // twice dPos2, dAngle2
+    const double fx = widen(axial);
+    V3<double> P, U, W;  // twice the reference's posCalc and the moments' damping vectors at the two ends
+    if (!bent) {
+        const double t2 = c.b3 * a2v.y, t4 = c.b3 * a2v.z, u2 = c.sqB3 * E2.y, u4 = c.sqB3 * E2.z;
+        const double u1 = c.sqB2 * D.z, u3 = c.sqB2 * D.y;
+        o.fNeg = V3<double>{fx, c.b1 * pos2.y - c.b2 * a2v.z, c.b1 * pos2.z + c.b2 * a2v.y};
+        o.mNeg = V3<double>{c.a2 * a2v.x, -t1 - t2, t3 - t4};
+        o.mPos = V3<double>{-o.mNeg.x, fma(-2.0, t2, -t1), fma(-2.0, t4, t3)};
+        P = V3<double>{c.sqA1 * D.x, c.sqB1 * D.y - c.sqB2 * E2.z, c.sqB1 * D.z + c.sqB2 * E2.y};
+        const double ux = c.sqA2 * E2.x;
+        U = V3<double>{-ux, u1 + u2, u4 - u3};
+        W = V3<double>{ux, fma(2.0, u2, u1), fma(2.0, u4, -u3)};
+    } else {
+        const V3<double> E1 = sub(a1v, oldA1);
+        o.fNeg = V3<double>{fx, c.b1 * pos2.y - c.b2 * (a1v.z + a2v.z), c.b1 * pos2.z + c.b2 * (a1v.y + a2v.y)};
+        o.mNeg = V3<double>{c.a2 * (a2v.x - a1v.x), -t1 - c.b3 * (2 * a1v.y + a2v.y), t3 - c.b3 * (2 * a1v.z + a2v.z)};
+        o.mPos = V3<double>{-o.mNeg.x, -t1 - c.b3 * (a1v.y + 2 * a2v.y), t3 - c.b3 * (a1v.z + 2 * a2v.z)};
+        P = V3<double>{c.sqA1 * D.x, c.sqB1 * D.y - c.sqB2 * (E1.z + E2.z), c.sqB1 * D.z + c.sqB2 * (E1.y + E2.y)};
+        const double ux = c.sqA2 * (E2.x - E1.x);
+        U = V3<double>{-ux, c.sqB2 * D.z + c.sqB3 * (2 * E1.y + E2.y), c.sqB3 * (2 * E1.z + E2.z) - c.sqB2 * D.y};
+        W = V3<double>{ux, c.sqB2 * D.z + c.sqB3 * (E1.y + 2 * E2.y), c.sqB3 * (E1.z + 2 * E2.z) - c.sqB2 * D.y};
+    }
+    if (!lvv) {
+        o.fPos = neg(o.fNeg);
+        return o;
+    }
+    if (c.same) {
+        o.fNeg = add(o.fNeg, scl(P, c.kN));
+        o.fPos = neg(o.fNeg);
+    } else {
+        o.fPos = neg(add(o.fNeg, scl(P, c.kP)));
+        o.fNeg = add(o.fNeg, scl(P, c.kN));
+    }
+    o.mNeg = sub(o.mNeg, scl(U, c.jN));
+    o.mPos = sub(o.mPos, scl(W, c.jP));
+    return o;
+}
+
 template <class R> __device__ __forceinline__ void link_update(const Dev &d, int l) {
+    static_assert(std::is_same<R, double>::value, "the FP64 step");
     const uint2 li = d.linfo[l];
     const int r = (int)li.x;
     if (d.status[r] != 0) return;
@@ -363,43 +522,35 @@ template <class R> __device__ __forceinline__ void link_update(const Dev &d, int
     const V3<R> oldA2{ls[6 * NL + l], ls[7 * NL + l], ls[8 * NL + l]};
 
     // orientLink (VX3_Link.cu:90-133)
-    V3<R> pos2 = to_axis_x(axis, V3<R>{(R)(pp.x - pn.x), (R)(pp.y - pn.y), (R)(pp.z - pn.z)});
-    Q4<R> angle1 = to_axis_xq(axis, Q4<R>{(R)qn.x, (R)qn.y, (R)qn.z, (R)qn.w});
-    Q4<R> angle2 = to_axis_xq(axis, Q4<R>{(R)qp.x, (R)qp.y, (R)qp.z, (R)qp.w});
+    V3<R> pos2 = to_axis_x(axis, V3<R>{pp.x - pn.x, pp.y - pn.y, pp.z - pn.z});
+    Q4<R> angle1 = to_axis_xq(axis, Q4<R>{qn.x, qn.y, qn.z, qn.w});
+    Q4<R> angle2 = to_axis_xq(axis, Q4<R>{qp.x, qp.y, qp.z, qp.w});
     const Q4<R> tot = qconj(angle1);
     pos2 = qrot(tot, pos2);
     angle2 = qmul(tot, angle2);
     angle1 = Q4<R>{1, 0, 0, 0};
-    const R restR = (R)rest;
-    const float SmallTurn = (float)((fabs(pos2.z) + fabs(pos2.y)) / pos2.x);
-    const float ExtendPerc = (float)(fabs(1 - pos2.x / restR));
-    const float HF = 1.2f, BEND = 0.05f, EXT = 0.50f;
     bool small = (fl & LF_SMALL) != 0, lvv = (fl & LF_LVV) != 0;
-    if (!small && SmallTurn < BEND && ExtendPerc < EXT) {
-        small = true;
-        lvv = false;
-    } else if (small && (SmallTurn > HF * BEND || ExtendPerc > HF * EXT)) {
-        small = false;
-        lvv = false;
-    }
+    turn_state(pos2, rest, small, lvv);
+    V3<R> a1v{0, 0, 0};
     if (small) {
-        pos2.x -= restR;
+        pos2.x -= rest;
     } else {
-        angle1 = from_angle_to_posx(angle1, pos2);
+        const R l2 = len(pos2);
+        angle1 = from_angle_to_posx(angle1, pos2, l2);
         angle2 = qmul(angle1, angle2);
-        pos2 = V3<R>{len(pos2) - restR, 0, 0};
+        pos2 = V3<R>{l2 - rest, 0, 0};
+        a1v = to_rotvec(angle1);
     }
-    const V3<R> a1v = to_rotvec(angle1), a2v = to_rotvec(angle2);
+    const V3<R> a2v = to_rotvec(angle2);
     ls[l] = pos2.x; ls[NL + l] = pos2.y; ls[2 * NL + l] = pos2.z;
-    ls[3 * NL + l] = a1v.x; ls[4 * NL + l] = a1v.y; ls[5 * NL + l] = a1v.z;
+    const bool bent = !small || !is_zero(oldA1);
+    if (bent) {
+        ls[3 * NL + l] = a1v.x; ls[4 * NL + l] = a1v.y; ls[5 * NL + l] = a1v.z;
+    }
     ls[6 * NL + l] = a2v.x; ls[7 * NL + l] = a2v.y; ls[8 * NL + l] = a2v.z;
 
-    // updateForces (VX3_Link.cu:135-218) + updateStrain (:220-260), linear model
-    const R half = (R)0.5;
-    const V3<R> dPos2 = scl(sub(pos2, oldPos2), half);
-    const V3<R> dA1 = scl(sub(a1v, oldA1), half);
-    const V3<R> dA2 = scl(sub(a2v, oldA2), half);
-    const float axialStrain = (float)(pos2.x / restR);
+    // updateForces (VX3_Link.cu:135-218) + updateStrain (:220-260)
+    const float axialStrain = (float)(pos2.x / rest);
     float2 sm = d.strain[l];
     sm.x = axialStrain;
     const float stress = link_stress(d, m, l, axialStrain, &sm.y);
@@ -418,99 +569,116 @@ template <class R> __device__ __forceinline__ void link_update(const Dev &d, int
         if (nfl != fl) d.linfo[l].y = nfl;
         return;
     }
-    const float b1 = m.b1, b2 = m.b2, b3 = m.b3, a2 = m.a2;
-    V3<R> fNeg{(R)(stress * m.area), b1 * pos2.y - b2 * (a1v.z + a2v.z), b1 * pos2.z + b2 * (a1v.y + a2v.y)};
-    V3<R> fPos = neg(fNeg);
-    V3<R> mNeg{a2 * (a2v.x - a1v.x), -b2 * pos2.z - b3 * (2 * a1v.y + a2v.y), b2 * pos2.y - b3 * (2 * a1v.z + a2v.z)};
-    V3<R> mPos{a2 * (a1v.x - a2v.x), -b2 * pos2.z - b3 * (a1v.y + 2 * a2v.y), b2 * pos2.y - b3 * (a1v.z + 2 * a2v.z)};
-    if (lvv) {
-        const float sqA1 = m.sqA1, sqA2xIp = m.sqA2xIp, sqB1 = m.sqB1, sqB2xFMp = m.sqB2xFMp, sqB3xIp = m.sqB3xIp;
-        const V3<R> posCalc{sqA1 * dPos2.x, sqB1 * dPos2.y - sqB2xFMp * (dA1.z + dA2.z),
-                            sqB1 * dPos2.z + sqB2xFMp * (dA1.y + dA2.y)};
-        // VX3_Voxel::dampingMultiplier (VX3_Voxel.h:206-208); previousDt is this robot's dt
-        // once a voxel has stepped, 0 for fixed voxels (they never step)
-        const float dtf = d.dt[r];
-        const uint32_t fnv = d.vinfo[e.x].y, fpv = d.vinfo[e.y].y;
-        const float dmN = d.vmat[fnv >> 8].dmc / ((fnv & VF_FIXED) ? 0.0f : dtf);
-        const float dmP = d.vmat[fpv >> 8].dmc / ((fpv & VF_FIXED) ? 0.0f : dtf);
-        fNeg = add(fNeg, scl(posCalc, dmN));
-        fPos = sub(fPos, scl(posCalc, dmP));
-        mNeg = sub(mNeg, scl(V3<R>{-sqA2xIp * (dA2.x - dA1.x), sqB2xFMp * dPos2.z + sqB3xIp * (2 * dA1.y + dA2.y),
-                                   -sqB2xFMp * dPos2.y + sqB3xIp * (2 * dA1.z + dA2.z)},
-                            (R)(half * dmN)));
-        mPos = sub(mPos, scl(V3<R>{sqA2xIp * (dA2.x - dA1.x), sqB2xFMp * dPos2.z + sqB3xIp * (dA1.y + 2 * dA2.y),
-                                   -sqB2xFMp * dPos2.y + sqB3xIp * (dA1.z + 2 * dA2.z)},
-                            (R)(half * dmP)));
-    } else {
-        lvv = true;
-    }
-    nfl |= lvv ? LF_LVV : 0u;
+    LinkForces f = link_forces(link_consts(d, fl >> 8, e, d.dt[r]), stress * m.area, lvv, bent, pos2, oldPos2, a1v, oldA1,
+                               a2v, oldA2);
+    nfl |= LF_LVV;
     if (!small) {
-        fNeg = qrotinv(angle1, fNeg);
-        mNeg = qrotinv(angle1, mNeg);
+        f.fNeg = qrotinv(angle1, f.fNeg);
+        f.mNeg = qrotinv(angle1, f.mNeg);
     }
-    fPos = qrotinv(angle2, fPos);
-    mPos = qrotinv(angle2, mPos);
-    store_slot(sNeg, to_axis_original(axis, fNeg), to_axis_original(axis, mNeg));
-    store_slot(sPos, to_axis_original(axis, fPos), to_axis_original(axis, mPos));
+    f.fPos = qrotinv(angle2, f.fPos);
+    f.mPos = qrotinv(angle2, f.mPos);
+    store_slot(sNeg, to_axis_original(axis, f.fNeg), to_axis_original(axis, f.mNeg));
+    store_slot(sPos, to_axis_original(axis, f.fPos), to_axis_original(axis, f.mPos));
     if (fl & LF_RUNTIME) new_link_scale(d, l, sNeg, sPos);
     if (nfl != fl) d.linfo[l].y = nfl;
-}
-
-template <class R> __global__ void __launch_bounds__(256) k_links(Dev d) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l < d.nl) link_update<R>(d, l);
 }
 
 // ------------------------------------------------------------ voxel pass
 // Temperature of a voxel at time t (gpu_update_temperature, VX3_VoxelyzeKernel.cu:625-650)
 // returned as the base size nomSize*(1+T*cte) (VX3_Voxel::baseSize); tempe gets T.
-template <bool EXACT> __device__ __forceinline__ double temperature_base_size(const RobotP &rp, const VMat &m,
-                                                                              double phase, double t,
-                                                                              double cur_bs, float *tempe) {
+template <bool EXACT = true>
+__device__ __forceinline__ double temperature_base_size(const RobotP &rp, const VMat &m, double phase, double t,
+                                                        double cur_bs, float *tempe) {
+    static_assert(EXACT, "the FP64 step");
     if (!(rp.vary_temp && rp.temp_period > 0)) return cur_bs;
     if (m.thermal_on_after > t || m.fixed) return cur_bs;
-    double T;
-    if (EXACT) {
-        T = rp.temp_amp * sin(2 * 3.1415926f * (t / rp.temp_period + phase));
-    } else {
-        // same phase in cycles, reduced to [0,1) in FP64, sine in FP32
-        double c = (double)(2 * 3.1415926f) * (t / rp.temp_period + phase) * (1.0 / 6.283185307179586);
-        c -= floor(c);
-        T = rp.temp_amp * (double)sinpif(2.0f * (float)c);
-    }
+    double T = rp.temp_amp * sin(2 * 3.1415926f * (t / rp.temp_period + phase));
     if (!rp.expansion && T > 0) T = 0;
     const float tf = (float)T;
     *tempe = tf;
     return m.nom_size * (1 + tf * m.cte);
 }
 
+// sine and cosine of the actuation argument 2*3.1415926f*t/P of a robot at its next step's time,
+// with that time and a bound on what the two ways to the temperature differ by: an argument of
+// up to 2 pi (t/P + 2) carries six roundings of itself between them
+__device__ __forceinline__ void actuation_phase(const Dev &d, int r, int parity, double t) {
+    const RobotP &rp = d.rp[r];
+    const double c = t / rp.temp_period, a = 2 * 3.1415926f * c;
+    double s, k;
+    sincos(a, &s, &k);
+    d.act[(size_t)parity * d.nr + r] = make_double4(s, k, fabs(rp.temp_amp) * 5e-15 * (fabs(c) + 4.0), t);
+}
+
+// The same temperature from the robot's sine and cosine and the voxel's own (of its phase), by
+// the addition theorem: 3 FP64 instructions instead of a division and a sine (about 45).  The
+// reference keeps T in 32 bits; T here is within act.z of its value, so where no rounding
+// boundary of FP32 (nor zero, the clamp) lies that near, the stored float is the reference's.
+// Elsewhere (about one voxel in 10^7) the reference's expression decides.
+__device__ __forceinline__ double next_base_size(const Dev &d, const RobotP &rp, const VMat &m, int v, int r, int parity,
+                                                 double t, double cur_bs, float *tempe) {
+    if (m.toa_pos && m.thermal_on_after > t) return cur_bs;
+    if (d.act) {
+        const double4 a = d.act[(size_t)parity * d.nr + r];
+        if (hi_word(a.w) == hi_word(t) && a.w == t) {
+            const double2 p = d.actv[v];
+            const double T = rp.temp_amp * fma(a.x, p.y, a.y * p.x);
+            const float lo = (float)(T - a.z), up = (float)(T + a.z);
+            if (!rp.expansion && lo > 0) {
+                *tempe = 0;
+                return m.nom_size;
+            }
+            if (lo == up) {
+                *tempe = lo;
+                return m.nom_size * widen(1 + lo * m.cte);
+            }
+        }
+    }
+    return temperature_base_size(rp, m, d.phase[v], t, cur_bs, tempe);
+}
+
+// sine and cosine of a voxel's phase term; NaN (the reference's expression decides every step)
+// for phases beyond two cycles, outside the bound above
+__device__ __forceinline__ double2 actuation_voxel(double phase) {
+    double s = NAN, k = NAN;
+    if (fabs(phase) <= 2.0) sincos(2 * 3.1415926f * phase, &s, &k);
+    return make_double2(s, k);
+}
+
+// the voxel is clear of the floor: baseSize/2 - nomSize/2 - z < 0, with a margin of several of the
+// FP32 magnitudes' truncations (floorPenetration, VX3_Voxel.h:185-188)
+__device__ __forceinline__ bool above_floor(double bs, double nom, double z) {
+    const float b = mag(bs), zf = signed_mag(z);
+    return zf > 0.5f * (b - mag(nom)) + 4e-6f * (b + fabsf(zf));
+}
+__device__ __forceinline__ float floor_penetration(double bs, double nom, double z) {
+    const double bsa = (bs + bs + bs) / 3.0f;  // baseSizeAverage (VX3_Voxel.h:102-105)
+    return (float)(bsa / 2 - nom / 2 - z);
+}
+
 template <class R> __device__ __forceinline__ void voxel_update(const Dev &d, int v, int parity) {
-    constexpr bool EXACT = std::is_same<R, double>::value;
+    static_assert(std::is_same<R, double>::value, "the FP64 step");
     const uint2 vi = d.vinfo[v];
     const int r = (int)vi.x;
     const RobotP &rp = d.rp[r];
     const double Tcur = d.T[(size_t)parity * d.nr + r];
     const int st = d.status[r];
     const float dtf = d.dt[r];
-    if (v == rp.voff) d.T[(size_t)(parity ^ 1) * d.nr + r] = (st == 0) ? Tcur + dtf : Tcur;  // currentTime += dt
+    const double dt = widen(dtf), tn = Tcur + dt;
+    if (v == rp.voff) d.T[(size_t)(parity ^ 1) * d.nr + r] = (st == 0) ? tn : Tcur;  // currentTime += dt
     if (st != 0) return;
     uint32_t fl = vi.y;
     if (fl & VF_FIXED) return;
-    const VMat m = d.vmat[fl >> 8];
-    const double dt = dtf;
+    const VMat &m = d.vmat[fl >> 8];
     double4 p = d.pos[v];
-    const double4 q = d.quat[v];
-    const double4 lm = d.linmom[v];
-    const double4 am = d.angmom[v];
-    const double tn = Tcur + dt;
 
     const bool actuated = rp.vary_temp && rp.temp_period > 0;
     float *tcur = d.tempe + (size_t)parity * d.nv, *tnext = d.tempe + (size_t)(parity ^ 1) * d.nv;
-    if (dt == 0.0f) {  // VX3_Voxel::timeStep returns before moving; temperature still follows time
+    if (dtf == 0.0f) {  // VX3_Voxel::timeStep returns before moving; temperature still follows time
         if (actuated) {
             float te = tcur[v];
-            p.w = temperature_base_size<EXACT>(rp, m, d.phase[v], tn, p.w, &te);
+            p.w = temperature_base_size(rp, m, d.phase[v], tn, p.w, &te);
             d.pos[v] = p;
             tnext[v] = te;
         }
@@ -532,12 +700,15 @@ template <class R> __device__ __forceinline__ void voxel_update(const Dev &d, in
         d.angmom[v] = make_double4(0, 0, 0, 0);
         if (actuated) {
             float te = tcur[v];
-            p.w = temperature_base_size<EXACT>(rp, m, d.phase[v], tn, p.w, &te);
+            p.w = next_base_size(d, rp, m, v, r, parity, tn, p.w, &te);
             tnext[v] = te;
         }
         d.pos[v] = p;
         return;
     }
+    const double4 q = d.quat[v];
+    const double4 lm = d.linmom[v];
+    const double4 am = d.angmom[v];
 
     // link force/moment sums in direction order 0..5 (VX3_Voxel::force/moment, VX3_Voxel.cu:350-397)
     V3<R> Fs{0, 0, 0}, Ms{0, 0, 0};
@@ -546,164 +717,102 @@ template <class R> __device__ __forceinline__ void voxel_update(const Dev &d, in
     for (int dir = 0; dir < 6; dir++) {
         if (fl & (1u << dir)) {
             const Slot<R> s = S[(size_t)dir * d.nv + v];
-            Fs = add(Fs, V3<R>{s.f[0], s.f[1], s.f[2]});
-            Ms = add(Ms, V3<R>{s.m[0], s.m[1], s.m[2]});
+            const V3<R> f{s.f[0], s.f[1], s.f[2]}, n{s.m[0], s.m[1], s.m[2]};
+            Fs = dir ? add(Fs, f) : f;
+            Ms = dir ? add(Ms, n) : n;
         }
     }
     bool stat = (fl & VF_STATIC) != 0;
     const bool floorOn = rp.floor != 0;
     const double bs = p.w;
-    const double bsa = (bs + bs + bs) / 3.0f;  // baseSizeAverage (VX3_Voxel.h:102-105)
-    // floorPenetration (VX3_Voxel.h:185-188), before the position update
-    const float pen = (float)(bsa / 2 - m.nom_size / 2 - p.z);
     V3<double> lmv{lm.x, lm.y, lm.z}, amv{am.x, am.y, am.z};
-    V3<double> tr;
+    const double mass_inv = widen(m.mass_inv), mom_inv = widen(m.mom_inv);
+    // the floor is off, or the voxel clear of it: no floor force, and the penetration is not needed
+    const bool off = !floorOn || above_floor(bs, m.nom_size, p.z);
+    const float pen = off ? -1.0f : floor_penetration(bs, m.nom_size, p.z);  // before the position update
 
-    if constexpr (EXACT) {
-        const Q4<double> o{q.x, q.y, q.z, q.w};
-        V3<double> F = qrot(o, Fs);
-        if (xi >= 0) F = add(F, V3<double>{ex.f[0], ex.f[1], ex.f[2]});  // external force (:363-364)
-        const V3<double> vel = scl(lmv, m.mass_inv);
-        F = sub(F, scl(vel, m.c_glob));
-        F.z += m.grav_force;
-        if (rp.collision) {
-            const double4 c = d.contact[v];
-            F = sub(F, V3<double>{c.x, c.y, c.z});
-        }
-        if (rp.cilia) {  // CiliaForce * Cilia (VX3_Voxel.cu:376), from k_extra_forces
-            const double4 c = d.cfv[v];
-            F = add(F, V3<double>{c.x, c.y, c.z});
-        } else {
-            F = add(F, V3<double>{0.0, 0.0, 0.0});  // no cilia: CiliaForce is 0
-        }
-        if (rp.ff_any) {  // force field (VX3_Voxel.cu:178-184), evaluated by k_extra_forces
-            const double4 ff = d.ffv[v];
-            F.x += ff.x;
-            F.y += ff.y;
-            F.z += ff.z;
-        }
-        V3<double> fric = F;
-        if (floorOn) {  // floorForce (VX3_Voxel.cu:399-426)
-            if (pen >= 0) {
-                const float normal = m.pstiff * pen;
-                F.z += normal - m.c_col * vel.z;
-                if (stat) {
-                    const float surf = (float)(F.x * F.x + F.y * F.y);
-                    const float fr = (m.mu_s * normal) * (m.mu_s * normal);
-                    if (surf > fr) stat = false;
-                } else {
-                    F = sub(F, scl(normalized(V3<double>{vel.x, vel.y, 0}), m.mu_k * normal));
-                }
-            } else {
-                stat = false;
-            }
-        }
-        fric = sub(F, fric);
-        lmv = add(lmv, scl(F, dt));
-        tr = scl(lmv, dt * m.mass_inv);
-        if (floorOn && pen >= 0) {
-            const double work = fric.x * tr.x + fric.y * tr.y;
-            const double hKe = 0.5 * m.mass_inv * (lmv.x * lmv.x + lmv.y * lmv.y);
-            if (hKe + work <= 0) stat = true;
-            if (stat) {
-                lmv.x = lmv.y = 0;
-                tr.x = tr.y = 0;
-            }
-        } else {
-            stat = false;
-        }
-        p.x += tr.x; p.y += tr.y; p.z += tr.z;
-        V3<double> M = qrot(o, Ms);
-        if (xi >= 0) M = add(M, V3<double>{ex.m[0], ex.m[1], ex.m[2]});  // external moment (:393-394)
-        M = sub(M, scl(scl(amv, m.mom_inv), m.c_glob_rot));
-        amv = add(amv, scl(M, dt));
-        Q4<double> on = qmul(from_rotvec(scl(amv, dt * m.mom_inv)), o);
-        if (dof) {  // fixed DOFs (VX3_Voxel.cu:222-257)
-            const short4 l = d.ijk[v];
-            if (dof & 1) { p.x = l.x * m.nom_size + ex.t.x; lmv.x = 0; }
-            if (dof & 2) { p.y = l.y * m.nom_size + ex.t.y; lmv.y = 0; }
-            if (dof & 4) { p.z = l.z * m.nom_size + ex.t.z; lmv.z = 0; }
-            if (dof & EXT_R) {
-                if ((dof & EXT_R) == EXT_R) {  // all rotations: the prescribed orientation
-                    on = Q4<double>{ex.q.x, ex.q.y, ex.q.z, ex.q.w};
-                    amv = V3<double>{0, 0, 0};
-                } else {  // some: zero those components of the rotation vector
-                    V3<double> rv = to_rotvec(on);
-                    if (dof & 8) { rv.x = 0; amv.x = 0; }
-                    if (dof & 16) { rv.y = 0; amv.y = 0; }
-                    if (dof & 32) { rv.z = 0; amv.z = 0; }
-                    on = from_rotvec(rv);
-                }
-            }
-        }
-        d.quat[v] = make_double4(on.w, on.x, on.y, on.z);
-    } else {
-        const Q4<float> o{(float)q.x, (float)q.y, (float)q.z, (float)q.w};
-        V3<float> F = qrot(o, Fs);
-        const V3<float> vel{(float)lm.x * m.mass_inv, (float)lm.y * m.mass_inv, (float)lm.z * m.mass_inv};
-        F = sub(F, scl(vel, m.c_glob));
-        F.z += m.grav_force;
-        if (rp.collision) {
-            const double4 c = d.contact[v];
-            F = sub(F, V3<float>{(float)c.x, (float)c.y, (float)c.z});
-        }
-        if (rp.cilia) {
-            const double4 c = d.cfv[v];
-            F = add(F, V3<float>{(float)c.x, (float)c.y, (float)c.z});
-        }
-        if (rp.ff_any) {
-            const double4 ff = d.ffv[v];
-            F = add(F, V3<float>{(float)ff.x, (float)ff.y, (float)ff.z});
-        }
-        V3<float> fric = F;
-        if (floorOn) {
-            if (pen >= 0) {
-                const float normal = m.pstiff * pen;
-                F.z += normal - m.c_col * vel.z;
-                if (stat) {
-                    if (F.x * F.x + F.y * F.y > (m.mu_s * normal) * (m.mu_s * normal)) stat = false;
-                } else {
-                    F = sub(F, scl(normalized(V3<float>{vel.x, vel.y, 0}), m.mu_k * normal));
-                }
-            } else {
-                stat = false;
-            }
-        }
-        fric = sub(F, fric);
-        lmv.x += (double)F.x * dt; lmv.y += (double)F.y * dt; lmv.z += (double)F.z * dt;
-        tr = scl(lmv, dt * (double)m.mass_inv);
-        if (floorOn && pen >= 0) {
-            const float work = fric.x * (float)tr.x + fric.y * (float)tr.y;
-            const float hKe = 0.5f * m.mass_inv * ((float)lmv.x * (float)lmv.x + (float)lmv.y * (float)lmv.y);
-            if (hKe + work <= 0) stat = true;
-            if (stat) {
-                lmv.x = lmv.y = 0;
-                tr.x = tr.y = 0;
-            }
-        } else {
-            stat = false;
-        }
-        p.x += tr.x; p.y += tr.y; p.z += tr.z;
-        V3<float> M = qrot(o, Ms);
-        const V3<float> avel{(float)am.x * m.mom_inv, (float)am.y * m.mom_inv, (float)am.z * m.mom_inv};
-        M = sub(M, scl(avel, m.c_glob_rot));
-        amv.x += (double)M.x * dt; amv.y += (double)M.y * dt; amv.z += (double)M.z * dt;
-        // q' = dq*q = q + (dq - 1)*q : the small increment in FP32, the sum in FP64
-        const float k = (float)(dt * (double)m.mom_inv);
-        const Q4<float> dq = from_rotvec(V3<float>{(float)amv.x * k, (float)amv.y * k, (float)amv.z * k});
-        const float th2 = dq.x * dq.x + dq.y * dq.y + dq.z * dq.z;
-        const float dw = (dq.w > 0.999f) ? -th2 / (1.0f + dq.w) : dq.w - 1.0f;  // dq.w - 1 without cancellation
-        const Q4<float> delta = qmul(Q4<float>{dw, dq.x, dq.y, dq.z}, o);
-        d.quat[v] = make_double4(q.x + delta.w, q.y + delta.x, q.z + delta.y, q.w + delta.z);
+    const Q4<double> o{q.x, q.y, q.z, q.w};
+    V3<double> F = qrot(o, Fs);
+    if (xi >= 0) F = add(F, V3<double>{ex.f[0], ex.f[1], ex.f[2]});  // external force (:363-364)
+    if (m.c_glob != 0.0f) F = sub(F, scl(scl(lmv, mass_inv), m.c_glob));
+    F.z += widen(m.grav_force);
+    if (rp.collision) {
+        const double4 c = d.contact[v];
+        F = sub(F, V3<double>{c.x, c.y, c.z});
     }
+    if (rp.cilia) {  // CiliaForce * Cilia (VX3_Voxel.cu:376), from k_extra_forces
+        const double4 c = d.cfv[v];
+        F = add(F, V3<double>{c.x, c.y, c.z});
+    }
+    if (rp.ff_any) {  // force field (VX3_Voxel.cu:178-184), evaluated by k_extra_forces
+        const double4 ff = d.ffv[v];
+        F.x += ff.x;
+        F.y += ff.y;
+        F.z += ff.z;
+    }
+    V3<double> fric{0, 0, 0};
+    if (pen >= 0) {  // floorForce (VX3_Voxel.cu:399-426)
+        fric = F;
+        const V3<double> vel = scl(lmv, mass_inv);
+        const float normal = m.pstiff * pen;
+        F.z += normal - m.c_col * vel.z;
+        if (stat) {
+            const float surf = (float)(F.x * F.x + F.y * F.y);
+            const float fr = (m.mu_s * normal) * (m.mu_s * normal);
+            if (surf > fr) stat = false;
+        } else {
+            F = sub(F, scl(normalized(V3<double>{vel.x, vel.y, 0}), m.mu_k * normal));
+        }
+        fric = sub(F, fric);
+    } else if (floorOn) {
+        stat = false;
+    }
+    lmv = add(lmv, scl(F, dt));
+    V3<double> tr = scl(lmv, dt * mass_inv);
+    if (pen >= 0) {
+        const double work = fric.x * tr.x + fric.y * tr.y;
+        const double hKe = 0.5 * m.mass_inv * (lmv.x * lmv.x + lmv.y * lmv.y);
+        if (hKe + work <= 0) stat = true;
+        if (stat) {
+            lmv.x = lmv.y = 0;
+            tr.x = tr.y = 0;
+        }
+    } else {
+        stat = false;
+    }
+    p.x += tr.x; p.y += tr.y; p.z += tr.z;
+    V3<double> M = qrot(o, Ms);
+    if (xi >= 0) M = add(M, V3<double>{ex.m[0], ex.m[1], ex.m[2]});  // external moment (:393-394)
+    if (m.c_glob_rot != 0.0f) M = sub(M, scl(scl(amv, mom_inv), m.c_glob_rot));
+    amv = add(amv, scl(M, dt));
+    Q4<double> on = qmul(from_half_rotvec(scl(amv, 0.5 * (dt * mom_inv))), o);
+    if (dof) {  // fixed DOFs (VX3_Voxel.cu:222-257)
+        const short4 l = d.ijk[v];
+        if (dof & 1) { p.x = l.x * m.nom_size + ex.t.x; lmv.x = 0; }
+        if (dof & 2) { p.y = l.y * m.nom_size + ex.t.y; lmv.y = 0; }
+        if (dof & 4) { p.z = l.z * m.nom_size + ex.t.z; lmv.z = 0; }
+        if (dof & EXT_R) {
+            if ((dof & EXT_R) == EXT_R) {  // all rotations: the prescribed orientation
+                on = Q4<double>{ex.q.x, ex.q.y, ex.q.z, ex.q.w};
+                amv = V3<double>{0, 0, 0};
+            } else {  // some: zero those components of the rotation vector
+                V3<double> rv = to_rotvec(on);
+                if (dof & 8) { rv.x = 0; amv.x = 0; }
+                if (dof & 16) { rv.y = 0; amv.y = 0; }
+                if (dof & 32) { rv.z = 0; amv.z = 0; }
+                on = from_rotvec(rv);
+            }
+        }
+    }
+    d.quat[v] = make_double4(on.w, on.x, on.y, on.z);
     // static friction freezes rotation (VX3_Voxel.cu:259-264), penetration after the move
-    if (floorOn && (float)(bsa / 2 - m.nom_size / 2 - p.z) >= 0 && stat) amv = V3<double>{0, 0, 0};
+    if (stat && !above_floor(bs, m.nom_size, p.z) && floor_penetration(bs, m.nom_size, p.z) >= 0) amv = V3<double>{0, 0, 0};
 
     // next step's temperature; tempe is double-buffered by step parity so that the
     // buffer of the step just taken keeps the value that step used (the reference's tempe)
     if (actuated) {
         float te = tcur[v];
-        p.w = temperature_base_size<EXACT>(rp, m, d.phase[v], tn, bs, &te);
+        p.w = next_base_size(d, rp, m, v, r, parity, tn, bs, &te);
         tnext[v] = te;
     }
     d.pos[v] = p;
@@ -711,11 +820,6 @@ template <class R> __device__ __forceinline__ void voxel_update(const Dev &d, in
     d.angmom[v] = make_double4(amv.x, amv.y, amv.z, 0.0);
     const uint32_t nfl = stat ? (fl | VF_STATIC) : (fl & ~VF_STATIC);
     if (nfl != fl) d.vinfo[v].y = nfl;
-}
-
-template <class R> __global__ void __launch_bounds__(256) k_voxels(Dev d, int parity) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < d.nv) voxel_update<R>(d, v, parity);
 }
 
 }  // namespace vx3g
