@@ -261,6 +261,10 @@ struct vx3g_ctx {
     void *flush = nullptr;
     size_t flush_bytes = 0;
     double *stage = nullptr;  // 4 doubles per voxel: host state exchange
+    std::vector<ResClass> res;  // launches of k_steps_mixed that together step the batch (empty: the passes)
+    std::vector<cudaStream_t> res_stream;
+    cudaEvent_t res_fork = nullptr;
+    std::vector<cudaEvent_t> res_join;
 
     template <class T> int alloc(T **p, size_t n) {
         void *q = nullptr;
@@ -300,6 +304,9 @@ struct vx3g_ctx {
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (side) cudaStreamDestroy(side);
+        for (auto &q : res_stream) cudaStreamDestroy(q);
+        for (auto &q : res_join) cudaEventDestroy(q);
+        if (res_fork) cudaEventDestroy(res_fork);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -352,6 +359,127 @@ int check_math_program(const vx3g_math_token *t, int *len, bool *reads_pos, std:
     return VX3G_ERR_INVALID;
 }
 
+// Whether and how k_steps_mixed steps the batch: mixed precision, whole robots in shared memory.
+// Batches with collisions, force fields, cilia, boundary conditions, signals or a changing link
+// table keep the passes, as does a batch with a robot beyond eight CTAs (about 4,500 voxels).
+// A robot takes the fewest CTAs that hold it in half an SM's shared memory, or one CTA with all of
+// it (two CTAs per SM against one: 1200-voxel robots 80 us a step against 101; but a 360-voxel
+// robot in one large CTA 20.6 us against 24.2 in a cluster of two), and more while the batch
+// leaves SMs idle: down to 96 voxels per CTA (864 voxels: 3.8 us a step in eight CTAs, 5.4 in four;
+// below 96 the cluster barriers cost more than the shorter phases save: 104 voxels 3.0 us in one
+// CTA, 3.4 in two).  Small robots are bundled up to the same measure.
+// lmoff, vmoff: the first link and voxel material of each robot
+int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<int> &vmoff) {
+    const Dev &d = c->d;
+    constexpr int kMost = 8;                 // CTAs of a cluster (portable size)
+    constexpr size_t kHalf = 115000;         // shared memory with which two CTAs share an SM
+    constexpr int kHalfThreads = kResThreads / 2;
+    const int goal = std::max(96, d.nv / (2 * 152));  // voxels per CTA that fill the 152 SMs twice
+    struct Plan {
+        std::vector<ResBundle> b;
+        size_t smem = 0;
+    };
+    Plan by[kMost];
+    auto up = [](int x, int m) { return (x + m - 1) / m * m; };
+    // the first link whose positive end is voxel v or a later one
+    auto link_at = [&](const ResBundle &b, int v) {
+        const auto f = c->ends.begin();
+        return (int)(std::lower_bound(f + b.l0, f + b.l0 + b.nl, v, [](const int2 &e, int x) { return e.y < x; }) - f);
+    };
+    // most entries a CTA's links take axis by axis, with K CTAs
+    auto entries = [&](const ResBundle &b, int K) {
+        int most = 0;
+        for (int j = 0; j < K; j++) {
+            const int a = std::min(b.v0 + j * b.q, b.v0 + b.nv), z = std::min(a + b.q, b.v0 + b.nv);
+            int n[3] = {0, 0, 0};
+            for (int l = link_at(b, a), e = link_at(b, z); l < e; l++) n[c->laxis[l]]++;
+            most = std::max(most, up(n[0], 32) + up(n[1], 32) + up(n[2], 32));
+        }
+        return most;
+    };
+    for (int r = 0; r < c->nr;) {
+        int e = r + 1;
+        while (e < c->nr && e - r < kResRobots && c->voff[e] - c->voff[r] < goal && c->voff[e + 1] - c->voff[r] <= goal * 4 / 3 &&
+               steps_mixed_bytes(up(c->voff[e + 1] - c->voff[r], 16), up(c->loff[e + 1] - c->loff[r], 16) + 96) <= kHalf)
+            e++;
+        ResBundle b{c->voff[r], c->voff[e] - c->voff[r], c->loff[r], c->loff[e] - c->loff[r], r, e - r, 0, 0,
+                    lmoff[r], lmoff[e] - lmoff[r], vmoff[r], vmoff[e] - vmoff[r]};
+        if (b.nlm > kResMats || b.nvm > kResMats) b.nlm = b.nvm = 0;
+        if (b.nv > 65535) return VX3G_OK;  // voxels are numbered in 16 bits
+        int K = 1;
+        bool fits = false;
+        for (; K <= kMost; K++) {
+            b.q = up((b.nv + K - 1) / K, 16);
+            if (b.q > 4096) continue;  // far beyond any CTA
+            b.lc = up(entries(b, K), 16);
+            fits = steps_mixed_bytes(b.q, b.lc) <= (K == 1 || K == kMost ? (size_t)kResSmem : kHalf);
+            if (fits && (b.q <= goal * 4 / 3 || K == kMost)) break;
+        }
+        if (!fits) return VX3G_OK;
+        by[K - 1].b.push_back(b);
+        by[K - 1].smem = std::max(by[K - 1].smem, steps_mixed_bytes(b.q, b.lc));
+        r = e;
+    }
+    CU(init_steps_mixed());
+    for (int K = kMost; K >= 1; K--) {
+        Plan &p = by[K - 1];
+        if (p.b.empty()) continue;
+        // the longest first: the SMs take the rest as they come free
+        std::stable_sort(p.b.begin(), p.b.end(), [](const ResBundle &a, const ResBundle &b) { return a.nl > b.nl; });
+        std::vector<int2> ctas;
+        std::vector<int> order;
+        int lc = 0;
+        for (const ResBundle &b : p.b) {
+            lc = std::max(lc, b.lc);
+            for (int j = 0; j < K; j++) {
+                const int a = std::min(b.v0 + j * b.q, b.v0 + b.nv), z = std::min(a + b.q, b.v0 + b.nv);
+                const int l0 = link_at(b, a), l1 = link_at(b, z), at = (int)order.size();
+                for (uint32_t x = 0; x < 3; x++) {
+                    for (int l = l0; l < l1; l++)
+                        if (c->laxis[l] == x) order.push_back(l);
+                    while ((order.size() - at) % 32) order.push_back(-1);
+                }
+                ctas.push_back(make_int2(at, (int)order.size() - at));
+            }
+        }
+        ResBundle *pb;
+        int2 *pc;
+        int *po, rc;
+        if ((rc = c->upload(&pb, p.b)) || (rc = c->upload(&pc, ctas)) || (rc = c->upload(&po, order))) return rc;
+        CU(cudaStreamSynchronize(c->stream));  // the host vectors end here
+        const int t = std::min(std::max(up(lc, 64), 64), p.smem <= kHalf ? kHalfThreads : kResThreads);
+        c->res.push_back(ResClass{K, t, (int)p.b.size(), p.smem, pb, pc, po});
+    }
+    // the cluster sizes run side by side, the first on the context's own stream
+    if (c->res.size() > 1) {
+        CU(cudaEventCreateWithFlags(&c->res_fork, cudaEventDisableTiming));
+        for (size_t i = 1; i < c->res.size(); i++) {
+            cudaStream_t q;
+            cudaEvent_t e;
+            CU(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+            c->res_stream.push_back(q);
+            CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            c->res_join.push_back(e);
+        }
+    }
+    return VX3G_OK;
+}
+
+// n steps by k_steps_mixed
+int step_resident(vx3g_ctx *c, int n) {
+    const int parity = (int)(c->steps & 1);
+    if (c->res.size() > 1) CU(cudaEventRecord(c->res_fork, c->stream));
+    for (size_t i = 1; i < c->res.size(); i++) {
+        CU(cudaStreamWaitEvent(c->res_stream[i - 1], c->res_fork, 0));
+        CU(launch_steps_mixed(c->d, parity, n, c->res[i], c->res_stream[i - 1]));
+        CU(cudaEventRecord(c->res_join[i - 1], c->res_stream[i - 1]));
+    }
+    CU(launch_steps_mixed(c->d, parity, n, c->res[0], c->stream));
+    for (size_t i = 1; i < c->res.size(); i++) CU(cudaStreamWaitEvent(c->stream, c->res_join[i - 1], 0));
+    c->steps += n;
+    return VX3G_OK;
+}
+
 int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     if (!desc || desc->n_robots <= 0 || !desc->robots) return fail(VX3G_ERR_INVALID, "empty batch descriptor");
     if (desc->precision != VX3G_PRECISION_FP64 && desc->precision != VX3G_PRECISION_MIXED)
@@ -368,6 +496,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     std::vector<VMat> vmats;
     std::vector<LMat> lmats;
     std::vector<int> lrob;  // the robot of each link material
+    std::vector<int> lmoff(c->nr + 1, 0), vmoff(c->nr + 1, 0);  // each robot's first link and voxel material
     bool any_actuated = false;
     std::vector<RobotP> rps(c->nr);
     std::vector<double4> pos, quat;
@@ -719,6 +848,8 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
             }
         }
         lrob.resize(lmats.size(), r);
+        lmoff[r + 1] = (int)lmats.size();
+        vmoff[r + 1] = (int)vmats.size();
         // lists in shared memory when the robot fits (lattice coordinates below 512, packed in 10 bits each)
         int cmax = 0;
         for (int k = 0; k < nvr; k++) {
@@ -812,10 +943,19 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     d.lmatd = nullptr;
     d.act = nullptr;
     d.actv = nullptr;
+    d.nlm = (int)lmats.size();
+    d.nvm = (int)vmats.size();
+    float4 *lrow = nullptr, *vrow = nullptr;
     LMatD *lmatd = nullptr;  // FP64: link constants and actuation phases (filled once the time step is known)
     int *lrob_d = nullptr;
-    if (!d.mixed) {
-        if ((rc = c->alloc(&lmatd, lmats.size())) || (rc = c->upload(&lrob_d, lrob))) return rc;
+    if ((rc = c->upload(&lrob_d, lrob))) return rc;
+    d.lrow = d.vrow = nullptr;
+    if (d.mixed) {
+        if ((rc = c->alloc(&lrow, 4 * lmats.size())) || (rc = c->alloc(&vrow, 3 * vmats.size()))) return rc;
+        d.lrow = lrow;
+        d.vrow = vrow;
+    } else {
+        if ((rc = c->alloc(&lmatd, lmats.size()))) return rc;
         d.lmatd = lmatd;
         if (any_actuated && ((rc = c->alloc(&d.act, 2 * (size_t)d.nr)) || (rc = c->alloc(&d.actv, d.nv)))) return rc;
     }
@@ -918,9 +1058,13 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         c->overlap = true;
     }
 
+    // (c->ends holds the lattice's links alone here: no attachment)
+    if (d.mixed && !d.ns && !d.any_dyn && !c->any_ff && !c->any_cilia && !c->any_bcs && !c->any_signals && (rc = plan_resident(c, lmoff, vmoff)))
+        return rc;
     launch_init_temperature(d, c->precision == VX3G_PRECISION_MIXED, c->stream);
     launch_dt(d, c->scratch, c->stream);
-    if (!d.mixed) launch_fp64_tables(d, lmatd, lrob_d, (int)lmats.size(), c->stream);
+    if (d.mixed) launch_rows_mixed(d, lrow, vrow, lrob_d, c->stream);
+    else launch_fp64_tables(d, lmatd, lrob_d, (int)lmats.size(), c->stream);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(c->stream));
     return VX3G_OK;
@@ -1027,6 +1171,11 @@ void vx3g_destroy(vx3g_ctx *c) { delete c; }
 int vx3g_step(vx3g_ctx *c, int n) {
     if (!c || n < 0) return fail(VX3G_ERR_INVALID, "bad arguments to vx3g_step");
     CU(cudaSetDevice(c->device));
+    while (n > 0 && !c->res.empty()) {
+        const int k = std::min(n, kResSteps);
+        if (int rc = step_resident(c, k)) return rc;
+        n -= k;
+    }
     while (n > 0) {
         const int parity = (int)(c->steps & 1);
         if (n >= c->chunk) {
@@ -1048,7 +1197,7 @@ int vx3g_step(vx3g_ctx *c, int n) {
 
 int vx3g_prepare_graphs(vx3g_ctx *c) {
     if (!c) return fail(VX3G_ERR_INVALID, "null context");
-    if (c->chunk == INT32_MAX) return VX3G_OK;  // graphs off
+    if (c->chunk == INT32_MAX || !c->res.empty()) return VX3G_OK;  // graphs off, or not used (k_steps_mixed)
     CU(cudaSetDevice(c->device));
     cudaGraphExec_t g;
     for (int parity = 0; parity < 2; parity++)

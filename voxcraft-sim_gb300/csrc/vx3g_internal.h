@@ -187,6 +187,9 @@ struct Dev {
     const LMatD *lmatd;
     double4 *act;
     double2 *actv;
+    // mixed contexts: the rows of the nlm link and nvm voxel materials (vx3g_mixed_math.cuh)
+    const float4 *lrow, *vrow;
+    int nlm, nvm;
     // collision
     int *csurf;     // collision surface list (global voxel index), NS entries
     int4 *ccell;    // x: the bucket of a collision-surface voxel in the large-robot grid (-1: not binned)
@@ -298,11 +301,34 @@ extern const LaunchShape kLinkShapes[kMixedShapes], kVoxelShapes[kMixedShapes];
 void launch_links_mixed(const Dev &d, cudaStream_t s, int shape = 0, bool pdl = true);
 // pdl = false when the kernel before it wrote voxel info (detach): no early start
 void launch_voxels_mixed(const Dev &d, int parity, cudaStream_t s, int shape = 0, bool pdl = true);
+// many mixed-precision steps in one launch (k_steps_mixed): bundles of robots, all those of one
+// cluster size in one launch
+struct ResBundle {
+    int v0, nv, l0, nl, r0, nr;  // voxels, links, robots
+    int q, lc;                   // voxels per CTA of the cluster; most links of a CTA (multiples of 16)
+    int lm0, nlm, vm0, nvm;      // its link and voxel materials (count 0: too many for shared memory)
+};
+struct ResClass {
+    int K, threads, count;  // cluster size, threads, bundles
+    size_t smem;            // a CTA's shared memory
+    const ResBundle *bundles;
+    const int2 *ctas;       // per CTA: its first entry in order, entries
+    const int *order;       // links, -1 where an axis is padded to whole warps
+};
+constexpr int kResRobots = 24;         // most robots of a bundle
+constexpr int kResMats = 24;           // most link (and voxel) materials of a bundle kept in shared memory
+constexpr int kResThreads = 768;
+constexpr int kResSteps = 256;         // most steps of one launch (about 20 ms on 1024 robots)
+constexpr int kResSmem = 227 * 1024;   // a CTA's shared memory
+size_t steps_mixed_bytes(int q, int lc);
+cudaError_t init_steps_mixed();
+cudaError_t launch_steps_mixed(const Dev &d, int parity, int n, const ResClass &c, cudaStream_t s);
 void launch_init_temperature(const Dev &d, int mixed, cudaStream_t s);
 // the mixed-precision voxel pass of the voxels with a boundary-condition external (after
 // the main pass, which skips them)
 void launch_voxels_bc_mixed(const Dev &d, int parity, cudaStream_t s);
 void launch_init_temperature_mixed(const Dev &d, cudaStream_t s);
+void launch_rows_mixed(const Dev &d, float4 *lrow, float4 *vrow, const int *lrob, cudaStream_t s);
 void launch_dt(const Dev &d, double *maxfreq2_scratch, cudaStream_t s);
 // surface-voxel collision of one step: displacement check and list rebuild (one
 // cooperative kernel), then the narrow phase

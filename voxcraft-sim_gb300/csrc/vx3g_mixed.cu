@@ -18,85 +18,11 @@
 // The voxel pass restates VX3_Voxel::timeStep (src/VX3/VX3_Voxel.cu:162-277) with the
 // same sums in FP32 and every accumulation (p += F dt, x += p dt/m, L += M dt,
 // q += (dq - 1) q) done as a two-sum into the hi/lo pair.
-#include <math_constants.h>
-
-#include "vx3g_step.cuh"
+#include "vx3g_mixed_math.cuh"
 
 namespace vx3g {
 
-__device__ __forceinline__ void quick_two_sum(float a, float b, float &s, float &e) {
-    s = a + b;
-    e = b - (s - a);
-}
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
-}
-// (hi, lo) += x
-__device__ __forceinline__ void df_add(float &hi, float &lo, float x) {
-    float s, e;
-    two_sum(hi, x, s, e);
-    e += lo;
-    quick_two_sum(s, e, hi, lo);
-}
-// (ah + al) - (bh + bl) to FP32 accuracy: the rounding of ah - bh is at most half an ulp of
-// the difference itself (and none when ah and bh are within a factor 2), so no two-sum is
-// needed when nothing is subtracted from the result afterwards
-__device__ __forceinline__ float df_diff(float ah, float al, float bh, float bl) { return (ah - bh) + (al - bl); }
-// (ah + al) - (bh + bl) - (ch + cl): the axial deviation of a link (a - b ~= c).  The
-// rounding of ah - bh is kept (two-sum): it can be as large as the deviation; s - ch is
-// exact (Sterbenz) while the link's strain lies between -50% and +100%, and otherwise
-// rounds a deviation as large as the rest length
-__device__ __forceinline__ float df_diff3(float ah, float al, float bh, float bl, float ch, float cl) {
-    float s, e;
-    two_sum(ah, -bh, s, e);
-    return (s - ch) + (e + ((al - bl) - cl));
-}
-
-// ToRotationVector (src/VX3/VX3_Quat3D.h:347-359) of a unit quaternion (w, v) in FP32.
-// The reference takes 1 - w^2 as the squared sine of the half angle and, below
-// 2.4e-3 (rotations under about 0.098 rad), does not evaluate the rotation vector
-// 2*acos(w)/sin(theta/2) * v but the approximation 2*sqrt((2 - 2w)/(1 - w^2)) * v =
-// 2*sqrt(2/(1 + w)) * v, which is smaller by about theta^2/96 relative: 2.6e-5 at
-// 0.05 rad, far above FP32 rounding, in every link's bending and torsion terms.  The
-// same two branches are taken here, with 1 - w^2 formed as |v|^2 (no cancellation)
-// and acos(w)/sin as atan2(|v|, w)/|v|.
-__device__ __forceinline__ V3<float> rotvec_f(float w, V3<float> v) {
-    const float s2 = v.x * v.x + v.y * v.y + v.z * v.z;
-    if (!(s2 > 0.0f)) return V3<float>{0, 0, 0};
-    if (s2 < 2.4e-3f) return scl(v, 2.82842712f * rsqrtf(1.0f + w));
-    const float is = rsqrtf(s2);  // s2 >= 2.4e-3 here
-    return scl(v, 2.0f * atan2f(s2 * is, w) * is);
-}
-
-// FromAngleToPosX (src/VX3/VX3_Quat3D.h:384-432) in FP32: the rotation taking r to
-// +x.  The reference forms theta = acos(n.x) for n = r/|r| and returns
-// (cos(theta/2), 0, n.z sin(theta/2)/|(n.y, n.z)|, -n.y sin(theta/2)/|(n.y, n.z)|).
-// With the half-angle identities cos(theta/2) = sqrt((1 + n.x)/2) and
-// sin(theta/2)/|(n.y, n.z)| = sqrt((1 - n.x)/2)/sqrt(1 - n.x^2) = 1/sqrt(2(1 + n.x))
-// that is (c/2, 0, n.z/c, -n.y/c) with c = sqrt(2(1 + n.x)): one square root and one
-// reciprocal instead of acos, sin and cos.  The small-angle shortcut and the
-// turned-around case (theta within 1e-7 of pi, where 1 + n.x underflows in FP32)
-// are the reference's.
-__device__ __forceinline__ Q4<float> from_angle_to_posx_f(Q4<float> q, V3<float> r) {
-    if (r.x == 0 && r.y == 0 && r.z == 0) return q;
-    const float yx = __fdividef(r.y, r.x), zx = __fdividef(r.z, r.x);
-    const float SA = 1.732e-2f;
-    if (yx < SA && yx > -SA && zx < SA && zx > -SA) {
-        q.x = 0;
-        q.y = 0.5f * zx;
-        q.z = -0.5f * yx;
-        q.w = 1 + 0.5f * (-q.y * q.y - q.z * q.z);
-        return q;
-    }
-    const float il = rsqrtf(r.x * r.x + r.y * r.y + r.z * r.z);
-    const float nx = r.x * il, ny = r.y * il, nz = r.z * il;
-    const float t = 2.0f * (1.0f + nx);
-    if (!(t > 0.0f)) return Q4<float>{0, 0, 1, 0};
-    const float ic = rsqrtf(t), c = t * ic;
-    return Q4<float>{0.5f * c, 0, nz * ic, -ny * ic};
-}
+using mx::df_diff;
 
 // ------------------------------------------------------------- collision narrow phase
 // handle_collision_attachment + VX3_Collision::updateContactForce
@@ -210,181 +136,54 @@ __device__ __forceinline__ void links_mixed_body(const Dev &d, int l) {
     const size_t NL = (size_t)d.nl;
     const float4 sa = lsA[l];
     const float2 sb = lsB[l];
-    const V3<float> oldPos2{sa.x, sa.y, sa.z};
     // angle1v is zero while a link is in the small-angle branch (the flag it entered
     // this step with says so); it is read and written only for large-angle links and
     // zeroed once when a link returns to the small branch
     const bool wasSmall = (li.y & LF_SMALL) != 0;
-    V3<float> oldA1{0, 0, 0};
-    if (!wasSmall) oldA1 = V3<float>{lsC[l], lsC[NL + l], lsC[2 * NL + l]};
-    const V3<float> oldA2{sa.w, sb.x, sb.y};
-    float2 sm = d.strain[l];
+    mx::LinkState s{{sa.x, sa.y, sa.z}, {0, 0, 0}, {sa.w, sb.x, sb.y}, d.strain[l], li.y};
+    if (!wasSmall) s.a1v = V3<float>{lsC[l], lsC[NL + l], lsC[2 * NL + l]};
     pdl_wait_then_release();  // the previous voxel pass has moved the endpoints
     const float4 *P = reinterpret_cast<const float4 *>(d.pos);
     const float4 *Q = reinterpret_cast<const float4 *>(d.quat);
-    const float4 pnH = P[2 * e.x], pnL = P[2 * e.x + 1], ppH = P[2 * e.y], ppL = P[2 * e.y + 1];
-    const float4 qnH = Q[2 * e.x], qnL = Q[2 * e.x + 1], qpH = Q[2 * e.y], qpL = Q[2 * e.y + 1];
+    const mx::Ends en{P[2 * e.x], P[2 * e.x + 1], Q[2 * e.x], Q[2 * e.x + 1]};
+    const mx::Ends ep{P[2 * e.y], P[2 * e.y + 1], Q[2 * e.y], Q[2 * e.y + 1]};
     const int r = (int)li.x;
     if (d.status[r] != 0) return;
     const uint32_t fl = li.y;
     if (fl & (LF_BOTH_FIXED | LF_GONE)) return;
     const int axis = fl & LF_AXIS;
-    const LMat &m = d.lmat[fl >> 8];
-
-    // rest length L = 0.5*(bsNeg + bsPos) as a hi/lo pair (VX3_Link::updateRestLength)
-    float Lh, Ll;
-    two_sum(pnH.w, ppH.w, Lh, Ll);
-    Ll += pnL.w + ppL.w;
-    quick_two_sum(0.5f * Lh, 0.5f * Ll, Lh, Ll);
-    // delta = (pPos - pNeg) - L*e_axis in the global frame
-    const float ax = axis == 0 ? Lh : 0.0f, ay = axis == 1 ? Lh : 0.0f, az = axis == 2 ? Lh : 0.0f;
-    const float axl = axis == 0 ? Ll : 0.0f, ayl = axis == 1 ? Ll : 0.0f, azl = axis == 2 ? Ll : 0.0f;
-    const V3<float> delta{df_diff3(ppH.x, ppL.x, pnH.x, pnL.x, ax, axl), df_diff3(ppH.y, ppL.y, pnH.y, pnL.y, ay, ayl),
-                          df_diff3(ppH.z, ppL.z, pnH.z, pnL.z, az, azl)};
-    const Q4<float> a1 = to_axis_xq(axis, Q4<float>{qnH.x, qnH.y, qnH.z, qnH.w});
-    const Q4<float> dq = to_axis_xq(axis, Q4<float>{df_diff(qpH.x, qpL.x, qnH.x, qnL.x), df_diff(qpH.y, qpL.y, qnH.y, qnL.y),
-                                                   df_diff(qpH.z, qpL.z, qnH.z, qnL.z), df_diff(qpH.w, qpL.w, qnH.w, qnL.w)});
-    const Q4<float> c = qconj(a1);
-    const Q4<float> cd = qmul(c, dq);  // angle2 = conj(q1)*q2 = |q1|^2 + conj(q1)*(q2-q1), |q1| = 1
-    const V3<float> rd = qrot(c, to_axis_x(axis, delta));
-    const float L = Lh;
-    float pxm = -2.0f * L * (a1.y * a1.y + a1.z * a1.z) + rd.x;  // pos2.x - L
-    float py = 2.0f * L * (a1.x * a1.y - a1.w * a1.z) + rd.y;
-    float pz = 2.0f * L * (a1.x * a1.z + a1.w * a1.y) + rd.z;
-    const float px = L + pxm;
-    // hysteresis on SmallTurn = (|pz| + |py|)/px and ExtendPerc = |pxm/L| (L > 0),
-    // compared without dividing: px < 0 (bent past 90 degrees) gives SmallTurn <= 0,
-    // px = 0 gives +inf (or NaN when the numerator is 0 too)
-    const float HF = 1.2f, BEND = 0.05f, EXT = 0.50f;
-    const float turn = fabsf(pz) + fabsf(py), ext = fabsf(pxm);
-    const bool turnBelow = px > 0.0f ? turn < BEND * px : px < 0.0f;
-    const bool turnAbove = px > 0.0f ? turn > (HF * BEND) * px : (px == 0.0f && turn > 0.0f);
-    bool small = (fl & LF_SMALL) != 0, lvv = (fl & LF_LVV) != 0;
-    if (!small && turnBelow && ext < EXT * L) {
-        small = true;
-        lvv = false;
-    } else if (small && (turnAbove || ext > (HF * EXT) * L)) {
-        small = false;
-        lvv = false;
+    mx::LinkForces f;
+    bool diverged;
+    mx::link_step(d, mx::link_rows(d.lrow, d.nlm, (int)(fl >> 8)), l, en, ep, s, f, diverged);
+    lsA[l] = make_float4(s.pos2.x, s.pos2.y, s.pos2.z, s.a2v.x);
+    lsB[l] = make_float2(s.a2v.y, s.a2v.z);
+    if (!((s.fl & LF_SMALL) && wasSmall)) {
+        lsC[l] = s.a1v.x; lsC[NL + l] = s.a1v.y; lsC[2 * NL + l] = s.a1v.z;
     }
-    Q4<float> angle1{1, 0, 0, 0};
-    float w2 = 1.0f + cd.w;
-    V3<float> v2{cd.x, cd.y, cd.z};
-    V3<float> pos2;
-    if (small) {
-        pos2 = V3<float>{pxm, py, pz};
-    } else {
-        angle1 = from_angle_to_posx_f(angle1, V3<float>{px, py, pz});
-        const Q4<float> a2 = qmul(angle1, Q4<float>{w2, v2.x, v2.y, v2.z});
-        w2 = a2.w;
-        v2 = V3<float>{a2.x, a2.y, a2.z};
-        const float l2 = px * px + py * py + pz * pz;
-        const float len2 = l2 > 0.0f ? l2 * rsqrtf(l2) : 0.0f;
-        pos2 = V3<float>{__fdividef(pxm * (px + L) + py * py + pz * pz, len2 + L), 0, 0};  // |pos2| - L
-    }
-    const V3<float> a1v = small ? V3<float>{0, 0, 0} : rotvec_f(angle1.w, V3<float>{angle1.x, angle1.y, angle1.z});
-    const V3<float> a2v = rotvec_f(w2, v2);
-    lsA[l] = make_float4(pos2.x, pos2.y, pos2.z, a2v.x);
-    lsB[l] = make_float2(a2v.y, a2v.z);
-    if (!(small && wasSmall)) {
-        lsC[l] = a1v.x; lsC[NL + l] = a1v.y; lsC[2 * NL + l] = a1v.z;
-    }
-
-    const V3<float> dPos2 = scl(sub(pos2, oldPos2), 0.5f);
-    const V3<float> dA1 = scl(sub(a1v, oldA1), 0.5f);
-    const V3<float> dA2 = scl(sub(a2v, oldA2), 0.5f);
-    // FP32 quotients in the hot paths use the hardware reciprocal (__fdividef: within 2 ulp, one
-    // fixed instruction pair, so every launch shape computes the same value)
-    const float axialStrain = __fdividef(pos2.x, L);
-    sm.x = axialStrain;
-    const float stress = link_stress(d, m, l, axialStrain, &sm.y);  // updateStrain (VX3_Link.cu:220-260)
-    d.strain[l] = sm;
-    if (axialStrain > 100) atomicOr(&d.status[r], 1);
-
-    uint32_t nfl = (fl & ~(LF_SMALL | LF_LVV)) | (small ? LF_SMALL : 0u);
-    if (m.eps_fail != -1.0f && sm.y > m.eps_fail) {
-        const V3<float> z{0, 0, 0};
-        store_slot_mx(d, 2 * axis, e.x, z, z);
-        store_slot_mx(d, 2 * axis + 1, e.y, z, z);
-        nfl |= lvv ? LF_LVV : 0u;
-        if (nfl != fl) d.linfo[l].y = nfl;
-        return;
-    }
-    const float b1 = m.b1, b2 = m.b2, b3 = m.b3, a2 = m.a2;
-    V3<float> fNeg{stress * m.area, b1 * pos2.y - b2 * (a1v.z + a2v.z), b1 * pos2.z + b2 * (a1v.y + a2v.y)};
-    V3<float> fPos = neg(fNeg);
-    V3<float> mNeg{a2 * (a2v.x - a1v.x), -b2 * pos2.z - b3 * (2 * a1v.y + a2v.y), b2 * pos2.y - b3 * (2 * a1v.z + a2v.z)};
-    V3<float> mPos{a2 * (a1v.x - a2v.x), -b2 * pos2.z - b3 * (a1v.y + 2 * a2v.y), b2 * pos2.y - b3 * (a1v.z + 2 * a2v.z)};
-    if (lvv) {
-        const V3<float> posCalc{m.sqA1 * dPos2.x, m.sqB1 * dPos2.y - m.sqB2xFMp * (dA1.z + dA2.z),
-                                m.sqB1 * dPos2.z + m.sqB2xFMp * (dA1.y + dA2.y)};
-        // dampingMultiplier / dt, infinite for a Fixed end (its numerator over a zero time step)
-        const float idt = __fdividef(1.0f, d.dt[r]);
-        const float dmN = m.dmcN * (m.fixN ? CUDART_INF_F : idt);
-        const float dmP = m.dmcP * (m.fixP ? CUDART_INF_F : idt);
-        fNeg = add(fNeg, scl(posCalc, dmN));
-        fPos = sub(fPos, scl(posCalc, dmP));
-        mNeg = sub(mNeg, scl(V3<float>{-m.sqA2xIp * (dA2.x - dA1.x), m.sqB2xFMp * dPos2.z + m.sqB3xIp * (2 * dA1.y + dA2.y),
-                                       -m.sqB2xFMp * dPos2.y + m.sqB3xIp * (2 * dA1.z + dA2.z)},
-                             0.5f * dmN));
-        mPos = sub(mPos, scl(V3<float>{m.sqA2xIp * (dA2.x - dA1.x), m.sqB2xFMp * dPos2.z + m.sqB3xIp * (dA1.y + 2 * dA2.y),
-                                       -m.sqB2xFMp * dPos2.y + m.sqB3xIp * (dA1.z + 2 * dA2.z)},
-                             0.5f * dmP));
-    } else {
-        lvv = true;
-    }
-    nfl |= lvv ? LF_LVV : 0u;
-    if (!small) {
-        fNeg = qrotinv(angle1, fNeg);
-        mNeg = qrotinv(angle1, mNeg);
-    }
-    const Q4<float> angle2{w2, v2.x, v2.y, v2.z};
-    fPos = qrotinv(angle2, fPos);
-    mPos = qrotinv(angle2, mPos);
-    store_slot_mx(d, 2 * axis, e.x, to_axis_original(axis, fNeg), to_axis_original(axis, mNeg));
-    store_slot_mx(d, 2 * axis + 1, e.y, to_axis_original(axis, fPos), to_axis_original(axis, mPos));
-    if (fl & LF_RUNTIME) new_link_scale_mx(d, l, 2 * axis, e.x, e.y);
-    if (nfl != fl) d.linfo[l].y = nfl;
+    d.strain[l] = s.strain;
+    if (diverged) atomicOr(&d.status[r], 1);
+    store_slot_mx(d, 2 * axis, e.x, f.fN, f.mN);
+    store_slot_mx(d, 2 * axis + 1, e.y, f.fP, f.mP);
+    if ((fl & LF_RUNTIME) && (s.fl & LF_LVV)) new_link_scale_mx(d, l, 2 * axis, e.x, e.y);
+    if (s.fl != fl) d.linfo[l].y = s.fl;
 }
 
-// base size nomSize*(1 + T*cte) as a hi/lo pair
-__device__ __forceinline__ void base_size_df(const VMat &m, float te, float &hi, float &lo) {
-    const float f = 1 + te * m.cte;
-    const float p = m.nom_hi * f;
-    const float err = fmaf(m.nom_hi, f, -p) + m.nom_lo * f;
-    quick_two_sum(p, err, hi, lo);
+__global__ void k_init_temperature_mixed(Dev d) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= d.nv) return;
+    const uint2 vi = d.vinfo[v];
+    const VMat &m = d.vmat[vi.y >> 8];
+    const RobotP &rp = d.rp[vi.x];
+    float te = d.tempe[v];
+    if (rp.vary_temp && rp.temp_period > 0 && !(m.thermal_on_after > 0.0) && !m.fixed)
+        te = mx::temperature(make_float2(0.0f, 0.0f), d.phc[v], 0.0f, rp.cyc_rate, rp.amp_f, rp.expansion != 0);
+    float4 *P = reinterpret_cast<float4 *>(d.pos);
+    mx::base_size(mx::vox_consts_mx(m), te, P[2 * v].w, P[2 * v + 1].w);
+    d.tempe[v] = te;
+    d.tempe[d.nv + v] = te;
 }
 
-// temperature at the end of a step (gpu_update_temperature, VX3_VoxelyzeKernel.cu:625-650)
-// from the cycles of the phase 2*3.1415926f*(t/P + phase) / (2 pi): the robot's cycles at
-// the step's start tc and the voxel's phase cycles ph, each frac(.) reduced in FP64 once
-// (by the writer of the robot's time, and at create) and held as FP32 hi + lo pairs, plus
-// the step's dt * cycles per second (about 5e-4 cycles, rounded to 3e-11).  The sum c_hi +
-// c_lo is formed with two-sums, and sin(2 pi c) = sin(2 pi c_hi) + 2 pi c_lo cos(2 pi c_hi),
-// the second term dropping (2 pi c_lo)^2 / 2 < 1e-13.  The FP32 sine of a rounded c alone
-// would carry up to 3.7e-7 rad of phase; with the correction the temperature is within
-// about one FP32 rounding of the FP64 step's, and no FP64 arithmetic runs per voxel.
-__device__ __forceinline__ float temperature_mx(const RobotP &rp, float2 tc, float2 ph, float dtf) {
-    float s, e;
-    two_sum(tc.x, ph.x, s, e);
-    s -= floorf(s);  // exact: s lies in [0, 2]
-    e += (tc.y + ph.y) + dtf * rp.cyc_rate;
-    float ch, cl;
-    two_sum(s, e, ch, cl);
-    float sn, cs;
-    sincospif(2.0f * ch, &sn, &cs);
-    float T = rp.amp_f * fmaf(6.28318531f * cl, cs, sn);
-    if (!rp.expansion && T > 0) T = 0;
-    return T;
-}
-
-// frac(c) as an FP32 hi + lo pair
-__device__ __forceinline__ float2 cycles_df(double c) {
-    c -= floor(c);
-    const float h = (float)c;
-    return make_float2(h, (float)(c - (double)h));
-}
-
+// ------------------------------------------------------------ voxel pass
 // The FP64 arithmetic of the mixed voxel pass, kept out of line: if-converted into the
 // pass, it would issue in every warp (GB300 runs FP64 at about 1/64 of the FP32 rate).
 // The robot's time and actuation cycles of the next step (one thread per robot):
@@ -392,7 +191,7 @@ __device__ __noinline__ void advance_time(const Dev &d, const RobotP &rp, int r,
     const double Tcur = d.T[(size_t)parity * d.nr + r];
     const double Tn = (st == 0) ? Tcur + dtf : Tcur;
     d.T[(size_t)(parity ^ 1) * d.nr + r] = Tn;
-    d.tcyc[(size_t)(parity ^ 1) * d.nr + r] = cycles_df(Tn * rp.inv_period * kCycle);
+    d.tcyc[(size_t)(parity ^ 1) * d.nr + r] = mx::cycles_df(Tn * rp.inv_period * kCycle);
 }
 // a material with TurnOnThermalExpansionAfterThisManySeconds > 0: is expansion on at the
 // end of this step?
@@ -400,22 +199,6 @@ __device__ __noinline__ bool thermal_on(const Dev &d, double toa, int r, int par
     return !(toa > d.T[(size_t)parity * d.nr + r] + dtf);
 }
 
-__global__ void k_init_temperature_mixed(Dev d) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= d.nv) return;
-    const uint2 vi = d.vinfo[v];
-    const VMat m = d.vmat[vi.y >> 8];
-    const RobotP &rp = d.rp[vi.x];
-    float te = d.tempe[v];
-    if (rp.vary_temp && rp.temp_period > 0 && !(m.thermal_on_after > 0.0) && !m.fixed)
-        te = temperature_mx(rp, make_float2(0.0f, 0.0f), d.phc[v], 0.0f);
-    float4 *P = reinterpret_cast<float4 *>(d.pos);
-    base_size_df(m, te, P[2 * v].w, P[2 * v + 1].w);
-    d.tempe[v] = te;
-    d.tempe[d.nv + v] = te;
-}
-
-// ------------------------------------------------------------ voxel pass
 // a double as an FP32 hi/lo pair
 __device__ __forceinline__ void set_df(float &hi, float &lo, double x) {
     hi = (float)x;
@@ -434,10 +217,7 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
     float4 *Qa = reinterpret_cast<float4 *>(d.quat);
     float4 *LM = reinterpret_cast<float4 *>(d.linmom);
     float4 *AM = reinterpret_cast<float4 *>(d.angmom);
-    float4 pH = P[2 * v], pL = P[2 * v + 1];
-    float4 qH = Qa[2 * v], qL = Qa[2 * v + 1];
-    float4 lH = LM[2 * v], lL = LM[2 * v + 1];
-    float4 aH = AM[2 * v], aL = AM[2 * v + 1];
+    mx::VoxelState s{P[2 * v], P[2 * v + 1], Qa[2 * v], Qa[2 * v + 1], LM[2 * v], LM[2 * v + 1], AM[2 * v], AM[2 * v + 1]};
     pdl_wait_then_release();  // the link pass (or the contact evaluation) of this step is done
     const int r = (int)vi.x;
     const RobotP &rp = d.rp[r];
@@ -448,23 +228,24 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
     uint32_t fl = vi.y;
     if (fl & VF_FIXED) return;
     if (!BC && rp.bcs && d.vext[v] >= 0) return;  // stepped by the BC pass
-    const VMat m = d.vmat[fl >> 8];
+    const mx::VoxC m = mx::vox_rows(d.vrow, d.nvm, (int)(fl >> 8));
     const bool actuated = rp.vary_temp && rp.temp_period > 0;
     float *tcur = d.tempe + (size_t)parity * d.nv, *tnext = d.tempe + (size_t)(parity ^ 1) * d.nv;
     const int xi = BC ? d.vext[v] : -1;  // boundary-condition external
     const int dof = BC ? d.ext[xi].dof : 0;
+    const double nom = BC ? d.vmat[fl >> 8].nom_size : 0.0;
     if (BC && dtf != 0.0f && dof == EXT_ALL) {  // isFixedAll (VX3_Voxel.cu:167-173)
         const ExtBC &e = d.ext[xi];
         const short4 l = d.ijk[v];
-        set_df(pH.x, pL.x, l.x * m.nom_size + e.t.x);
-        set_df(pH.y, pL.y, l.y * m.nom_size + e.t.y);
-        set_df(pH.z, pL.z, l.z * m.nom_size + e.t.z);
-        set_df(qH.x, qL.x, e.q.x);
-        set_df(qH.y, qL.y, e.q.y);
-        set_df(qH.z, qL.z, e.q.z);
-        set_df(qH.w, qL.w, e.q.w);
-        Qa[2 * v] = qH;
-        Qa[2 * v + 1] = qL;
+        set_df(s.pH.x, s.pL.x, l.x * nom + e.t.x);
+        set_df(s.pH.y, s.pL.y, l.y * nom + e.t.y);
+        set_df(s.pH.z, s.pL.z, l.z * nom + e.t.z);
+        set_df(s.qH.x, s.qL.x, e.q.x);
+        set_df(s.qH.y, s.qL.y, e.q.y);
+        set_df(s.qH.z, s.qL.z, e.q.z);
+        set_df(s.qH.w, s.qL.w, e.q.w);
+        Qa[2 * v] = s.qH;
+        Qa[2 * v + 1] = s.qL;
         const float4 z4 = make_float4(0, 0, 0, 0);
         LM[2 * v] = z4;
         LM[2 * v + 1] = z4;
@@ -483,15 +264,15 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
         }
         bool stat = (fl & VF_STATIC) != 0;
         const bool floorOn = rp.floor != 0;
-        const Q4<float> o{qH.x, qH.y, qH.z, qH.w};
-        V3<float> F = qrot(o, Fs);
+        const Q4<float> o{s.qH.x, s.qH.y, s.qH.z, s.qH.w};
+        V3<float> F = mx::rotate_voxel(o, Fs);
         if (BC) F = add(F, V3<float>{d.ext[xi].f[0], d.ext[xi].f[1], d.ext[xi].f[2]});  // external force
-        const V3<float> vel{(lH.x + lL.x) * m.mass_inv, (lH.y + lL.y) * m.mass_inv, (lH.z + lL.z) * m.mass_inv};
-        F = sub(F, scl(vel, m.c_glob));
-        F.z += m.grav_force;
+        const V3<float> vel = mx::velocity(s.lH, s.lL, m.a.x);
+        F = mx::fma3(-m.a.z, vel, F);
+        F.z = mx::plus(F.z, m.b.y);
         if (rp.collision) {
             const float4 c = reinterpret_cast<const float4 *>(d.contact)[v];
-            F = sub(F, V3<float>{c.x, c.y, c.z});
+            F = mx::diff(F, V3<float>{c.x, c.y, c.z});
         }
         if (rp.cilia) {  // CiliaForce * Cilia (VX3_Voxel.cu:376), evaluated in FP64 by k_extra_forces
             const double4 c = d.cfv[v];
@@ -501,126 +282,56 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
             const double4 ff = d.ffv[v];
             F = add(F, V3<float>{(float)ff.x, (float)ff.y, (float)ff.z});
         }
-        // floor penetration bsa/2 - nom/2 - z with bsa = base size (VX3_Voxel.h:185-188)
-        const float pen = 0.5f * ((pH.w - m.nom_hi) + (pL.w - m.nom_lo)) - (pH.z + pL.z);
-        V3<float> fric = F;
-        if (floorOn) {
-            if (pen >= 0) {
-                const float normal = m.pstiff * pen;
-                F.z += normal - m.c_col * vel.z;
-                if (stat) {
-                    if (F.x * F.x + F.y * F.y > (m.mu_s * normal) * (m.mu_s * normal)) stat = false;
-                } else {
-                    // the horizontal velocity's direction (normalized(): unchanged when zero)
-                    const float h2 = vel.x * vel.x + vel.y * vel.y;
-                    const float k = h2 > 0.0f ? rsqrtf(h2) : 1.0f;
-                    F = sub(F, scl(V3<float>{vel.x * k, vel.y * k, 0}, m.mu_k * normal));
-                }
-            } else {
-                stat = false;
-            }
-        }
-        fric = sub(F, fric);
-        df_add(lH.x, lL.x, F.x * dtf);
-        df_add(lH.y, lL.y, F.y * dtf);
-        df_add(lH.z, lL.z, F.z * dtf);
-        const float km = dtf * m.mass_inv;
-        V3<float> tr{(lH.x + lL.x) * km, (lH.y + lL.y) * km, (lH.z + lL.z) * km};
-        if (floorOn && pen >= 0) {
-            const float lx = lH.x + lL.x, ly = lH.y + lL.y;
-            const float work = fric.x * tr.x + fric.y * tr.y;
-            const float hKe = 0.5f * m.mass_inv * (lx * lx + ly * ly);
-            if (hKe + work <= 0) stat = true;
-            if (stat) {
-                lH.x = lL.x = lH.y = lL.y = 0;
-                tr.x = tr.y = 0;
-            }
-        } else {
-            stat = false;
-        }
-        df_add(pH.x, pL.x, tr.x);
-        df_add(pH.y, pL.y, tr.y);
-        df_add(pH.z, pL.z, tr.z);
-        V3<float> M = qrot(o, Ms);
+        mx::move(s, m, F, vel, floorOn, dtf, stat);
+        V3<float> M = mx::rotate_voxel(o, Ms);
         if (BC) M = add(M, V3<float>{d.ext[xi].m[0], d.ext[xi].m[1], d.ext[xi].m[2]});  // external moment
-        const V3<float> avel{(aH.x + aL.x) * m.mom_inv, (aH.y + aL.y) * m.mom_inv, (aH.z + aL.z) * m.mom_inv};
-        M = sub(M, scl(avel, m.c_glob_rot));
-        df_add(aH.x, aL.x, M.x * dtf);
-        df_add(aH.y, aL.y, M.y * dtf);
-        df_add(aH.z, aL.z, M.z * dtf);
-        // q' = Quat(angMom*dt/I)*q = q + (dq - 1)*q (FromRotationVector, VX3_Quat3D.h:363-377)
-        const float ki = dtf * m.mom_inv;
-        const V3<float> th{0.5f * (aH.x + aL.x) * ki, 0.5f * (aH.y + aL.y) * ki, 0.5f * (aH.z + aL.z) * ki};
-        const float m2 = th.x * th.x + th.y * th.y + th.z * th.z;
-        float dw, sfac;
-        if (m2 * m2 < 5.328e-15f) {
-            dw = -0.5f * m2;
-            sfac = 1.0f - m2 * (1.0f / 6.0f);
-        } else if (m2 < 0.25f) {
-            // |theta| < 0.5 rad: cos|theta| - 1 and sin|theta| / |theta| as their Taylor series in
-            // m2 = |theta|^2, truncated where the next term is below 3e-10 (no square root,
-            // sine or division; the same values to FP32 rounding)
-            dw = m2 * (-0.5f + m2 * (1.0f / 24 + m2 * (-1.0f / 720 + m2 * (1.0f / 40320 - m2 * (1.0f / 3628800)))));
-            sfac = 1.0f + m2 * (-1.0f / 6 + m2 * (1.0f / 120 + m2 * (-1.0f / 5040 + m2 * (1.0f / 362880))));
-        } else {
-            const float im = rsqrtf(m2);  // 1 / |theta|, m2 >= 0.25 here
-            float sn, cs;
-            sincospif(m2 * im * 0.159154943f, &sn, &cs);  // sin, cos of |theta| / 2
-            dw = -2.0f * sn * sn;
-            sfac = 2.0f * sn * cs * im;
-        }
-        const Q4<float> delta = qmul(Q4<float>{dw, th.x * sfac, th.y * sfac, th.z * sfac}, o);
-        df_add(qH.x, qL.x, delta.w);
-        df_add(qH.y, qL.y, delta.x);
-        df_add(qH.z, qL.z, delta.y);
-        df_add(qH.w, qL.w, delta.z);
+        mx::turn(s, m, mx::fma3(-m.a.w, mx::velocity(s.aH, s.aL, fabsf(m.a.y)), M), dtf);
         if (BC && dof) {  // fixed DOFs (VX3_Voxel.cu:222-257), in FP64 on the hi/lo pairs
             const ExtBC &e = d.ext[xi];
             if (dof & EXT_T) {
                 const short4 l = d.ijk[v];
-                if (dof & 1) { set_df(pH.x, pL.x, l.x * m.nom_size + e.t.x); lH.x = lL.x = 0; }
-                if (dof & 2) { set_df(pH.y, pL.y, l.y * m.nom_size + e.t.y); lH.y = lL.y = 0; }
-                if (dof & 4) { set_df(pH.z, pL.z, l.z * m.nom_size + e.t.z); lH.z = lL.z = 0; }
+                if (dof & 1) { set_df(s.pH.x, s.pL.x, l.x * nom + e.t.x); s.lH.x = s.lL.x = 0; }
+                if (dof & 2) { set_df(s.pH.y, s.pL.y, l.y * nom + e.t.y); s.lH.y = s.lL.y = 0; }
+                if (dof & 4) { set_df(s.pH.z, s.pL.z, l.z * nom + e.t.z); s.lH.z = s.lL.z = 0; }
             }
             if ((dof & EXT_R) == EXT_R) {  // all rotations: the prescribed orientation
-                set_df(qH.x, qL.x, e.q.x);
-                set_df(qH.y, qL.y, e.q.y);
-                set_df(qH.z, qL.z, e.q.z);
-                set_df(qH.w, qL.w, e.q.w);
-                aH.x = aH.y = aH.z = aL.x = aL.y = aL.z = 0;
+                set_df(s.qH.x, s.qL.x, e.q.x);
+                set_df(s.qH.y, s.qL.y, e.q.y);
+                set_df(s.qH.z, s.qL.z, e.q.z);
+                set_df(s.qH.w, s.qL.w, e.q.w);
+                s.aH.x = s.aH.y = s.aH.z = s.aL.x = s.aL.y = s.aL.z = 0;
             } else if (dof & EXT_R) {  // some: those rotation-vector components zeroed
-                V3<double> rv = to_rotvec(Q4<double>{(double)qH.x + qL.x, (double)qH.y + qL.y, (double)qH.z + qL.z,
-                                                     (double)qH.w + qL.w});
-                if (dof & 8) { rv.x = 0; aH.x = aL.x = 0; }
-                if (dof & 16) { rv.y = 0; aH.y = aL.y = 0; }
-                if (dof & 32) { rv.z = 0; aH.z = aL.z = 0; }
+                V3<double> rv = to_rotvec(Q4<double>{(double)s.qH.x + s.qL.x, (double)s.qH.y + s.qL.y,
+                                                     (double)s.qH.z + s.qL.z, (double)s.qH.w + s.qL.w});
+                if (dof & 8) { rv.x = 0; s.aH.x = s.aL.x = 0; }
+                if (dof & 16) { rv.y = 0; s.aH.y = s.aL.y = 0; }
+                if (dof & 32) { rv.z = 0; s.aH.z = s.aL.z = 0; }
                 const Q4<double> q = from_rotvec(rv);
-                set_df(qH.x, qL.x, q.w);
-                set_df(qH.y, qL.y, q.x);
-                set_df(qH.z, qL.z, q.y);
-                set_df(qH.w, qL.w, q.z);
+                set_df(s.qH.x, s.qL.x, q.w);
+                set_df(s.qH.y, s.qL.y, q.x);
+                set_df(s.qH.z, s.qL.z, q.y);
+                set_df(s.qH.w, s.qL.w, q.z);
             }
         }
-        const float pen2 = 0.5f * ((pH.w - m.nom_hi) + (pL.w - m.nom_lo)) - (pH.z + pL.z);
-        if (floorOn && pen2 >= 0 && stat) aH.x = aH.y = aH.z = aL.x = aL.y = aL.z = 0;
+        if (floorOn && mx::penetration(s, m) >= 0 && stat) s.aH.x = s.aH.y = s.aH.z = s.aL.x = s.aL.y = s.aL.z = 0;
         const uint32_t nfl = stat ? (fl | VF_STATIC) : (fl & ~VF_STATIC);
         if (nfl != fl) d.vinfo[v].y = nfl;
-        Qa[2 * v] = qH;
-        Qa[2 * v + 1] = qL;
-        LM[2 * v] = lH;
-        LM[2 * v + 1] = lL;
-        AM[2 * v] = aH;
-        AM[2 * v + 1] = aL;
+        Qa[2 * v] = s.qH;
+        Qa[2 * v + 1] = s.qL;
+        LM[2 * v] = s.lH;
+        LM[2 * v + 1] = s.lL;
+        AM[2 * v] = s.aH;
+        AM[2 * v + 1] = s.aL;
     }
     if (actuated) {  // next step's temperature and base size
         float te = tcur[v];
-        if (!m.toa_pos || thermal_on(d, m.thermal_on_after, r, parity, dtf))
-            te = temperature_mx(rp, d.tcyc[(size_t)parity * d.nr + r], d.phc[v], dtf);
-        base_size_df(m, te, pH.w, pL.w);
+        if (m.a.y > 0.0f || thermal_on(d, d.vmat[fl >> 8].thermal_on_after, r, parity, dtf))
+            te = mx::temperature(d.tcyc[(size_t)parity * d.nr + r], d.phc[v], dtf, rp.cyc_rate, rp.amp_f, rp.expansion != 0);
+        mx::base_size(m, te, s.pH.w, s.pL.w);
         tnext[v] = te;
     }
-    P[2 * v] = pH;
-    P[2 * v + 1] = pL;
+    P[2 * v] = s.pH;
+    P[2 * v + 1] = s.pL;
 }
 
 // the voxels with a boundary-condition external, after the main voxel pass
@@ -685,6 +396,343 @@ void launch_voxels_mixed(const Dev &d, int parity, cudaStream_t s, int shape, bo
         case 5: launch_pdl(k_voxels_mixed<64, 16>, d.nv, 64, s, pdl, d, parity); break;
         default: launch_pdl(k_voxels_mixed<256, 1>, d.nv, 256, s, pdl, d, parity); break;
     }
+}
+// ------------------------------------------------------------ many steps in one launch
+// The link and voxel passes are bound by the latency of their dependent loads, and on a batch
+// beyond the L2 by HBM (1024 robots, 7.1e5 voxels: 120 us a step, of which 76 us are the bytes at
+// the copy rate; issue slots 25% used).  Robots never touch each other, so here a cluster of CTAs
+// keeps a bundle of whole robots in its shared memory and takes n steps there: nothing leaves
+// the cluster between steps.  A CTA owns a contiguous range of q voxels of the bundle and the
+// links whose positive end is among them (links are made in the voxel order of that end); the
+// negative end may be in a CTA of lower rank, reached through distributed shared memory.  Two
+// barriers per step: after the links (forces written to the six rows of each end) and after the
+// voxels.  Bound by instruction issue and the two phases' dependency chains: 62% of the issue
+// slots used, 83 us a step on those 1024 robots; 2.7 us instead of 5.9 on one robot of 104 voxels.
+// Two CTAs of 384 threads per SM (113 KB each), so that one's loads overlap the other's
+// arithmetic: 1200-voxel robots 80 us a step against 101 with one CTA of 768 threads.
+struct ResRobot {
+    double T[2];     // time by parity
+    float2 tc[2];    // actuation cycles by parity
+    double inv_period;
+    float dt, cyc_rate, amp;
+    int status, actuated, expansion, floor;
+};
+// A CTA's arrays, all computed from q (voxels) and lc (links), multiples of 16.  Float4 planes of q:
+// position hi, lo, orientation hi, lo, six force rows; then the link and material rows and the
+// robots; then float2, float and byte planes.
+struct ResSmem {
+    int q, lc;
+    __device__ __forceinline__ static float4 *base() {
+        extern __shared__ float4 rsm[];
+        return rsm;
+    }
+    __device__ __forceinline__ float4 &PH(int i) const { return base()[i]; }
+    __device__ __forceinline__ float4 &PL(int i) const { return base()[q + i]; }
+    __device__ __forceinline__ float4 &QH(int i) const { return base()[2 * q + i]; }
+    __device__ __forceinline__ float4 &QL(int i) const { return base()[3 * q + i]; }
+    __device__ __forceinline__ float4 &SA(int dir, int i) const { return base()[(4 + dir) * q + i]; }
+    __device__ __forceinline__ float4 &LA(int i) const { return base()[10 * q + i]; }
+    __device__ __forceinline__ float4 &lrow(int i) const { return base()[10 * q + lc + i]; }
+    __device__ __forceinline__ float4 &vrow(int i) const { return base()[10 * q + lc + 4 * kResMats + i]; }
+    __device__ __forceinline__ ResRobot &rob(int i) const {
+        return reinterpret_cast<ResRobot *>(base() + 10 * q + lc + 7 * kResMats)[i];
+    }
+    __device__ __forceinline__ float2 *f2() const {
+        return reinterpret_cast<float2 *>(base() + 10 * q + lc + 7 * kResMats + kResRobots * sizeof(ResRobot) / 16);
+    }
+    __device__ __forceinline__ float2 &SB(int dir, int i) const { return f2()[dir * q + i]; }
+    __device__ __forceinline__ float2 &ph(int i) const { return f2()[6 * q + i]; }
+    __device__ __forceinline__ float2 &LB(int i) const { return f2()[7 * q + i]; }
+    __device__ __forceinline__ float2 &ST(int i) const { return f2()[7 * q + lc + i]; }
+    __device__ __forceinline__ float *f1() const { return reinterpret_cast<float *>(f2() + 7 * q + 2 * lc); }
+    __device__ __forceinline__ float &mom(int k, int i) const { return f1()[k * q + i]; }  // linear hi, lo, angular hi, lo
+    __device__ __forceinline__ float &te(int i) const { return f1()[12 * q + i]; }
+    __device__ __forceinline__ uint32_t &vi(int i) const { return reinterpret_cast<uint32_t *>(f1())[13 * q + i]; }
+    __device__ __forceinline__ float &LC(int k, int i) const { return f1()[14 * q + k * lc + i]; }
+    __device__ __forceinline__ uint32_t &fl(int i) const { return reinterpret_cast<uint32_t *>(f1())[14 * q + 3 * lc + i]; }
+    __device__ __forceinline__ uint32_t &le(int i) const { return reinterpret_cast<uint32_t *>(f1())[14 * q + 4 * lc + i]; }  // ends in the bundle
+    __device__ __forceinline__ unsigned char &rb(int i) const {  // robot in the bundle
+        return reinterpret_cast<unsigned char *>(f1() + 14 * q + 5 * lc)[i];
+    }
+};
+static_assert(sizeof(ResRobot) * kResRobots % 16 == 0, "alignment of the arrays after the robots");
+static_assert(kResRobots <= 32, "one bit per robot of a bundle");
+size_t steps_mixed_bytes(int q, int lc) {
+    return (size_t)q * (10 * 16 + 7 * 8 + 14 * 4 + 1) + (size_t)lc * (16 + 2 * 8 + 5 * 4) + kResRobots * sizeof(ResRobot) +
+           kResMats * 7 * 16;
+}
+
+template <bool CLUSTER> __device__ __forceinline__ void res_sync() {
+    if (CLUSTER) asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    else __syncthreads();
+}
+// the address in the shared memory of cluster rank k of what p points to in this CTA's
+template <class T> __device__ __forceinline__ T *res_map(T *p, int k) {
+    T *q;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(k));
+    return q;
+}
+
+template <bool CLUSTER>
+__device__ __forceinline__ void res_link(const Dev &d, const ResSmem &S, const ResBundle &B, int i, const int *lid, int rank, int K) {
+    const uint32_t fl = S.fl(i);
+    if (fl & (LF_BOTH_FIXED | LF_GONE)) return;
+    const int q = B.q, vb = rank * q, axis = (int)(fl & LF_AXIS);
+    const uint32_t e = S.le(i);
+    const int ip = (int)(e >> 16) - vb;
+    int in = (int)(e & 0xffffu) - vb, own = rank;
+    ResRobot &R = S.rob(S.rb(ip));
+    if (R.status != 0) return;
+    if (CLUSTER && in < 0) {  // the negative end is in a CTA of lower rank
+        own = (int)(e & 0xffffu) / q;
+        in = (int)(e & 0xffffu) - own * q;
+    }
+    mx::Ends en;
+    if (CLUSTER && own != rank)
+        en = mx::Ends{*res_map(&S.PH(in), own), *res_map(&S.PL(in), own), *res_map(&S.QH(in), own), *res_map(&S.QL(in), own)};
+    else en = mx::Ends{S.PH(in), S.PL(in), S.QH(in), S.QL(in)};
+    const mx::Ends ep{S.PH(ip), S.PL(ip), S.QH(ip), S.QL(ip)};
+    const float4 sa = S.LA(i);
+    const float2 sb = S.LB(i);
+    const bool wasSmall = (fl & LF_SMALL) != 0;
+    mx::LinkState st{{sa.x, sa.y, sa.z}, {0, 0, 0}, {sa.w, sb.x, sb.y}, S.ST(i), fl};
+    if (!wasSmall) st.a1v = V3<float>{S.LC(0, i), S.LC(1, i), S.LC(2, i)};
+    mx::LinkForces f;
+    bool diverged;
+    const int lm = (int)(fl >> 8);
+    mx::link_step(d, B.nlm ? mx::link_rows(&S.lrow(0), B.nlm, lm - B.lm0) : mx::link_rows(d.lrow, d.nlm, lm), *lid, en, ep, st, f,
+                  diverged);
+    S.LA(i) = make_float4(st.pos2.x, st.pos2.y, st.pos2.z, st.a2v.x);
+    S.LB(i) = make_float2(st.a2v.y, st.a2v.z);
+    if (!((st.fl & LF_SMALL) && wasSmall)) S.LC(0, i) = st.a1v.x, S.LC(1, i) = st.a1v.y, S.LC(2, i) = st.a1v.z;
+    S.ST(i) = st.strain;
+    S.fl(i) = st.fl;
+    const float4 na = make_float4(f.fN.x, f.fN.y, f.fN.z, f.mN.x);
+    const float2 nb = make_float2(f.mN.y, f.mN.z);
+    if (CLUSTER && own != rank) *res_map(&S.SA(2 * axis, in), own) = na, *res_map(&S.SB(2 * axis, in), own) = nb;
+    else S.SA(2 * axis, in) = na, S.SB(2 * axis, in) = nb;
+    S.SA(2 * axis + 1, ip) = make_float4(f.fP.x, f.fP.y, f.fP.z, f.mP.x);
+    S.SB(2 * axis + 1, ip) = make_float2(f.mP.y, f.mP.z);
+    if (diverged) {
+        atomicOr(&d.status[B.r0 + S.rb(ip)], 1);
+        if (!CLUSTER) atomicOr(&R.status, 1);
+        else
+            for (int k = 0; k < K; k++) atomicOr(res_map(&R.status, k), 1);
+    }
+}
+
+__device__ __forceinline__ void res_voxel(const Dev &d, const ResSmem &S, const ResBundle &B, int i, int v, int parity, bool last) {
+    const uint32_t fl = S.vi(i);
+    const ResRobot &R = S.rob(S.rb(i));
+    if (R.status != 0 || (fl & VF_FIXED)) return;
+    const float dtf = R.dt;
+    const mx::VoxC m = B.nvm ? mx::vox_rows(&S.vrow(0), B.nvm, (int)(fl >> 8) - B.vm0) : mx::vox_rows(d.vrow, d.nvm, (int)(fl >> 8));
+    mx::VoxelState s;
+    s.pH = S.PH(i), s.pL = S.PL(i);
+    if (dtf != 0.0f) {
+        s.qH = S.QH(i), s.qL = S.QL(i);
+        s.lH = make_float4(S.mom(0, i), S.mom(1, i), S.mom(2, i), 0.0f);
+        s.lL = make_float4(S.mom(3, i), S.mom(4, i), S.mom(5, i), 0.0f);
+        s.aH = make_float4(S.mom(6, i), S.mom(7, i), S.mom(8, i), 0.0f);
+        s.aL = make_float4(S.mom(9, i), S.mom(10, i), S.mom(11, i), 0.0f);
+        V3<float> Fs{0, 0, 0}, Ms{0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < 6; k++)
+            if (fl & (1u << k)) {
+                const float4 a = S.SA(k, i);
+                const float2 b = S.SB(k, i);
+                Fs = V3<float>{mx::plus(Fs.x, a.x), mx::plus(Fs.y, a.y), mx::plus(Fs.z, a.z)};
+                Ms = V3<float>{mx::plus(Ms.x, a.w), mx::plus(Ms.y, b.x), mx::plus(Ms.z, b.y)};
+            }
+        bool stat = (fl & VF_STATIC) != 0;
+        const Q4<float> o{s.qH.x, s.qH.y, s.qH.z, s.qH.w};
+        const V3<float> vel = mx::velocity(s.lH, s.lL, m.a.x);
+        V3<float> F = mx::fma3(-m.a.z, vel, mx::rotate_voxel(o, Fs));
+        F.z = mx::plus(F.z, m.b.y);
+        mx::move(s, m, F, vel, R.floor != 0, dtf, stat);
+        mx::turn(s, m, mx::fma3(-m.a.w, mx::velocity(s.aH, s.aL, fabsf(m.a.y)), mx::rotate_voxel(o, Ms)), dtf);
+        if (R.floor && mx::penetration(s, m) >= 0 && stat) s.aH = s.aL = make_float4(0, 0, 0, 0);
+        const uint32_t nfl = stat ? (fl | VF_STATIC) : (fl & ~VF_STATIC);
+        if (nfl != fl) S.vi(i) = nfl;
+        S.QH(i) = s.qH, S.QL(i) = s.qL;
+        const float w[12] = {s.lH.x, s.lH.y, s.lH.z, s.lL.x, s.lL.y, s.lL.z, s.aH.x, s.aH.y, s.aH.z, s.aL.x, s.aL.y, s.aL.z};
+#pragma unroll
+        for (int k = 0; k < 12; k++) S.mom(k, i) = w[k];
+    }
+    if (R.actuated) {  // next step's temperature and base size
+        float te = S.te(i);
+        if (last) d.tempe[(size_t)parity * d.nv + v] = te;  // the temperature the last step used
+        if (m.a.y > 0.0f || !(d.vmat[fl >> 8].thermal_on_after > R.T[parity] + dtf))
+            te = mx::temperature(R.tc[parity], S.ph(i), dtf, R.cyc_rate, R.amp, R.expansion != 0);
+        mx::base_size(m, te, s.pH.w, s.pL.w);
+        S.te(i) = te;
+    }
+    S.PH(i) = s.pH, S.PL(i) = s.pL;
+}
+
+// bundles, one per cluster; ctas: the first entry and the entries in `order` of each CTA's links,
+// axis by axis, each axis filled up to whole warps with -1
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kResThreads, 1) k_steps_mixed(Dev d, int parity, int n, const ResBundle *bundles, const int2 *ctas,
+                                                                const int *order) {
+    int rank = 0, K = 1;
+    if (CLUSTER) {
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(K));
+    }
+    const ResBundle B = bundles[blockIdx.x / K];
+    const int q = B.q;
+    const ResSmem S{q, B.lc};
+    const int tid = threadIdx.x, T = blockDim.x;
+    const int vb = rank * q, nv = max(0, min(q, B.nv - vb)), v0 = B.v0 + vb;  // this CTA's voxels
+    const int nl = ctas[blockIdx.x].y;
+    const int *lid = order + ctas[blockIdx.x].x;
+    const float4 *P = reinterpret_cast<const float4 *>(d.pos), *Qa = reinterpret_cast<const float4 *>(d.quat);
+    const float4 *LM = reinterpret_cast<const float4 *>(d.linmom), *AM = reinterpret_cast<const float4 *>(d.angmom);
+    for (int i = tid; i < nv; i += T) {
+        const int v = v0 + i;
+        S.PH(i) = P[2 * v], S.PL(i) = P[2 * v + 1], S.QH(i) = Qa[2 * v], S.QL(i) = Qa[2 * v + 1];
+        const float4 a = LM[2 * v], b = LM[2 * v + 1], c = AM[2 * v], e = AM[2 * v + 1];
+        const float m[12] = {a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z, e.x, e.y, e.z};
+#pragma unroll
+        for (int k = 0; k < 12; k++) S.mom(k, i) = m[k];
+        const uint2 vi = d.vinfo[v];
+        S.vi(i) = vi.y;
+        S.rb(i) = (unsigned char)((int)vi.x - B.r0);
+        S.ph(i) = d.phc[v];
+        S.te(i) = d.tempe[(size_t)parity * d.nv + v];
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            S.SA(k, i) = make_float4(0, 0, 0, 0);
+            S.SB(k, i) = make_float2(0, 0);
+        }
+    }
+    for (int i = tid; i < nl; i += T) {
+        const int l = lid[i];
+        S.fl(i) = LF_GONE;
+        if (l < 0) continue;
+        S.LA(i) = mixed_lstate_a(d)[l];
+        S.LB(i) = mixed_lstate_b(d)[l];
+        S.ST(i) = d.strain[l];
+        const uint32_t fl = d.linfo[l].y;
+        S.fl(i) = fl;
+        const int2 e = d.ends[l];
+        S.le(i) = (uint32_t)(e.x - B.v0) | (uint32_t)(e.y - B.v0) << 16;
+        if (!(fl & LF_SMALL))
+            for (int k = 0; k < 3; k++) S.LC(k, i) = mixed_lstate_c(d)[(size_t)k * d.nl + l];
+    }
+    for (int i = tid; i < 4 * B.nlm; i += T) S.lrow(i) = d.lrow[(size_t)(i / B.nlm) * d.nlm + B.lm0 + i % B.nlm];
+    for (int i = tid; i < 3 * B.nvm; i += T) S.vrow(i) = d.vrow[(size_t)(i / B.nvm) * d.nvm + B.vm0 + i % B.nvm];
+    for (int i = tid; i < B.nr; i += T) {
+        const int r = B.r0 + i;
+        const RobotP &rp = d.rp[r];
+        ResRobot R;
+        for (int k = 0; k < 2; k++) R.T[k] = d.T[(size_t)k * d.nr + r], R.tc[k] = d.tcyc[(size_t)k * d.nr + r];
+        R.inv_period = rp.inv_period;
+        R.dt = rp.nv ? d.dt[r] : 0.0f;  // a robot without voxels stays at its time
+        R.cyc_rate = rp.cyc_rate, R.amp = rp.amp_f;
+        R.status = d.status[r];
+        R.actuated = rp.vary_temp && rp.temp_period > 0;
+        R.expansion = rp.expansion, R.floor = rp.floor;
+        S.rob(i) = R;
+    }
+    res_sync<CLUSTER>();
+    unsigned stopped = 0;  // robots that were not running when the launch began
+    for (int i = 0; i < B.nr; i++) stopped |= (unsigned)(S.rob(i).status != 0) << i;
+    if (CLUSTER) res_sync<CLUSTER>();  // before any CTA can mark a robot in another's copy
+    for (int s = 0; s < n; s++, parity ^= 1) {
+        for (int i = tid; i < nl; i += T) res_link<CLUSTER>(d, S, B, i, lid + i, rank, K);
+        res_sync<CLUSTER>();
+        for (int i = tid; i < nv; i += T) res_voxel(d, S, B, i, v0 + i, parity, s == n - 1);
+        // the robots' time and actuation cycles
+        for (int i = T - 1 - tid; i < B.nr; i += T) {
+            ResRobot &R = S.rob(i);
+            const double Tn = R.status == 0 ? R.T[parity] + R.dt : R.T[parity];
+            R.T[parity ^ 1] = Tn;
+            R.tc[parity ^ 1] = mx::cycles_df(Tn * R.inv_period * kCycle);
+        }
+        res_sync<CLUSTER>();
+    }
+    float4 *Po = reinterpret_cast<float4 *>(d.pos), *Qo = reinterpret_cast<float4 *>(d.quat);
+    float4 *Lo = reinterpret_cast<float4 *>(d.linmom), *Ao = reinterpret_cast<float4 *>(d.angmom);
+    float4 *ga = reinterpret_cast<float4 *>(d.slots);
+    float2 *gb = reinterpret_cast<float2 *>(ga + 6 * (size_t)d.nv);
+    for (int i = tid; i < nv; i += T) {
+        const int v = v0 + i, r = S.rb(i);
+        const uint32_t fl = S.vi(i);
+        if ((stopped >> r) & 1u) continue;
+        if (!(fl & VF_FIXED)) {
+            Po[2 * v] = S.PH(i), Po[2 * v + 1] = S.PL(i), Qo[2 * v] = S.QH(i), Qo[2 * v + 1] = S.QL(i);
+            Lo[2 * v] = make_float4(S.mom(0, i), S.mom(1, i), S.mom(2, i), 0.0f);
+            Lo[2 * v + 1] = make_float4(S.mom(3, i), S.mom(4, i), S.mom(5, i), 0.0f);
+            Ao[2 * v] = make_float4(S.mom(6, i), S.mom(7, i), S.mom(8, i), 0.0f);
+            Ao[2 * v + 1] = make_float4(S.mom(9, i), S.mom(10, i), S.mom(11, i), 0.0f);
+            d.vinfo[v].y = fl;
+            if (S.rob(r).actuated) {
+                d.tempe[(size_t)parity * d.nv + v] = S.te(i);
+                if (S.rob(r).status != 0) d.tempe[(size_t)(parity ^ 1) * d.nv + v] = S.te(i);  // diverged on the way
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++)
+            if (fl & (1u << k)) {
+                ga[(size_t)k * d.nv + v] = S.SA(k, i);
+                gb[(size_t)k * d.nv + v] = S.SB(k, i);
+            }
+    }
+    for (int i = tid; i < nl; i += T) {
+        const int l = lid[i];
+        if (l < 0) continue;
+        const int ip = (int)(S.le(i) >> 16) - vb;
+        if ((stopped >> S.rb(ip)) & 1u) continue;
+        mixed_lstate_a(d)[l] = S.LA(i);
+        mixed_lstate_b(d)[l] = S.LB(i);
+        d.strain[l] = S.ST(i);
+        const uint32_t fl = S.fl(i);
+        for (int k = 0; k < 3; k++) mixed_lstate_c(d)[(size_t)k * d.nl + l] = (fl & LF_SMALL) ? 0.0f : S.LC(k, i);
+        d.linfo[l].y = fl;
+    }
+    if (rank == 0)
+        for (int i = tid; i < B.nr; i += T)
+            for (int k = 0; k < 2; k++) d.T[(size_t)k * d.nr + B.r0 + i] = S.rob(i).T[k], d.tcyc[(size_t)k * d.nr + B.r0 + i] = S.rob(i).tc[k];
+}
+
+cudaError_t init_steps_mixed() {
+    cudaError_t e = cudaFuncSetAttribute(k_steps_mixed<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_steps_mixed<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
+    return e;
+}
+
+cudaError_t launch_steps_mixed(const Dev &d, int parity, int n, const ResClass &c, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(c.count * c.K));
+    cfg.blockDim = dim3((unsigned)c.threads);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)c.K;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = c.K > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, c.K > 1 ? k_steps_mixed<true> : k_steps_mixed<false>, d, parity, n, c.bundles, c.ctas, c.order);
+}
+
+// the material rows (lrob: the robot of each link material), once the time step is known
+__global__ void k_rows_mixed(Dev d, float4 *lrow, float4 *vrow, const int *lrob) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < d.nlm) {
+        const mx::LinkC c = mx::link_consts_mx(d.lmat[i], d.dt[lrob[i]]);
+        lrow[i] = c.a, lrow[d.nlm + i] = c.b, lrow[2 * (size_t)d.nlm + i] = c.c, lrow[3 * (size_t)d.nlm + i] = c.e;
+    }
+    if (i < d.nvm) {
+        const mx::VoxC c = mx::vox_consts_mx(d.vmat[i]);
+        vrow[i] = c.a, vrow[d.nvm + i] = c.b, vrow[2 * (size_t)d.nvm + i] = c.c;
+    }
+}
+void launch_rows_mixed(const Dev &d, float4 *lrow, float4 *vrow, const int *lrob, cudaStream_t s) {
+    const int n = d.nlm > d.nvm ? d.nlm : d.nvm;
+    if (n) k_rows_mixed<<<(n + 127) / 128, 128, 0, s>>>(d, lrow, vrow, lrob);
 }
 void launch_init_temperature_mixed(const Dev &d, cudaStream_t s) {
     if (d.nv) k_init_temperature_mixed<<<(d.nv + 255) / 256, 256, 0, s>>>(d);
