@@ -183,7 +183,8 @@ __global__ void k_extra_forces(Dev d, int parity) {
 }
 
 void launch_extra_forces(const Dev &d, int parity, cudaStream_t s) {
-    if ((d.ffv || d.cfv) && d.nv) k_extra_forces<<<(d.nv + 255) / 256, 256, 0, s>>>(d, parity);
+    const int t = fp64_threads(d.nv, 256);
+    if ((d.ffv || d.cfv) && d.nv) k_extra_forces<<<(d.nv + t - 1) / t, t, 0, s>>>(d, parity);
 }
 
 // ---------------------------------------------------------------- signals
@@ -384,19 +385,6 @@ __device__ __forceinline__ float4 pos_f(const Dev &d, int v) {
     return make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
 }
 
-// robot r's lists are rebuilt this step; the first voxel to say so puts a robot of the
-// shared-memory path on the work list of coll_list_robots
-__device__ __forceinline__ void flag_robot(const Dev &d, int r) {
-    if (*(volatile int *)&d.cflag[1 + r]) return;
-    if (atomicOr(&d.cflag[1 + r], 1) != 0) return;
-    atomicOr(d.cflag, 1);
-    const int k = d.rp[r].lchunks;
-    if (k) {
-        const unsigned long long old = atomicAdd(d.lwork_ctr, (1ull << 32) | (unsigned long long)k);
-        if ((old >> 32) < (unsigned long long)d.nr) d.lwork[old >> 32] = make_int2(r, (int)(old & 0xffffffffull));
-    }
-}
-
 // 1. has surface voxel s moved more than half the skin since its robot's last build?
 __device__ __forceinline__ void coll_check(const Dev &d, int s) {
     const int v = d.csurf[s];
@@ -407,10 +395,7 @@ __device__ __forceinline__ void coll_check(const Dev &d, int s) {
         const float4 h = P[0], l = P[1];
         const float4 lm = reinterpret_cast<const float4 *>(d.linmom)[2 * (size_t)v];
         const VMat &m = d.vmat[d.vinfo[v].y >> 8];
-        float4 *R = d.crec + 2 * (size_t)v;
-        R[0] = make_float4(h.x, h.y, h.z, h.w + l.w);
-        R[1] = make_float4(l.x, l.y, l.z, m.pstiff);
-        d.crec[2 * (size_t)d.nv + v] = make_float4(lm.x * m.mass_inv, lm.y * m.mass_inv, lm.z * m.mass_inv, m.c_col);
+        contact_record(d, v, h, l, lm, m.mass_inv, m.pstiff, m.c_col);
     }
     if (d.any_dyn) {  // robots whose surface follows their link table
         const uint2 vi = d.vinfo[v];
@@ -1385,18 +1370,18 @@ __global__ void k_coll_eval(Dev d) {
     d.contact[v] = make_double4(acc.x, acc.y, acc.z, 0.0);
 }
 
-cudaError_t launch_coll_prepare(const Dev &d, cudaStream_t s) {
+cudaError_t launch_coll_prepare(const Dev &d, cudaStream_t s, bool check) {
     if (!d.ns) return cudaSuccess;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &cs);
     if (e != cudaSuccess) return e;
-    if (cs == cudaStreamCaptureStatusNone) {
-        // single steps start from clear flags (inside graphs the narrow phase clears them)
+    if (check && cs == cudaStreamCaptureStatusNone) {
+        // a checked single step starts from clear flags (otherwise the narrow phase clears them)
         if ((e = cudaMemsetAsync(d.cflag, 0, sizeof(int) * (1 + (size_t)d.nr), s)) != cudaSuccess ||
             (e = cudaMemsetAsync(d.lwork_ctr, 0, sizeof(unsigned long long), s)) != cudaSuccess)
             return e;
     }
-    k_coll_check<<<(d.ns + 255) / 256, 256, 0, s>>>(d);
+    if (check) k_coll_check<<<(d.ns + 255) / 256, 256, 0, s>>>(d);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)d.cgrid);
     cfg.blockDim = dim3(kLocalListThreads);

@@ -1047,6 +1047,12 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         (rc = c->alloc(&d.lwork_ctr, 1)))
         return rc;
     d.crec = nullptr;
+    d.vsurf = nullptr;
+    if (d.mixed && d.ns && !d.any_dyn) {
+        std::vector<int> vsurf(pos.size(), -1);
+        for (size_t k = 0; k < csurf.size(); k++) vsurf[csurf[k]] = (int)k;
+        if ((rc = c->upload(&d.vsurf, vsurf))) return rc;
+    }
     if (d.mixed && d.ns && (rc = c->alloc(&d.crec, 3 * (size_t)d.nv))) return rc;
     CU(init_collision(d));
     // the contact evaluation beside the link pass, except with attachment (its links are made
@@ -1056,7 +1062,15 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         CU(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
         CU(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
         c->overlap = true;
+        // the rebuild beside the link pass too where robots rebuild in shared memory, some in most
+        // steps (256 robots 157 -> 142 us a step, 64 small ones 16.2 -> 14.8); not where one large
+        // body rarely does (a folded 64^3 body 54.4 us a step against 55.8 so)
+        c->fork_early = d.nhash == 0 ? 1 : 0;
     }
+    // launch shapes until vx3g_autotune is called: (256, 4) for links, (256, 1) for voxels, whose loads
+    // all go out at once (256 colliding robots 161.2 -> 157.5 us a step, a 64^3 body 45.4 -> 44.5,
+    // against (256, 1) for both; with (64, 14) for voxels 158.7 and 45.3)
+    c->shape_links = 1;
 
     // (c->ends holds the lattice's links alone here: no attachment)
     if (d.mixed && !d.ns && !d.any_dyn && !c->any_ff && !c->any_cilia && !c->any_bcs && !c->any_signals && (rc = plan_resident(c, lmoff, vmoff)))
@@ -1087,7 +1101,9 @@ void enqueue_voxels(vx3g_ctx *c, int parity, bool extra = true) {
     launch_remove(c->d, parity, c->stream);        // SecondaryExperiment robots only (end of the step)
 }
 
-cudaError_t enqueue_step(vx3g_ctx *c, int parity) {
+// check: the first step of a call or a graph, whose displacement check no voxel pass has done
+cudaError_t enqueue_step(vx3g_ctx *c, int parity, bool check = true) {
+    check = check || !c->d.vsurf;
     if (!c->overlap) {
         enqueue_links(c);
         // with attachment the cilia force is taken before any link is made: from the surface the
@@ -1100,17 +1116,17 @@ cudaError_t enqueue_step(vx3g_ctx *c, int parity) {
     // the check / list rebuild, then the contact evaluation on the side stream beside the
     // link pass (disjoint outputs: contact forces; link forces and link state), joined
     // before the voxel pass, which reads both
-    cudaError_t e = c->fork_early ? cudaSuccess : launch_coll_prepare(c->d, c->stream);
+    cudaError_t e = c->fork_early ? cudaSuccess : launch_coll_prepare(c->d, c->stream, check);
     if (e != cudaSuccess || (e = cudaEventRecord(c->ev_fork, c->stream)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(c->side, c->ev_fork, 0)) != cudaSuccess ||
-        (c->fork_early && (e = launch_coll_prepare(c->d, c->side)) != cudaSuccess))
+        (c->fork_early && (e = launch_coll_prepare(c->d, c->side, check)) != cudaSuccess))
         return e;
     launch_coll_eval(c->d, c->side);
+    launch_extra_forces(c->d, parity, c->stream);  // of the state the step starts with: beside the contacts too
     launch_links_mixed(c->d, c->stream, c->shape_links, false);
     if ((e = cudaEventRecord(c->ev_join, c->side)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(c->stream, c->ev_join, 0)) != cudaSuccess)
         return e;
-    launch_extra_forces(c->d, parity, c->stream);
     launch_detach(c->d, c->stream);
     launch_voxels_mixed(c->d, parity, c->stream, c->shape_voxels, false);
     launch_voxels_bc_mixed(c->d, parity, c->stream);
@@ -1124,7 +1140,7 @@ int get_graph(vx3g_ctx *c, int parity, cudaGraphExec_t *out) {
         cudaGraph_t g;
         CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t ce = cudaSuccess;
-        for (int i = 0; i < c->chunk && ce == cudaSuccess; i++) ce = enqueue_step(c, (parity + i) & 1);
+        for (int i = 0; i < c->chunk && ce == cudaSuccess; i++) ce = enqueue_step(c, (parity + i) & 1, i == 0);
         cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
         if (ce != cudaSuccess) {
             if (ee == cudaSuccess) cudaGraphDestroy(g);
@@ -1176,7 +1192,7 @@ int vx3g_step(vx3g_ctx *c, int n) {
         if (int rc = step_resident(c, k)) return rc;
         n -= k;
     }
-    while (n > 0) {
+    for (bool first = true; n > 0; first = false) {
         const int parity = (int)(c->steps & 1);
         if (n >= c->chunk) {
             cudaGraphExec_t g;
@@ -1186,7 +1202,7 @@ int vx3g_step(vx3g_ctx *c, int n) {
             n -= c->chunk;
             c->steps += c->chunk;
         } else {
-            CU(enqueue_step(c, parity));
+            CU(enqueue_step(c, parity, first));
             n -= 1;
             c->steps += 1;
         }
@@ -1719,7 +1735,7 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
             cudaGraph_t gr;
             CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             cudaError_t ce = cudaSuccess;
-            for (int i = 0; i < G && ce == cudaSuccess; i++) ce = enqueue_step(c, (p0 + i) & 1);
+            for (int i = 0; i < G && ce == cudaSuccess; i++) ce = enqueue_step(c, (p0 + i) & 1, i == 0);
             const cudaError_t ee = cudaStreamEndCapture(c->stream, &gr);
             if (ce != cudaSuccess || ee != cudaSuccess) {
                 if (ee == cudaSuccess) cudaGraphDestroy(gr);

@@ -191,6 +191,9 @@ struct Dev {
     const float4 *lrow, *vrow;
     int nlm, nvm;
     // collision
+    // mixed precision, where the surface keeps: per voxel its entry in csurf or -1; the voxel pass then
+    // does the next step's displacement check (NULL: k_coll_check does, every step)
+    int *vsurf;
     int *csurf;     // collision surface list (global voxel index), NS entries
     int4 *ccell;    // x: the bucket of a collision-surface voxel in the large-robot grid (-1: not binned)
     float4 *cposf;  // FP32 position per collision-surface voxel, written by the displacement check
@@ -333,7 +336,8 @@ void launch_dt(const Dev &d, double *maxfreq2_scratch, cudaStream_t s);
 // surface-voxel collision of one step: displacement check and list rebuild (one
 // cooperative kernel), then the narrow phase
 cudaError_t launch_collision(const Dev &d, cudaStream_t s);
-cudaError_t launch_coll_prepare(const Dev &d, cudaStream_t s);  // the check / rebuild kernel alone
+// the displacement check (left out where the voxel pass before did it) and the rebuild alone
+cudaError_t launch_coll_prepare(const Dev &d, cudaStream_t s, bool check = true);
 // the force field (d.ffv) and the cilia force (d.cfv) of the voxels of robots that have
 // them, at the start of the step of the given time parity
 void launch_extra_forces(const Dev &d, int parity, cudaStream_t s);

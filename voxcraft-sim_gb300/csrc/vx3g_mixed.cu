@@ -32,6 +32,9 @@ using mx::df_diff;
 // in ascending partner order as the FP64 pass does.
 // ATTACH: the batch has robots with EnableAttach (their pairs linked this step have their
 // contact added, then taken back); the other instance carries none of that code
+// candidates in flight per surface voxel: a 64^3 body's evaluation 11.7 us with one, 10.8 with two,
+// 14.7 with four (registers against resident warps); 64 small robots' 7.4, 5.1, 4.9
+constexpr int kEvalAhead = 2;
 template <bool ATTACH> __global__ void __launch_bounds__(256) k_coll_eval_mixed(Dev d) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) {  // the rebuild (if any) is done; the next check starts clear
@@ -40,17 +43,23 @@ template <bool ATTACH> __global__ void __launch_bounds__(256) k_coll_eval_mixed(
     }
     if (s >= d.ns) return;
     const int v = d.csurf[s];
+    const int n = d.nnb[s];
+    const int *lst = d.nbr + s;  // slot-major: entry k at lst[k*ns]
+    const size_t ns = (size_t)d.ns;
+    // kEvalAhead candidates at a time: their list entries, read one group ahead, then their
+    // 32-byte sectors in flight together, so the chain of dependent loads is a fraction as long
+    int un[kEvalAhead];
+#pragma unroll
+    for (int j = 0; j < kEvalAhead; j++) un[j] = j < n ? lst[j * ns] : v;
+    const float4 *R = d.crec;  // contact records of this step (written by the displacement check)
     const uint2 vi = d.vinfo[v];
+    const float4 pvH = R[2 * v], pvL = R[2 * v + 1];
     const int r = (int)vi.x;
     if (d.cflag[1 + r]) d.cflag[1 + r] = 0;
     // stopped robots and robots flagged before this step keep their contact forces; the
     // divergence bit is left out because the link pass, which may set it, runs beside
     // this kernel (a diverged robot never steps again, so its contacts feed nothing)
     if (d.status[r] & ~1) return;
-    const int n = d.nnb[s];
-    const int *lst = d.nbr + s;  // slot-major: entry k at lst[k*ns]
-    const size_t ns = (size_t)d.ns;
-    const float4 *R = d.crec;  // contact records of this step (written by the displacement check)
     // pairs linked by this step's attachment: contact added, then taken back
     const bool att = ATTACH && d.rp[r].attach && d.acnt[r] > 0;
     V3<float> acc{0, 0, 0};
@@ -59,46 +68,56 @@ template <bool ATTACH> __global__ void __launch_bounds__(256) k_coll_eval_mixed(
         acc = V3<float>{c.x, c.y, c.z};
     }
     if (n) {
-        const float4 pvH = R[2 * v], pvL = R[2 * v + 1], wv = R[2 * d.nv + v];
+        const float4 wv = R[2 * d.nv + v];
         const float bv = pvH.w;  // baseSizeAverage = baseSize (isotropic)
-        for (int k = 0; k < n; k++) {
-            const int u = lst[k * ns];  // partner voxel, ascending
-            const float4 puH = R[2 * u], puL = R[2 * u + 1];  // one 32-byte sector
-            // offset from the later surface voxel (voxel1) to the earlier one (voxel2)
-            const float sg = u < v ? 1.0f : -1.0f;
-            const float ox = sg * df_diff(puH.x, puL.x, pvH.x, pvL.x);
-            const float oy = sg * df_diff(puH.y, puL.y, pvH.y, pvL.y);
-            const float oz = sg * df_diff(puH.z, puL.z, pvH.z, pvL.z);
-            const float bu = puH.w;
-            const float wd = (bv + bu) * 0.625f;
-            // |offset| and its reciprocal from one hardware reciprocal square root (coincident
-            // voxels, d2 = 0, give dist = NaN and are skipped; the reference's force is NaN there)
-            const float d2 = ox * ox + oy * oy + oz * oz;
-            const float inv = rsqrtf(d2);
-            const float dist = d2 * inv;
-            if (!(dist <= wd)) continue;
-            const float rel = wd - dist;
-            if (!(rel > 0)) continue;
-            const float4 wu = R[2 * d.nv + u];
-            const float pstiff = __fdividef(2.0f * pvL.w * puL.w, pvL.w + puL.w);  // 2 / (1/a + 1/b)
-            const float dampC = 0.5f * (wv.w + wu.w);
-            const float ux = ox * inv, uy = oy * inv, uz = oz * inv;
-            const float w1x = wv.x, w1y = wv.y, w1z = wv.z;
-            const float w2x = wu.x, w2y = wu.y, w2z = wu.z;
-            // voxel1 = the later one: rv = w1.u - w2.u with (1, 2) = (v, u) when u < v, else (u, v)
-            const float rv = sg * ((w1x * ux + w1y * uy + w1z * uz) - (w2x * ux + w2y * uy + w2z * uz));
-            const float f = pstiff * rel + dampC * rv;
-            // v.contactForce += force (v is voxel1) or -= force (v is voxel2); force along u
-            if (ATTACH && att && linked_to(d, v, u)) {  // (acc + c) - c
-                const float cx = sg * ux * f, cy = sg * uy * f, cz = sg * uz * f;
-                acc.x = (acc.x + cx) - cx;
-                acc.y = (acc.y + cy) - cy;
-                acc.z = (acc.z + cz) - cz;
-                continue;
+        for (int k = 0; k < n; k += kEvalAhead) {
+            int uu[kEvalAhead];
+            float4 hi[kEvalAhead], lo[kEvalAhead];
+#pragma unroll
+            for (int j = 0; j < kEvalAhead; j++) uu[j] = un[j];
+#pragma unroll
+            for (int j = 0; j < kEvalAhead; j++) hi[j] = R[2 * uu[j]], lo[j] = R[2 * uu[j] + 1];
+#pragma unroll
+            for (int j = 0; j < kEvalAhead; j++) un[j] = k + kEvalAhead + j < n ? lst[(k + kEvalAhead + j) * ns] : v;
+#pragma unroll
+            for (int j = 0; j < kEvalAhead; j++) {
+                if (k + j >= n) break;
+                const int u = uu[j];  // partner voxel, ascending
+                const float4 puH = hi[j], puL = lo[j];
+                // offset from the later surface voxel (voxel1) to the earlier one (voxel2)
+                const float sg = u < v ? 1.0f : -1.0f;
+                const float ox = mx::mul(sg, df_diff(puH.x, puL.x, pvH.x, pvL.x));
+                const float oy = mx::mul(sg, df_diff(puH.y, puL.y, pvH.y, pvL.y));
+                const float oz = mx::mul(sg, df_diff(puH.z, puL.z, pvH.z, pvL.z));
+                const float bu = puH.w;
+                const float wd = mx::mul(mx::plus(bv, bu), 0.625f);
+                // |offset| and its reciprocal from one hardware reciprocal square root (coincident
+                // voxels, d2 = 0, give dist = NaN and are skipped; the reference's force is NaN there)
+                const float d2 = fmaf(oz, oz, mx::dot_a(ox, ox, oy, oy));
+                const float inv = rsqrtf(d2);
+                const float dist = mx::mul(d2, inv);
+                if (!(dist <= wd)) continue;
+                const float rel = mx::minus(wd, dist);
+                if (!(rel > 0)) continue;
+                const float4 wu = R[2 * d.nv + u];
+                const float pstiff = __fdividef(mx::mul(mx::mul(2.0f, pvL.w), puL.w), mx::plus(pvL.w, puL.w));  // 2 / (1/a + 1/b)
+                const float dampC = mx::mul(0.5f, mx::plus(wv.w, wu.w));
+                const float ux = mx::mul(ox, inv), uy = mx::mul(oy, inv), uz = mx::mul(oz, inv);
+                // voxel1 = the later one: rv = w1.u - w2.u with (1, 2) = (v, u) when u < v, else (u, v)
+                const float rv = mx::mul(sg, mx::minus(fmaf(wv.z, uz, mx::dot_a(wv.x, ux, wv.y, uy)),
+                                                       fmaf(wu.z, uz, mx::dot_a(wu.x, ux, wu.y, uy))));
+                const float f = mx::dot_a(pstiff, rel, dampC, rv);
+                // v.contactForce += force (v is voxel1) or -= force (v is voxel2); force along u
+                if (ATTACH && att && linked_to(d, v, u)) {  // (acc + c) - c
+                    const float cx = mx::mul(mx::mul(sg, ux), f), cy = mx::mul(mx::mul(sg, uy), f), cz = mx::mul(mx::mul(sg, uz), f);
+                    acc = V3<float>{mx::minus(mx::plus(acc.x, cx), cx), mx::minus(mx::plus(acc.y, cy), cy),
+                                    mx::minus(mx::plus(acc.z, cz), cz)};
+                    continue;
+                }
+                acc.x = fmaf(mx::mul(sg, ux), f, acc.x);
+                acc.y = fmaf(mx::mul(sg, uy), f, acc.y);
+                acc.z = fmaf(mx::mul(sg, uz), f, acc.z);
             }
-            acc.x += sg * ux * f;
-            acc.y += sg * uy * f;
-            acc.z += sg * uz * f;
         }
     }
     reinterpret_cast<float4 *>(d.contact)[v] = make_float4(acc.x, acc.y, acc.z, 0.0f);
@@ -219,6 +238,12 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
     float4 *AM = reinterpret_cast<float4 *>(d.angmom);
     mx::VoxelState s{P[2 * v], P[2 * v + 1], Qa[2 * v], Qa[2 * v + 1], LM[2 * v], LM[2 * v + 1], AM[2 * v], AM[2 * v + 1]};
     pdl_wait_then_release();  // the link pass (or the contact evaluation) of this step is done
+    // what depends on the voxel's number alone, beside the robot's and the materials' loads
+    float *tcur = d.tempe + (size_t)parity * d.nv, *tnext = d.tempe + (size_t)(parity ^ 1) * d.nv;
+    float te = tcur[v];
+    const float2 ph = d.phc[v];
+    const float4 ct = d.ns ? reinterpret_cast<const float4 *>(d.contact)[v] : make_float4(0, 0, 0, 0);
+    const int si = d.vsurf ? d.vsurf[v] : -1;
     const int r = (int)vi.x;
     const RobotP &rp = d.rp[r];
     const int st = d.status[r];
@@ -230,7 +255,6 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
     if (!BC && rp.bcs && d.vext[v] >= 0) return;  // stepped by the BC pass
     const mx::VoxC m = mx::vox_rows(d.vrow, d.nvm, (int)(fl >> 8));
     const bool actuated = rp.vary_temp && rp.temp_period > 0;
-    float *tcur = d.tempe + (size_t)parity * d.nv, *tnext = d.tempe + (size_t)(parity ^ 1) * d.nv;
     const int xi = BC ? d.vext[v] : -1;  // boundary-condition external
     const int dof = BC ? d.ext[xi].dof : 0;
     const double nom = BC ? d.vmat[fl >> 8].nom_size : 0.0;
@@ -270,10 +294,7 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
         const V3<float> vel = mx::velocity(s.lH, s.lL, m.a.x);
         F = mx::fma3(-m.a.z, vel, F);
         F.z = mx::plus(F.z, m.b.y);
-        if (rp.collision) {
-            const float4 c = reinterpret_cast<const float4 *>(d.contact)[v];
-            F = mx::diff(F, V3<float>{c.x, c.y, c.z});
-        }
+        if (rp.collision) F = mx::diff(F, V3<float>{ct.x, ct.y, ct.z});
         if (rp.cilia) {  // CiliaForce * Cilia (VX3_Voxel.cu:376), evaluated in FP64 by k_extra_forces
             const double4 c = d.cfv[v];
             F = add(F, V3<float>{(float)c.x, (float)c.y, (float)c.z});
@@ -324,14 +345,24 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
         AM[2 * v + 1] = s.aL;
     }
     if (actuated) {  // next step's temperature and base size
-        float te = tcur[v];
         if (m.a.y > 0.0f || thermal_on(d, d.vmat[fl >> 8].thermal_on_after, r, parity, dtf))
-            te = mx::temperature(d.tcyc[(size_t)parity * d.nr + r], d.phc[v], dtf, rp.cyc_rate, rp.amp_f, rp.expansion != 0);
+            te = mx::temperature(d.tcyc[(size_t)parity * d.nr + r], ph, dtf, rp.cyc_rate, rp.amp_f, rp.expansion != 0);
         mx::base_size(m, te, s.pH.w, s.pL.w);
         tnext[v] = te;
     }
     P[2 * v] = s.pH;
     P[2 * v + 1] = s.pL;
+    // the next step's displacement check (k_coll_check), while the voxel is at hand: 64 bytes written
+    // instead of a kernel that reads 80 and writes 64 (2.3 us of a 64^3 body's step, 9 us of 256
+    // colliding robots')
+    if (si >= 0) {
+        const float4 q = d.cref[si];
+        const float px = mx::plus(s.pH.x, s.pL.x), py = mx::plus(s.pH.y, s.pL.y), pz = mx::plus(s.pH.z, s.pL.z);
+        d.cposf[si] = make_float4(px, py, pz, mx::plus(s.pH.w, s.pL.w));
+        contact_record(d, v, s.pH, s.pL, s.lH, m.a.x, m.b.z, m.b.x);
+        const float ex = mx::minus(px, q.x), ey = mx::minus(py, q.y), ez = mx::minus(pz, q.z);
+        if (fmaf(ez, ez, mx::dot_a(ex, ex, ey, ey)) > q.w) flag_robot(d, r);
+    }
 }
 
 // the voxels with a boundary-condition external, after the main voxel pass

@@ -325,6 +325,32 @@ __device__ inline V3<double> force_field(const Dev &d, const RobotP &rp, double 
                       rp.ff[2] >= 0 ? math_eval(d.ftok + rp.ff[2], x, y, z, t, nv) : 0.0};
 }
 
+#if defined(__CUDACC__)
+// robot r's lists are rebuilt this step; the first voxel to say so puts a robot of the
+// shared-memory path on the work list of coll_list_robots
+__device__ __forceinline__ void flag_robot(const Dev &d, int r) {
+    if (*(volatile int *)&d.cflag[1 + r]) return;
+    if (atomicOr(&d.cflag[1 + r], 1) != 0) return;
+    atomicOr(d.cflag, 1);
+    const int k = d.rp[r].lchunks;
+    if (k) {
+        const unsigned long long old = atomicAdd(d.lwork_ctr, (1ull << 32) | (unsigned long long)k);
+        if ((old >> 32) < (unsigned long long)d.nr) d.lwork[old >> 32] = make_int2(r, (int)(old & 0xffffffffull));
+    }
+}
+
+// mixed precision: voxel v's contact record (Dev::crec) from its position pair, momentum (hi) and
+// material; each rounding on its own in either unit
+__device__ __forceinline__ void contact_record(const Dev &d, int v, float4 h, float4 l, float4 lm, float mass_inv, float pstiff,
+                                               float c_col) {
+    float4 *R = d.crec + 2 * (size_t)v;
+    R[0] = make_float4(h.x, h.y, h.z, __fadd_rn(h.w, l.w));
+    R[1] = make_float4(l.x, l.y, l.z, pstiff);
+    d.crec[2 * (size_t)d.nv + v] = make_float4(__fmul_rn(lm.x, mass_inv), __fmul_rn(lm.y, mass_inv), __fmul_rn(lm.z, mass_inv), c_col);
+}
+
+#endif
+
 // ------------------------------------------------------------- link material models
 // VX3_Material::stress (src/VX3/VX3_Material.cu:90-124) of link material m at strain eps:
 // zero past failure; the linear law for linear models, in compression and on the first
