@@ -390,6 +390,14 @@ __device__ __forceinline__ void coll_check(const Dev &d, int s) {
     const int v = d.csurf[s];
     const float4 p = pos_f(d, v), q = d.cref[s];  // q.w: squared displacement limit
     d.cposf[s] = p;  // the positions a rebuild on the shared-memory path lists from
+    if (d.cdv) {  // FP64: this step's contact record of the voxel (k_coll_eval)
+        const VMat &m = d.vmat[d.vinfo[v].y >> 8];
+        const double bs = d.pos[v].w;
+        const double4 lm = d.linmom[v];
+        const V3<double> w = scl(V3<double>{lm.x, lm.y, lm.z}, m.mass_inv);
+        d.cfl[v] = p;
+        d.cdv[v] = make_double4(w.x, w.y, w.z, (bs + bs + bs) / 3.0f);  // baseSizeAverage (VX3_Voxel.h:102-105)
+    }
     if (d.crec) {  // mixed precision: this step's contact record of the voxel (k_coll_eval_mixed)
         const float4 *P = reinterpret_cast<const float4 *>(d.pos) + 2 * (size_t)v;
         const float4 h = P[0], l = P[1];
@@ -1290,26 +1298,12 @@ cudaError_t init_collision(Dev &d) {
     return cudaSuccess;
 }
 
-// force on voxel1 from the pair (voxel1, voxel2) as VX3_Collision computes it
-__device__ __forceinline__ V3<double> pair_force(const Dev &d, int v1, int v2, double bsa1, double bsa2) {
-    const VMat &m1 = d.vmat[d.vinfo[v1].y >> 8];
-    const VMat &m2 = d.vmat[d.vinfo[v2].y >> 8];
-    const double pstiff = 2.0f / (1.0f / m1.pstiff + 1.0f / m2.pstiff);
-    const double dampC = 0.5f * (m1.c_col + m2.c_col);
-    const double4 p1 = load_state(d, d.pos, v1), p2 = load_state(d, d.pos, v2);
-    const V3<double> offset{p2.x - p1.x, p2.y - p1.y, p2.z - p1.z};
-    const double nom = (bsa1 + bsa2) * 0.625;
-    const double rel = nom - len(offset);
-    if (!(rel > 0)) return V3<double>{0, 0, 0};
-    const V3<double> u = normalized(offset);
-    const double4 l1 = load_state(d, d.linmom, v1), l2 = load_state(d, d.linmom, v2);
-    const V3<double> w1 = scl(V3<double>{l1.x, l1.y, l1.z}, m1.mass_inv);
-    const V3<double> w2 = scl(V3<double>{l2.x, l2.y, l2.z}, m2.mass_inv);
-    const double rv = (w1.x * u.x + w1.y * u.y + w1.z * u.z) - (w2.x * u.x + w2.y * u.y + w2.z * u.z);
-    return scl(u, pstiff * rel + dampC * rv);
-}
-
-// 3. exact test and contact forces on the listed pairs, ascending partner order
+// 3. exact test and contact forces (VX3_Collision) on the listed pairs, ascending partner order.
+// FP64 instructions bind this kernel on a body in contact (a folded 64^3 body: 555 us of a 1010 us
+// step): the prefilter reads FP32 records and costs none; baseSizeAverage and the velocities come
+// from the displacement check, once per voxel instead of once per contact and end; a pair takes
+// one square root, not three (the envelope test's distance is the force's); the envelope's
+// per-axis tests follow from the distance test (sqrt(x*x + ...) >= |x| in IEEE arithmetic too).
 __global__ void k_coll_eval(Dev d) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) {  // the rebuild (if any) is done; the next check starts clear
@@ -1318,13 +1312,13 @@ __global__ void k_coll_eval(Dev d) {
     }
     if (s >= d.ns) return;
     const int v = d.csurf[s];
+    const int n = d.nnb[s];
+    const int *lst = d.nbr + s;  // slot-major: entry k at lst[k*ns]
+    const size_t ns = (size_t)d.ns;
     const uint2 vi = d.vinfo[v];
     const int r = (int)vi.x;
     if (d.cflag[1 + r]) d.cflag[1 + r] = 0;
     if (d.status[r] != 0) return;
-    const int n = d.nnb[s];
-    const int *lst = d.nbr + s;  // slot-major: entry k at lst[k*ns]
-    const size_t ns = (size_t)d.ns;
     // attachment linked some pairs this step: their contact is added, then taken back
     // (VX3_VoxelyzeKernel.cu:824-826); a listed pair with a link was linked this step
     // (a link makes its robot rebuild its lists in the next step)
@@ -1335,34 +1329,36 @@ __global__ void k_coll_eval(Dev d) {
         acc = V3<double>{c.x, c.y, c.z};
     }
     if (n) {
-        const float4 pf = pos_f(d, v);
-        const double4 pv = load_state(d, d.pos, v);
-        double bsa = 0;
-        bool have_bsa = false;
+        const float4 pf = d.cfl[v];
+        const double4 pv = d.pos[v], cv = d.cdv[v];
+        const VMat &mv = d.vmat[vi.y >> 8];
+        const float kv = mv.pstiff, dv = mv.c_col;
+        int un = lst[0];
         for (int k = 0; k < n; k++) {
-            const int u = lst[k * ns];  // partner voxel, ascending
+            const int u = un;  // partner voxel, ascending
+            if (k + 1 < n) un = lst[(k + 1) * ns];
             // FP32 prefilter against the current cutoff: only pairs within 0.1% of it reach FP64
-            const float4 tf = pos_f(d, u);
+            const float4 tf = d.cfl[u];
             const float ex = tf.x - pf.x, ey = tf.y - pf.y, ez = tf.z - pf.z;
             const float cw = (pf.w + tf.w) * 0.625f * 1.001f;
             if (ex * ex + ey * ey + ez * ez > cw * cw) continue;
-            if (!have_bsa) {
-                bsa = (pv.w + pv.w + pv.w) / 3.0f;  // baseSizeAverage (VX3_Voxel.h:102-105)
-                have_bsa = true;
-            }
-            const double4 pu = load_state(d, d.pos, u);
-            const double bu = (pu.w + pu.w + pu.w) / 3.0f;
-            // exact envelope test, voxel1 = the later surface voxel
-            const double4 &pa = u < v ? pv : pu, &pb = u < v ? pu : pv;
-            const double ba = u < v ? bsa : bu, bb = u < v ? bu : bsa;
-            const V3<double> diff{pa.x - pb.x, pa.y - pb.y, pa.z - pb.z};
-            const double wd = (ba + bb) * 0.625;
-            if (diff.x > wd || diff.x < -wd) continue;
-            if (diff.y > wd || diff.y < -wd) continue;
-            if (diff.z > wd || diff.z < -wd) continue;
-            if (len(diff) > wd) continue;
+            // offset from the later surface voxel (voxel1) to the earlier one (voxel2)
+            const bool first = u < v;
+            const double4 pu = d.pos[u], cu = d.cdv[u];
+            const double4 &p1 = first ? pv : pu, &p2 = first ? pu : pv, &c1 = first ? cv : cu, &c2 = first ? cu : cv;
+            const V3<double> off{p2.x - p1.x, p2.y - p1.y, p2.z - p1.z};
+            const double l = len(off);
+            const double rel = (c1.w + c2.w) * 0.625 - l;
+            if (!(rel > 0)) continue;
+            const VMat &mu = d.vmat[d.vinfo[u].y >> 8];
+            const float ku = mu.pstiff, du = mu.c_col;
+            const float pstiff = 2.0f / (1.0f / (first ? kv : ku) + 1.0f / (first ? ku : kv));
+            const float dampC = 0.5f * ((first ? dv : du) + (first ? du : dv));
+            const V3<double> un3 = l > 0 ? vdiv(off, l) : off;  // normalized
+            const double rv = (c1.x * un3.x + c1.y * un3.y + c1.z * un3.z) - (c2.x * un3.x + c2.y * un3.y + c2.z * un3.z);
             // v.contactForce += force (v is voxel1) or += -force (v is voxel2)
-            const V3<double> f = u < v ? pair_force(d, v, u, bsa, bu) : neg(pair_force(d, u, v, bu, bsa));
+            V3<double> f = scl(un3, widen(pstiff) * rel + widen(dampC) * rv);
+            if (!first) f = neg(f);
             acc = add(acc, f);
             if (att && linked_to(d, v, u)) acc = sub(acc, f);
         }
@@ -1381,7 +1377,10 @@ cudaError_t launch_coll_prepare(const Dev &d, cudaStream_t s, bool check) {
             (e = cudaMemsetAsync(d.lwork_ctr, 0, sizeof(unsigned long long), s)) != cudaSuccess)
             return e;
     }
-    if (check) k_coll_check<<<(d.ns + 255) / 256, 256, 0, s>>>(d);
+    if (check) {
+        const int t = d.mixed ? 256 : fp64_threads(d.ns, 256);
+        k_coll_check<<<(d.ns + t - 1) / t, t, 0, s>>>(d);
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)d.cgrid);
     cfg.blockDim = dim3(kLocalListThreads);

@@ -1048,6 +1048,9 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         return rc;
     d.crec = nullptr;
     d.vsurf = nullptr;
+    d.cfl = nullptr;
+    d.cdv = nullptr;
+    if (!d.mixed && d.ns && ((rc = c->alloc(&d.cfl, d.nv)) || (rc = c->alloc(&d.cdv, d.nv)))) return rc;
     if (d.mixed && d.ns && !d.any_dyn) {
         std::vector<int> vsurf(pos.size(), -1);
         for (size_t k = 0; k < csurf.size(); k++) vsurf[csurf[k]] = (int)k;

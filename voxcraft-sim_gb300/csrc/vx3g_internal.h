@@ -203,6 +203,10 @@ struct Dev {
     // contact candidate, four voxels to a cache line -- and [2NV+v] {velocity (linMom hi /
     // m); collision damping}, read for the candidates in contact (NULL in FP64)
     float4 *crec;
+    // FP64: per voxel, written by the displacement check: FP32 position and base size; velocity and
+    // baseSizeAverage (NULL in mixed precision)
+    float4 *cfl;
+    double4 *cdv;
     unsigned *cpk;  // per collision-surface voxel: packed lattice word (kPackMask, kPackFixed; shared-memory path)
     float4 *cref;   // position at the last list build (w: squared displacement that forces a rebuild)
     int *nbr;       // candidate lists, slot-major [kNbrCap][NS]: partner voxel indices, ascending

@@ -131,6 +131,17 @@ __device__ __forceinline__ float signed_mag(double x) {
     return int_float(float_int(mag(x)) | (hi_word(x) & (int)0x80000000));
 }
 
+// qmul and qrotinv by a quaternion with x = 0 (FromAngleToPosX): the products with it, zeros, left out
+__device__ __forceinline__ Q4<double> qmul_x0(Q4<double> a, Q4<double> f) {
+    return Q4<double>{a.w * f.w - a.y * f.y - a.z * f.z, a.w * f.x + a.y * f.z - a.z * f.y, a.w * f.y + a.y * f.w + a.z * f.x,
+                      a.w * f.z - a.y * f.x + a.z * f.w};
+}
+__device__ __forceinline__ V3<double> qrotinv_x0(Q4<double> q, V3<double> f) {
+    const double tw = q.y * f.y + q.z * f.z, tx = q.w * f.x - q.y * f.z + q.z * f.y;
+    const double ty = q.w * f.y - q.z * f.x, tz = q.w * f.z + q.y * f.x;
+    return V3<double>{tx * q.w + ty * q.z - tz * q.y, tw * q.y - tx * q.z + ty * q.w, tw * q.z + tx * q.y + tz * q.w};
+}
+
 // ToRotationVector (VX3_Quat3D.h:347-359), its comparisons on the bits (|w| >= 1; 1 - w^2 >= 0)
 __device__ __forceinline__ V3<double> to_rotvec(Q4<double> q) {
     if ((unsigned)((hi_word(q.w) & 0x7fffffff) - 0x3ff00000) <= 0x40000000u) return V3<double>{0, 0, 0};  // |w| >= 1
@@ -563,17 +574,23 @@ template <class R> __device__ __forceinline__ void link_update(const Dev &d, int
     } else {
         const R l2 = len(pos2);
         angle1 = from_angle_to_posx(angle1, pos2, l2);
-        angle2 = qmul(angle1, angle2);
+        angle2 = qmul_x0(angle1, angle2);
         pos2 = V3<R>{l2 - rest, 0, 0};
         a1v = to_rotvec(angle1);
     }
     const V3<R> a2v = to_rotvec(angle2);
     ls[l] = pos2.x; ls[NL + l] = pos2.y; ls[2 * NL + l] = pos2.z;
-    const bool bent = !small || !is_zero(oldA1);
+    bool bent = !small || !is_zero(oldA1);
     if (bent) {
         ls[3 * NL + l] = a1v.x; ls[4 * NL + l] = a1v.y; ls[5 * NL + l] = a1v.z;
     }
     ls[6 * NL + l] = a2v.x; ls[7 * NL + l] = a2v.y; ls[8 * NL + l] = a2v.z;
+
+#if defined(__CUDA_ARCH__)
+    // a warp with a bent link takes the terms of a bent link for all (zeros add nothing): one of the two
+    // forms instead of both in turn
+    bent = __any_sync(__activemask(), bent);
+#endif
 
     // updateForces (VX3_Link.cu:135-218) + updateStrain (:220-260)
     const float axialStrain = (float)(pos2.x / rest);
@@ -599,8 +616,8 @@ template <class R> __device__ __forceinline__ void link_update(const Dev &d, int
                                a2v, oldA2);
     nfl |= LF_LVV;
     if (!small) {
-        f.fNeg = qrotinv(angle1, f.fNeg);
-        f.mNeg = qrotinv(angle1, f.mNeg);
+        f.fNeg = qrotinv_x0(angle1, f.fNeg);
+        f.mNeg = qrotinv_x0(angle1, f.mNeg);
     }
     f.fPos = qrotinv(angle2, f.fPos);
     f.mPos = qrotinv(angle2, f.mPos);
