@@ -120,18 +120,37 @@ __device__ __forceinline__ void rotvec_adj(Q q, V lv, Q &lq) {
     lq.w += dg * (q.x * lv.x + q.y * lv.y + q.z * lv.z);
 }
 
-// adjoint of q = FromRotationVector(in) (VX3_Quat3D.h:363-377): returns dL/d(in)
-__device__ __forceinline__ V from_rotvec_adj(V in, Q lq) {
-    const V th{0.5 * in.x, 0.5 * in.y, 0.5 * in.z};
-    const double m2 = dot(th, th);
+// FromRotationVector (VX3_Quat3D.h:363-377) of 2*th, with what its adjoint uses again: m = |th|, its
+// square, sine and cosine (sincos gives the bits of both for 27 FP64 instructions instead of 43)
+struct HalfTurn {
+    V th;
+    double m2, m, sn, cs;
+    bool tiny;
+};
+__device__ __forceinline__ Q from_half_turn(V th, HalfTurn &h) {
+    h.th = th;
+    h.m2 = dot(th, th);
+    h.tiny = h.m2 * h.m2 < 5.328e-15;
+    h.m = h.sn = h.cs = 0.0;
+    if (h.tiny) return from_half_rotvec(th);
+    h.m = sqrt(h.m2);
+    sincos(h.m, &h.sn, &h.cs);
+    const double s = h.sn / h.m;
+    return Q{h.cs, th.x * s, th.y * s, th.z * s};
+}
+
+// adjoint of q = FromRotationVector(2*th): returns dL/d(2*th)
+__device__ __forceinline__ V from_rotvec_adj(const HalfTurn &h, Q lq) {
+    const V th = h.th;
+    const double m2 = h.m2;
     const V lxyz{lq.x, lq.y, lq.z};
     V lth;
-    if (m2 * m2 < 5.328e-15) {  // w = 1 - m2/2, xyz = th*(1 - m2/6)
+    if (h.tiny) {  // w = 1 - m2/2, xyz = th*(1 - m2/6)
         const double s = 1.0 - m2 / 6.0;
         const double lm2 = -0.5 * lq.w - dot(th, lxyz) / 6.0;
         lth = V{s * lxyz.x + 2 * th.x * lm2, s * lxyz.y + 2 * th.y * lm2, s * lxyz.z + 2 * th.z * lm2};
     } else {                    // w = cos(m), xyz = th*sin(m)/m
-        const double m = sqrt(m2), sn = sin(m), cs = cos(m);
+        const double m = h.m, sn = h.sn, cs = h.cs;
         const double s = sn / m, ds = (m * cs - sn) / m2;
         const double lm = -sn * lq.w + dot(th, lxyz) * ds;
         lth = V{s * lxyz.x + lm * th.x / m, s * lxyz.y + lm * th.y / m, s * lxyz.z + lm * th.z / m};
@@ -165,7 +184,9 @@ __device__ __forceinline__ void from_angle_to_posx_adj(V r, Q lq, V &lr) {
     const double theta = acos(n.x);
     if (theta > 3.14159265358979 - 1e-7) return;  // constant (0, 0, 1, 0)
     // q = (cos(a), 0, n.z*ai*sin(a), -n.y*ai*sin(a)), a = theta/2, ai = 1/sqrt(n.y^2 + n.z^2)
-    const double ai = 1.0 / sqrt(n.z * n.z + n.y * n.y), a = 0.5 * theta, sa = sin(a), ca = cos(a);
+    const double ai = 1.0 / sqrt(n.z * n.z + n.y * n.y), a = 0.5 * theta;
+    double sa, ca;
+    sincos(a, &sa, &ca);
     double la = -sa * lq.w, lsa = n.z * ai * lq.y - n.y * ai * lq.z, lai = n.z * sa * lq.y - n.y * sa * lq.z;
     V ln{0, ai * -sa * lq.z, ai * sa * lq.y};
     la += ca * lsa;
@@ -192,6 +213,7 @@ struct LinkFwd {
     Q a1, a2, c, A2, B1, B2;  // B1/B2: the frames of the two ends after orientLink
     V fN0, mN0, mP0;  // elastic parts in the link frame
     V pc, uN, uP;     // damping parts (with lvv)
+    LMatD k;  // the link's constants
     V fN, mN, fP, mP; // end forces/moments before the rotations by B1 (large angle) and B2
     V sN_f, sN_m, sP_f, sP_m;  // slot values (original frame)
 };
@@ -223,17 +245,8 @@ __device__ __forceinline__ void link_forward(const Dev &d, const Snap &s, int l,
     Q angle1{1, 0, 0, 0}, angle2 = o.A2;
     const double restR = rest;
     o.L = restR;
-    const float SmallTurn = (float)((fabs(pos2.z) + fabs(pos2.y)) / pos2.x);
-    const float ExtendPerc = (float)(fabs(1 - pos2.x / restR));
-    const float HF = 1.2f, BEND = 0.05f, EXT = 0.50f;
     bool small = (fl & LF_SMALL) != 0, lvv = (fl & LF_LVV) != 0;
-    if (!small && SmallTurn < BEND && ExtendPerc < EXT) {
-        small = true;
-        lvv = false;
-    } else if (small && (SmallTurn > HF * BEND || ExtendPerc > HF * EXT)) {
-        small = false;
-        lvv = false;
-    }
+    turn_state(pos2, restR, small, lvv);
     o.small = small;
     if (small) {
         pos2.x -= restR;
@@ -245,7 +258,7 @@ __device__ __forceinline__ void link_forward(const Dev &d, const Snap &s, int l,
     o.B1 = angle1;
     o.B2 = angle2;
     o.pos2 = pos2;
-    const V a1v = to_rotvec(angle1), a2v = to_rotvec(angle2);
+    const V a1v = small ? V{0, 0, 0} : to_rotvec(angle1), a2v = to_rotvec(angle2);
     o.a1v = a1v;
     o.a2v = a2v;
     const double half = 0.5;
@@ -271,38 +284,34 @@ __device__ __forceinline__ void link_forward(const Dev &d, const Snap &s, int l,
     o.sN_f = o.sN_m = o.sP_f = o.sP_m = z;
     o.pc = o.uN = o.uP = z;
     o.dmN = o.dmP = 0;
+    o.k = link_consts(d, fl >> 8, e, d.dt[r]);
+    const LMatD &c = o.k;
     if (o.failed) return;
-    const float b1 = m.b1, b2 = m.b2, b3 = m.b3, a2 = m.a2;
-    V fNeg{(double)(stress * m.area), b1 * pos2.y - b2 * (a1v.z + a2v.z), b1 * pos2.z + b2 * (a1v.y + a2v.y)};
+    V fNeg{(double)(stress * m.area), c.b1 * pos2.y - c.b2 * (a1v.z + a2v.z), c.b1 * pos2.z + c.b2 * (a1v.y + a2v.y)};
     V fPos = neg(fNeg);
-    V mNeg{a2 * (a2v.x - a1v.x), -b2 * pos2.z - b3 * (2 * a1v.y + a2v.y), b2 * pos2.y - b3 * (2 * a1v.z + a2v.z)};
-    V mPos{a2 * (a1v.x - a2v.x), -b2 * pos2.z - b3 * (a1v.y + 2 * a2v.y), b2 * pos2.y - b3 * (a1v.z + 2 * a2v.z)};
+    V mNeg{c.a2 * (a2v.x - a1v.x), -c.b2 * pos2.z - c.b3 * (2 * a1v.y + a2v.y), c.b2 * pos2.y - c.b3 * (2 * a1v.z + a2v.z)};
+    V mPos{c.a2 * (a1v.x - a2v.x), -c.b2 * pos2.z - c.b3 * (a1v.y + 2 * a2v.y), c.b2 * pos2.y - c.b3 * (a1v.z + 2 * a2v.z)};
     o.fN0 = fNeg;
     o.mN0 = mNeg;
     o.mP0 = mPos;
     if (lvv) {
-        const float sqA1 = m.sqA1, sqA2xIp = m.sqA2xIp, sqB1 = m.sqB1, sqB2xFMp = m.sqB2xFMp, sqB3xIp = m.sqB3xIp;
         const V dPos2 = o.dP, dA1 = o.dA1, dA2 = o.dA2;
-        const V posCalc{sqA1 * dPos2.x, sqB1 * dPos2.y - sqB2xFMp * (dA1.z + dA2.z),
-                        sqB1 * dPos2.z + sqB2xFMp * (dA1.y + dA2.y)};
-        const float dtf = d.dt[li.x];
-        const uint32_t fnv = s.vinfo[e.x].y, fpv = s.vinfo[e.y].y;
-        const float dmN = d.vmat[fnv >> 8].dmc / ((fnv & VF_FIXED) ? 0.0f : dtf);
-        const float dmP = d.vmat[fpv >> 8].dmc / ((fpv & VF_FIXED) ? 0.0f : dtf);
+        const V posCalc{c.sqA1 * dPos2.x, c.sqB1 * dPos2.y - c.sqB2 * (dA1.z + dA2.z), c.sqB1 * dPos2.z + c.sqB2 * (dA1.y + dA2.y)};
+        const double dmN = 2 * c.kN, dmP = 2 * c.kP;
         fNeg = add(fNeg, scl(posCalc, dmN));
         fPos = sub(fPos, scl(posCalc, dmP));
-        const V uN{-sqA2xIp * (dA2.x - dA1.x), sqB2xFMp * dPos2.z + sqB3xIp * (2 * dA1.y + dA2.y),
-                   -sqB2xFMp * dPos2.y + sqB3xIp * (2 * dA1.z + dA2.z)};
-        const V uP{sqA2xIp * (dA2.x - dA1.x), sqB2xFMp * dPos2.z + sqB3xIp * (dA1.y + 2 * dA2.y),
-                   -sqB2xFMp * dPos2.y + sqB3xIp * (dA1.z + 2 * dA2.z)};
-        mNeg = sub(mNeg, scl(uN, (double)(half * dmN)));
-        mPos = sub(mPos, scl(uP, (double)(half * dmP)));
+        const V uN{-c.sqA2 * (dA2.x - dA1.x), c.sqB2 * dPos2.z + c.sqB3 * (2 * dA1.y + dA2.y),
+                   -c.sqB2 * dPos2.y + c.sqB3 * (2 * dA1.z + dA2.z)};
+        const V uP{c.sqA2 * (dA2.x - dA1.x), c.sqB2 * dPos2.z + c.sqB3 * (dA1.y + 2 * dA2.y),
+                   -c.sqB2 * dPos2.y + c.sqB3 * (dA1.z + 2 * dA2.z)};
+        mNeg = sub(mNeg, scl(uN, c.kN));
+        mPos = sub(mPos, scl(uP, c.kP));
         o.pc = posCalc;
         o.uN = uN;
         o.uP = uP;
         // a fixed end's force is never used; its (infinite) multiplier is left out of the adjoint
-        o.dmN = (fnv & VF_FIXED) ? 0.0 : (double)dmN;
-        o.dmP = (fpv & VF_FIXED) ? 0.0 : (double)dmP;
+        o.dmN = (s.vinfo[e.x].y & VF_FIXED) ? 0.0 : dmN;
+        o.dmP = (s.vinfo[e.y].y & VF_FIXED) ? 0.0 : dmP;
     }
     o.fN = fNeg;
     o.mN = mNeg;
@@ -357,12 +366,19 @@ __device__ __forceinline__ void adj_voxel(const Dev &d, const Snap &s, const Adj
     // ---- forward recompute (voxel_update<double>, same operation order)
     V F0{0, 0, 0}, M0{0, 0, 0};
     const Slot<double> *S = (const Slot<double> *)d.slots;
-    for (int dir = 0; dir < 6; dir++)
-        if (fl & (1u << dir)) {
-            const Slot<double> sl = S[(size_t)dir * d.nv + v];
-            F0 = add(F0, V{sl.f[0], sl.f[1], sl.f[2]});
-            M0 = add(M0, V{sl.m[0], sl.m[1], sl.m[2]});
-        }
+    const size_t nv = d.nv;
+    if (s.fsum) {
+        const double *f = s.fsum + v;
+        F0 = V{f[0], f[nv], f[2 * nv]};
+        M0 = V{f[3 * nv], f[4 * nv], f[5 * nv]};
+    } else {
+        for (int dir = 0; dir < 6; dir++)
+            if (fl & (1u << dir)) {
+                const Slot<double> sl = S[(size_t)dir * d.nv + v];
+                F0 = add(F0, V{sl.f[0], sl.f[1], sl.f[2]});
+                M0 = add(M0, V{sl.m[0], sl.m[1], sl.m[2]});
+            }
+    }
     bool stat = (fl & VF_STATIC) != 0;
     const bool floorOn = rp.floor != 0;
     const double bs = p4.w;
@@ -372,9 +388,9 @@ __device__ __forceinline__ void adj_voxel(const Dev &d, const Snap &s, const Adj
     const V vel = scl(lm, m.mass_inv);
     F = sub(F, scl(vel, m.c_glob));
     F.z += m.grav_force;
-    if (rp.collision) {  // this step's contact force (recomputed into d.contact for this state)
-        const double4 c = d.contact[v];
-        F = sub(F, V{c.x, c.y, c.z});
+    if (rp.collision) {  // this step's contact force
+        const double *f = s.fsum + v;
+        F = sub(F, V{f[6 * nv], f[7 * nv], f[8 * nv]});
     }
     F = add(F, V{0.0, 0.0, 0.0});
     if (rp.ff[0] >= 0 || rp.ff[1] >= 0 || rp.ff[2] >= 0) {  // force field: depends on time only (record checks)
@@ -431,21 +447,24 @@ __device__ __forceinline__ void adj_voxel(const Dev &d, const Snap &s, const Adj
     const V am1 = add(am, scl(M, dt));
     const double ki = dt * m.mom_inv;
     const V theta = scl(am1, ki);
-    const Q dq = from_rotvec(theta);
+    HalfTurn turn;
+    const Q dq = from_half_turn(V{0.5 * theta.x, 0.5 * theta.y, 0.5 * theta.z}, turn);
     const bool zero_am = floorOn && (float)(bsa / 2 - m.nom_size / 2 - pz1) >= 0 && stat;
     // ---- reverse
     const V lpos1 = vload(lv), llm_out = vload(lv + 7), lam_out = vload(lv + 10);
     const Q lo1{lv[3], lv[4], lv[5], lv[6]};
-    V lpos = lpos1, llm{0, 0, 0}, lam{0, 0, 0};
-    Q lq{0, 0, 0, 0}, ldq{0, 0, 0, 0};
+    // sums start from -0, to which adding x gives x exactly: the compiler drops that addition
+    const double o0 = -0.0;
+    V lpos = lpos1, llm{o0, o0, o0}, lam{o0, o0, o0};
+    Q lq{o0, o0, o0, o0}, ldq{o0, o0, o0, o0};
     qmul_adj(dq, o, lo1, ldq, lq);  // q1 = dq*q
     V lam1 = zero_am ? V{0, 0, 0} : lam_out;
-    lam1 = add(lam1, scl(from_rotvec_adj(theta, ldq), ki));
+    lam1 = add(lam1, scl(from_rotvec_adj(turn, ldq), ki));
     lam = add(lam, lam1);
     const V lM = scl(lam1, dt);
     lam = sub(lam, scl(lM, (double)m.mom_inv * (double)m.c_glob_rot));
     double lE = -dot(scl(am, m.mom_inv), lM) * (double)m.c_glob_rot / (2.0 * (double)m.E);
-    V lM0{0, 0, 0};
+    V lM0{o0, o0, o0};
     qrot_adj(o, M0, lM, lq, lM0);
     V ltr = lpos1;
     if (zero_xy) ltr.x = ltr.y = 0;
@@ -481,7 +500,7 @@ __device__ __forceinline__ void adj_voxel(const Dev &d, const Snap &s, const Adj
     lvel = sub(lvel, scl(lFt, m.c_glob));
     lE += -dot(vel, lFt) * (double)m.c_glob / (2.0 * (double)m.E);
     llm = add(llm, scl(lvel, m.mass_inv));
-    V lF0{0, 0, 0};
+    V lF0{o0, o0, o0};
     qrot_adj(o, F0, lFt, lq, lF0);
     lo[0] = lpos.x; lo[1] = lpos.y; lo[2] = lpos.z;
     lo[3] = lq.w; lo[4] = lq.x; lo[5] = lq.y; lo[6] = lq.z;
@@ -517,19 +536,21 @@ __device__ __forceinline__ void adj_link(const Dev &d, const Snap &s, const AdjB
         return;
     }
     const LMat &m = d.lmat[fl >> 8];
-    const double b1 = m.b1, b2 = m.b2, b3 = m.b3, ka2 = m.a2;
-    const double sqA1 = m.sqA1, sqA2 = m.sqA2xIp, sqB1 = m.sqB1, sqB2 = m.sqB2xFMp, sqB3 = m.sqB3xIp;
+    const LMatD &k = o.k;
+    const double b1 = k.b1, b2 = k.b2, b3 = k.b3, ka2 = k.a2;
+    const double sqA1 = k.sqA1, sqA2 = k.sqA2, sqB1 = k.sqB1, sqB2 = k.sqB2, sqB3 = k.sqB3;
+    const double o0 = -0.0;  // (as in adj_voxel)
     const double L = o.L;
     // lambda of the new local state (pos2, angle1v, angle2v) from the next step
     V lpos2 = vload(lloc), la1v = vload(lloc + 3), la2v = vload(lloc + 6);
     V loP{0, 0, 0}, loA1{0, 0, 0}, loA2{0, 0, 0};
-    Q lB1{0, 0, 0, 0}, lB2{0, 0, 0, 0};
+    Q lB1{o0, o0, o0, o0}, lB2{o0, o0, o0, o0};
     double lL = 0, lEl = 0;
     if (!o.failed) {
         const double *lFn = a.lF + 6 * (size_t)e.x, *lFp = a.lF + 6 * (size_t)e.y;
         const V lfNr = to_axis_x(axis, vload(lFn)), lmNr = to_axis_x(axis, vload(lFn + 3));
         const V lfPr = to_axis_x(axis, vload(lFp)), lmPr = to_axis_x(axis, vload(lFp + 3));
-        V lfN{0, 0, 0}, lmN{0, 0, 0}, lfP{0, 0, 0}, lmP{0, 0, 0};
+        V lfN{o0, o0, o0}, lmN{o0, o0, o0}, lfP{o0, o0, o0}, lmP{o0, o0, o0};
         if (o.small) {
             lfN = lfNr;
             lmN = lmNr;
@@ -591,7 +612,7 @@ __device__ __forceinline__ void adj_link(const Dev &d, const Snap &s, const AdjB
     }
     rotvec_adj(o.B2, la2v, lB2);
     V lP{0, 0, 0};
-    Q lA2{0, 0, 0, 0};
+    Q lA2{o0, o0, o0, o0};
     lL += -lpos2.x;
     if (o.small) {  // B1 = identity, B2 = A2, pos2 = P - (L, 0, 0)
         lA2 = lB2;
@@ -604,9 +625,9 @@ __device__ __forceinline__ void adj_link(const Dev &d, const Snap &s, const AdjB
         from_angle_to_posx_adj(o.P, lB1, lP);
     }
     // P = qrot(c, p0), A2 = c*a2, c = conj(a1)
-    Q lc{0, 0, 0, 0}, la2{0, 0, 0, 0};
+    Q lc{o0, o0, o0, o0}, la2{o0, o0, o0, o0};
     qmul_adj(o.c, o.a2, lA2, lc, la2);
-    V lp0{0, 0, 0};
+    V lp0{o0, o0, o0};
     qrot_adj(o.c, o.p0, lP, lc, lp0);
     const Q la1{lc.w, -lc.x, -lc.y, -lc.z};
     const Q lqn = axis_q_T(axis, la1), lqp = axis_q_T(axis, la2);
@@ -654,9 +675,11 @@ __device__ __forceinline__ void adj_gather(const Dev &d, const Snap &s, const Ad
     const double t = s.T[(size_t)a.parity * d.nr + r];
     if (rp.vary_temp && rp.temp_period > 0 && !(m.thermal_on_after > t) && !m.fixed) {
         const double arg = 2 * 3.1415926f * (t / rp.temp_period + d.phase[v]);
-        const double T = rp.temp_amp * sin(arg);
+        double sn, cs;
+        sincos(arg, &sn, &cs);
+        const double T = rp.temp_amp * sn;
         if (rp.expansion || !(T > 0))
-            a.gphase[v] += lbs * m.nom_size * (double)m.cte * rp.temp_amp * cos(arg) * (double)(2 * 3.1415926f);
+            a.gphase[v] += lbs * m.nom_size * (double)m.cte * rp.temp_amp * cs * (double)(2 * 3.1415926f);
     }
     a.glogE[v] += lE * (double)m.E * 2.302585092994046;  // dE/dlog10(E) = E ln 10
 }
@@ -698,10 +721,7 @@ __device__ __forceinline__ void adj_contact(const Dev &d, const Snap &s, const A
             const V diff{p1.x - p2.x, p1.y - p2.y, p1.z - p2.z};
             const double wd = (b1 + b2) * 0.625;
             if (diff.x > wd || diff.x < -wd || diff.y > wd || diff.y < -wd || diff.z > wd || diff.z < -wd) continue;
-            if (len(diff) > wd) continue;
-            const V off{p2.x - p1.x, p2.y - p1.y, p2.z - p1.z};
-            const double relf = (b1 + b2) * 0.625 - len(off);
-            if (!(relf > 0)) continue;
+            if (!(wd > len(diff))) continue;
             // the pair's force on v and its derivatives
             const uint2 ui = s.vinfo[u];
             const VMat &mu_ = d.vmat[ui.y >> 8];

@@ -17,6 +17,10 @@ struct Snap {
     uint2 *linfo;
     double *T;        // 2*NR
     int *status;      // NR
+    // recompute store (NULL elsewhere): per voxel the link force, the link moment and, with
+    // collisions, the contact force of the step from this state, kept instead of computed again
+    // (six or nine component-major arrays)
+    double *fsum;
 };
 
 struct AdjBufs {
@@ -38,14 +42,12 @@ struct AdjBufs {
 
 // copies one state: n voxels, l links, r robots
 void launch_snap_copy(const Snap &dst, const Snap &src, int nv, int nl, int nr, cudaStream_t st);
-// reverse of one step, in three launches per step when steps are chained:
-// slots(k) first; then per step voxel+link(k); then gather(k) fused with slots(k-1)
-// (ss = nullptr for the last gather of a sweep)
-void launch_adj_slots(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st);
-void launch_adj_voxel_link(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st);
-void launch_adj_gather_slots(const Dev &d, const Snap &sg, const Snap *ss, const AdjBufs &a, cudaStream_t st);
-// with collisions: the contact forces of the step must be in d.contact (and the candidate
-// lists valid) for the voxel adjoint; then the contact adjoint, then the gather
+// reverse of a chain of steps: voxel (last step), link, then per step gather of the step after
+// fused with the voxel adjoint, link, and at the end the gather of the first step (sv = nullptr).
+// With collisions the contact adjoint after the link's (the candidate lists valid for the state).
+void launch_adj_voxel(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st);
+void launch_adj_link(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st);
+void launch_adj_gather_voxel(const Dev &d, const Snap &sg, const Snap *sv, const AdjBufs &a, cudaStream_t st);
 void launch_adj_contact(const Dev &d, const Snap &s, const AdjBufs &a, cudaStream_t st);
 // dL/d(final state) for L = sum_r w_r . COM_r(end); also zeroes the link-state adjoint
 void launch_adj_seed(const Dev &d, const AdjBufs &a, cudaStream_t st);

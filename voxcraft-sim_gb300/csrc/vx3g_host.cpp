@@ -209,6 +209,11 @@ void from_slot(const double4 &s, bool mixed, double out[4]) {
 
 }  // namespace
 
+struct SnapMem {  // a snapshot and its device memory
+    Snap s;
+    void *mem;
+};
+
 struct vx3g_ctx {
     int precision = 0, chunk = 100, device = 0, nr = 0;
     cudaStream_t stream = nullptr;
@@ -246,11 +251,10 @@ struct vx3g_ctx {
     bool any_attach = false;     // some robot has EnableAttach (runtime links)
     bool any_acond = false;      // some robot has an attach condition
     std::vector<double> mass_tot;  // per robot: mass of the measured voxels (the COM's weights)
-    bool any_collision = false;
+    bool any_collision = false;    // some robot has collisions and surface voxels
+    int sum_rows = 6;              // arrays of Snap::fsum: 9 where some robot has RobotP::collision
     // recorded run (vx3g_record) and the adjoint's buffers (vx3g_backward)
-    std::vector<void *> rec_mem;
-    std::vector<Snap> rec_ck, rec_store;
-    Snap rec_end{};
+    std::vector<SnapMem> rec_ck, rec_store, rec_end;  // kept from run to run of the same lengths
     void *rec_slots = nullptr;
     int64_t rec_start = -1;
     int rec_n = 0, rec_k = 0;
@@ -284,10 +288,11 @@ struct vx3g_ctx {
         if (stream) cudaStreamSynchronize(stream);
         for (auto &g : adj_graphs) cudaGraphExecDestroy(g.second);
         adj_graphs.clear();
-        for (void *p : rec_mem) cudaFree(p);
-        rec_mem.clear();
-        rec_ck.clear();
-        rec_store.clear();
+        for (auto *list : {&rec_ck, &rec_store, &rec_end}) {
+            for (auto &m : *list) cudaFree(m.mem);
+            list->clear();
+        }
+        if (rec_slots) cudaFree(rec_slots);
         rec_slots = nullptr;
         rec_start = -1;
     }
@@ -653,6 +658,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         rp.vary_temp = R.vary_temp ? 1 : 0;
         rp.expansion = R.enable_expansion ? 1 : 0;
         rp.collision = R.enable_collision ? 1 : 0;
+        if (rp.collision) c->sum_rows = 9;
         rp.detach = R.enable_detach ? 1 : 0;
         c->any_detach |= R.enable_detach != 0;
         // SecondaryExperiment: the voxels of a material with RemoveFromSimulationAfterThisManySeconds > 0
@@ -943,6 +949,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     d.lmatd = nullptr;
     d.act = nullptr;
     d.actv = nullptr;
+    d.fsum = nullptr;
     d.nlm = (int)lmats.size();
     d.nvm = (int)vmats.size();
     float4 *lrow = nullptr, *vrow = nullptr;
@@ -1830,7 +1837,8 @@ size_t snap_bytes(const Dev &d) {
            al256(2 * nr * sizeof(double)) + al256(nr * sizeof(int));
 }
 
-Snap carve(const Dev &d, char *p) {
+// fsum: with the sums of the recompute store
+Snap carve(const Dev &d, char *p, bool fsum) {
     const size_t nv = d.nv, nl = d.nl, nr = d.nr;
     auto take = [&p](size_t n) {
         char *q = p;
@@ -1849,6 +1857,7 @@ Snap carve(const Dev &d, char *p) {
     s.linfo = (uint2 *)take(nl * sizeof(uint2));
     s.T = (double *)take(2 * nr * sizeof(double));
     s.status = (int *)take(nr * sizeof(int));
+    s.fsum = fsum ? (double *)p : nullptr;
     return s;
 }
 
@@ -1858,17 +1867,22 @@ Snap live_snap(const Dev &d) {
     s.vinfo = d.vinfo; s.tempe = d.tempe;
     s.lstate = (double *)d.lstate; s.strain = d.strain; s.linfo = d.linfo;
     s.T = d.T; s.status = d.status;
+    s.fsum = nullptr;
     return s;
 }
 
-int alloc_snaps(vx3g_ctx *c, std::vector<Snap> &out, int n) {
-    const size_t sb = snap_bytes(c->d);
-    for (int i = 0; i < n; i++) {
+// makes `out` hold n snapshots, keeping those it has
+int size_snaps(vx3g_ctx *c, std::vector<SnapMem> &out, int n, bool fsum) {
+    const size_t sb = snap_bytes(c->d) + (fsum ? c->sum_rows * (size_t)c->d.nv * sizeof(double) : 0);
+    while ((int)out.size() > n) {
+        cudaFree(out.back().mem);
+        out.pop_back();
+    }
+    while ((int)out.size() < n) {
         void *m = nullptr;
-        cudaError_t e = cudaMalloc(&m, sb);
+        const cudaError_t e = cudaMalloc(&m, sb);
         if (e != cudaSuccess) return fail(VX3G_ERR_NOMEM, std::string("cudaMalloc (state snapshots): ") + cudaGetErrorString(e));
-        c->rec_mem.push_back(m);
-        out.push_back(carve(c->d, (char *)m));
+        out.push_back({carve(c->d, (char *)m, fsum), m});
     }
     return VX3G_OK;
 }
@@ -1881,37 +1895,39 @@ cudaError_t enqueue_adj_segment(vx3g_ctx *c, const AdjBufs &a0, int len, int p0)
     const Snap live = live_snap(d);
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < len && e == cudaSuccess; i++) {
-        launch_snap_copy(c->rec_store[i], live, d.nv, d.nl, d.nr, c->stream);
+        launch_snap_copy(c->rec_store[i].s, live, d.nv, d.nl, d.nr, c->stream);
+        c->d.fsum = c->rec_store[i].s.fsum;
         e = enqueue_step(c, (p0 + i) & 1);
+        c->d.fsum = nullptr;
     }
     AdjBufs a = a0;
-    if (!c->any_collision) {
-        launch_adj_slots(d, c->rec_store[len - 1], a, c->stream);
-        for (int i = len - 1; i >= 0; i--) {
-            a.parity = (p0 + i) & 1;
-            launch_adj_voxel_link(d, c->rec_store[i], a, c->stream);
-            launch_adj_gather_slots(d, c->rec_store[i], i > 0 ? &c->rec_store[i - 1] : nullptr, a, c->stream);
-        }
-        return e;
-    }
-    // with collisions, per reverse step: the step's contact forces from its stored state
-    // (the candidate lists checked and rebuilt against that state as the forward pass
-    // does), then the link-force recompute, the voxel and link adjoints, the contact
-    // adjoint and the gather
+    // per reverse step: the gather of the step after with the voxel adjoint, the link adjoint and,
+    // with collisions, the candidate lists checked and rebuilt against the step's state as the
+    // forward pass does, and the contact adjoint
+    Snap after{};
     for (int i = len - 1; i >= 0 && e == cudaSuccess; i--) {
-        const Snap &st = c->rec_store[i];
-        Dev ds = d;
-        ds.pos = st.pos;
-        ds.linmom = st.linmom;
-        ds.vinfo = st.vinfo;
-        ds.status = st.status;
-        e = launch_collision(ds, c->stream);
+        const Snap &st = c->rec_store[i].s;
+        if (c->any_collision) {
+            Dev ds = d;
+            ds.pos = st.pos;
+            ds.linmom = st.linmom;
+            ds.vinfo = st.vinfo;
+            ds.status = st.status;
+            e = launch_coll_prepare(ds, c->stream, true);
+        }
+        if (i == len - 1) {
+            a.parity = (p0 + i) & 1;
+            launch_adj_voxel(d, st, a, c->stream);
+        } else {
+            a.parity = (p0 + i + 1) & 1;
+            launch_adj_gather_voxel(d, after, &st, a, c->stream);
+        }
         a.parity = (p0 + i) & 1;
-        launch_adj_slots(d, st, a, c->stream);
-        launch_adj_voxel_link(d, st, a, c->stream);
-        launch_adj_contact(d, st, a, c->stream);
-        launch_adj_gather_slots(d, st, nullptr, a, c->stream);
+        launch_adj_link(d, st, a, c->stream);
+        if (c->any_collision) launch_adj_contact(d, st, a, c->stream);
+        after = st;
     }
+    if (len > 0) launch_adj_gather_voxel(d, after, nullptr, a, c->stream);
     return e;
 }
 
@@ -1959,9 +1975,13 @@ int vx3g_record(vx3g_ctx *c, int n, int k) {
         return fail(VX3G_ERR_UNSUPPORTED, "the adjoint of a changing link table (detach, removal) is not implemented");
     CU(cudaSetDevice(c->device));
     CU(cudaStreamSynchronize(c->stream));
-    c->free_record();
+    c->rec_start = -1;
     const int nck = (n + k - 1) / k;
-    int rc = alloc_snaps(c, c->rec_ck, nck);
+    // the snapshots and the backward graphs are kept for a run of the same lengths (allocating and
+    // instantiating them took 3.1 ms of the 38.0 ms of a first run of 200 steps of a 12x12x6 body); else
+    // all go first, so that the two runs' memory is never held together
+    if (n != c->rec_n || k != c->rec_k) c->free_record();
+    int rc = size_snaps(c, c->rec_ck, nck, false);
     if (rc) {
         c->free_record();
         return rc;
@@ -1972,7 +1992,7 @@ int vx3g_record(vx3g_ctx *c, int n, int k) {
     c->rec_n = n;
     c->rec_k = k;
     for (int j = 0; j < nck; j++) {
-        launch_snap_copy(c->rec_ck[j], live, d.nv, d.nl, d.nr, c->stream);
+        launch_snap_copy(c->rec_ck[j].s, live, d.nv, d.nl, d.nr, c->stream);
         rc = vx3g_step(c, std::min(k, n - j * k));
         if (rc) {
             c->free_record();
@@ -2026,25 +2046,26 @@ int vx3g_backward(vx3g_ctx *c, const double *dL_dcom, double *dL_dphase, double 
     }
     const int n = c->rec_n, k = c->rec_k;
     const int store = std::min(n, k);
-    if ((int)c->rec_store.size() < store || !c->rec_slots) {  // recompute store + the end state
+    if ((int)c->rec_store.size() != store) {  // (the graphs name the store's snapshots)
+        CU(cudaStreamSynchronize(c->stream));
         for (auto &g : c->adj_graphs) cudaGraphExecDestroy(g.second);
         c->adj_graphs.clear();
-        c->rec_store.clear();
-        std::vector<Snap> end;
-        if ((rc = alloc_snaps(c, c->rec_store, store)) || (rc = alloc_snaps(c, end, 1))) return rc;
-        c->rec_end = end[0];
-        void *m = nullptr;
-        cudaError_t e = cudaMalloc(&m, (36 + 4) * nv * sizeof(double));  // slots + contact forces
-        if (e != cudaSuccess) return fail(VX3G_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        c->rec_mem.push_back(m);
-        c->rec_slots = m;
+        if ((rc = size_snaps(c, c->rec_store, store, true))) return rc;
+    }
+    if ((rc = size_snaps(c, c->rec_end, 1, false))) return rc;
+    if (!c->rec_slots) {
+        const cudaError_t e = cudaMalloc(&c->rec_slots, (36 + 4) * nv * sizeof(double));  // slots + contact forces
+        if (e != cudaSuccess) {
+            c->rec_slots = nullptr;
+            return fail(VX3G_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        }
     }
     AdjBufs a = c->ab;
     CU(cudaMemcpyAsync((void *)a.w, dL_dcom, 3 * nr * 8, cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemsetAsync(a.gphase, 0, nv * 8, c->stream));
     CU(cudaMemsetAsync(a.glogE, 0, nv * 8, c->stream));
     const Snap live = live_snap(d);
-    launch_snap_copy(c->rec_end, live, d.nv, d.nl, d.nr, c->stream);
+    launch_snap_copy(c->rec_end[0].s, live, d.nv, d.nl, d.nr, c->stream);
     CU(cudaMemcpyAsync(c->rec_slots, d.slots, 36 * nv * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     CU(cudaMemcpyAsync((double *)c->rec_slots + 36 * nv, d.contact, nv * sizeof(double4), cudaMemcpyDeviceToDevice,
                        c->stream));
@@ -2053,13 +2074,13 @@ int vx3g_backward(vx3g_ctx *c, const double *dL_dcom, double *dL_dphase, double 
     for (int j = nck - 1; j >= 0; j--) {
         const int len = std::min(k, n - j * k);
         const int p0 = (int)((c->rec_start + (int64_t)j * k) & 1);
-        launch_snap_copy(live, c->rec_ck[j], d.nv, d.nl, d.nr, c->stream);
+        launch_snap_copy(live, c->rec_ck[j].s, d.nv, d.nl, d.nr, c->stream);
         launch_actuation(d, p0, c->stream);
         cudaGraphExec_t g = nullptr;
         if ((rc = adj_segment_graph(c, a, len, p0, &g))) return rc;
         CU(cudaGraphLaunch(g, c->stream));
     }
-    launch_snap_copy(live, c->rec_end, d.nv, d.nl, d.nr, c->stream);
+    launch_snap_copy(live, c->rec_end[0].s, d.nv, d.nl, d.nr, c->stream);
     launch_actuation(d, (int)(c->steps & 1), c->stream);
     CU(cudaMemcpyAsync(d.slots, c->rec_slots, 36 * nv * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     CU(cudaMemcpyAsync(d.contact, (double *)c->rec_slots + 36 * nv, nv * sizeof(double4), cudaMemcpyDeviceToDevice,

@@ -187,6 +187,7 @@ struct Dev {
     const LMatD *lmatd;
     double4 *act;
     double2 *actv;
+    double *fsum;  // where the FP64 voxel pass keeps its sums (Snap::fsum), or NULL
     // mixed contexts: the rows of the nlm link and nvm voxel materials (vx3g_mixed_math.cuh)
     const float4 *lrow, *vrow;
     int nlm, nvm;

@@ -765,6 +765,16 @@ template <class R> __device__ __forceinline__ void voxel_update(const Dev &d, in
             Ms = dir ? add(Ms, n) : n;
         }
     }
+    if (d.fsum) {  // the backward pass's recompute keeps them (Snap::fsum)
+        const size_t nv = d.nv;
+        double *f = d.fsum + v;
+        f[0] = Fs.x, f[nv] = Fs.y, f[2 * nv] = Fs.z;
+        f[3 * nv] = Ms.x, f[4 * nv] = Ms.y, f[5 * nv] = Ms.z;
+        if (rp.collision) {
+            const double4 c = d.contact[v];
+            f[6 * nv] = c.x, f[7 * nv] = c.y, f[8 * nv] = c.z;
+        }
+    }
     bool stat = (fl & VF_STATIC) != 0;
     const bool floorOn = rp.floor != 0;
     const double bs = p.w;
