@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -391,13 +392,18 @@ int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<
         const auto f = c->ends.begin();
         return (int)(std::lower_bound(f + b.l0, f + b.l0 + b.nl, v, [](const int2 &e, int x) { return e.y < x; }) - f);
     };
+    // links l0 to l1 - 1 by axis (two sums that vectorise; a counter per axis waits on its own stores)
+    auto axes = [&](int l0, int l1) {
+        int n1 = 0, n2 = 0;
+        for (int l = l0; l < l1; l++) n1 += c->laxis[l] == 1, n2 += c->laxis[l] == 2;
+        return std::array<int, 3>{l1 - l0 - n1 - n2, n1, n2};
+    };
     // most entries a CTA's links take axis by axis, with K CTAs
     auto entries = [&](const ResBundle &b, int K) {
         int most = 0;
         for (int j = 0; j < K; j++) {
             const int a = std::min(b.v0 + j * b.q, b.v0 + b.nv), z = std::min(a + b.q, b.v0 + b.nv);
-            int n[3] = {0, 0, 0};
-            for (int l = link_at(b, a), e = link_at(b, z); l < e; l++) n[c->laxis[l]]++;
+            const auto n = axes(link_at(b, a), link_at(b, z));
             most = std::max(most, up(n[0], 32) + up(n[1], 32) + up(n[2], 32));
         }
         return most;
@@ -431,26 +437,27 @@ int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<
         if (p.b.empty()) continue;
         // the longest first: the SMs take the rest as they come free
         std::stable_sort(p.b.begin(), p.b.end(), [](const ResBundle &a, const ResBundle &b) { return a.nl > b.nl; });
-        std::vector<int2> ctas;
-        std::vector<int> order;
-        int lc = 0;
+        std::vector<int2> ctas, links;
+        int lc = 0, at = 0;
         for (const ResBundle &b : p.b) {
             lc = std::max(lc, b.lc);
             for (int j = 0; j < K; j++) {
                 const int a = std::min(b.v0 + j * b.q, b.v0 + b.nv), z = std::min(a + b.q, b.v0 + b.nv);
-                const int l0 = link_at(b, a), l1 = link_at(b, z), at = (int)order.size();
-                for (uint32_t x = 0; x < 3; x++) {
-                    for (int l = l0; l < l1; l++)
-                        if (c->laxis[l] == x) order.push_back(l);
-                    while ((order.size() - at) % 32) order.push_back(-1);
-                }
-                ctas.push_back(make_int2(at, (int)order.size() - at));
+                const int l0 = link_at(b, a), l1 = link_at(b, z);
+                const auto n = axes(l0, l1);
+                const int len = up(n[0], 32) + up(n[1], 32) + up(n[2], 32);
+                links.push_back(make_int2(l0, l1));
+                ctas.push_back(make_int2(at, len));
+                at += len;
             }
         }
         ResBundle *pb;
-        int2 *pc;
+        int2 *pc, *pl;
         int *po, rc;
-        if ((rc = c->upload(&pb, p.b)) || (rc = c->upload(&pc, ctas)) || (rc = c->upload(&po, order))) return rc;
+        if ((rc = c->upload(&pb, p.b)) || (rc = c->upload(&pc, ctas)) || (rc = c->upload(&pl, links)) ||
+            (rc = c->alloc(&po, at)))
+            return rc;
+        CU(launch_res_order(d, pl, pc, (int)ctas.size(), po, c->stream));
         CU(cudaStreamSynchronize(c->stream));  // the host vectors end here
         const int t = std::min(std::max(up(lc, 64), 64), p.smem <= kHalf ? kHalfThreads : kResThreads);
         c->res.push_back(ResClass{K, t, (int)p.b.size(), p.smem, pb, pc, po});

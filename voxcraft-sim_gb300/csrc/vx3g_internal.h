@@ -330,6 +330,8 @@ constexpr int kResSteps = 256;         // most steps of one launch (about 20 ms 
 constexpr int kResSmem = 227 * 1024;   // a CTA's shared memory
 size_t steps_mixed_bytes(int q, int lc);
 cudaError_t init_steps_mixed();
+// ResClass::order from each CTA's links (first, end) and its entries
+cudaError_t launch_res_order(const Dev &d, const int2 *links, const int2 *ctas, int n, int *order, cudaStream_t s);
 cudaError_t launch_steps_mixed(const Dev &d, int parity, int n, const ResClass &c, cudaStream_t s);
 void launch_init_temperature(const Dev &d, int mixed, cudaStream_t s);
 // the mixed-precision voxel pass of the voxels with a boundary-condition external (after

@@ -728,6 +728,31 @@ __global__ void __launch_bounds__(kResThreads, 1) k_steps_mixed(Dev d, int parit
             for (int k = 0; k < 2; k++) d.T[(size_t)k * d.nr + B.r0 + i] = S.rob(i).T[k], d.tcyc[(size_t)k * d.nr + B.r0 + i] = S.rob(i).tc[k];
 }
 
+// the links of each CTA of k_steps_mixed axis by axis, each axis padded with -1 to whole warps: one warp
+// per CTA.  On the host this and its upload took 15 of the 96 ms that a batch of 1024 robots took to create.
+__global__ void __launch_bounds__(32) k_res_order(const uint2 *linfo, const int2 *links, const int2 *ctas, int *order) {
+    const int lane = threadIdx.x;
+    const int2 lk = links[blockIdx.x];
+    int at = ctas[blockIdx.x].x;
+    for (uint32_t x = 0; x < 3; x++) {
+        int n = 0;
+        for (int l0 = lk.x; l0 < lk.y; l0 += 32) {
+            const int l = l0 + lane;
+            const bool hit = l < lk.y && (linfo[l].y & LF_AXIS) == x;
+            const unsigned m = __ballot_sync(~0u, hit);
+            if (hit) order[at + n + __popc(m & ((1u << lane) - 1))] = l;
+            n += __popc(m);
+        }
+        const int end = (n + 31) / 32 * 32;
+        if (n + lane < end) order[at + n + lane] = -1;
+        at += end;
+    }
+}
+cudaError_t launch_res_order(const Dev &d, const int2 *links, const int2 *ctas, int n, int *order, cudaStream_t s) {
+    k_res_order<<<n, 32, 0, s>>>(d.linfo, links, ctas, order);
+    return cudaGetLastError();
+}
+
 cudaError_t init_steps_mixed() {
     cudaError_t e = cudaFuncSetAttribute(k_steps_mixed<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_steps_mixed<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
