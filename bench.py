@@ -480,10 +480,17 @@ def main():
     peak, peak_kind = peaks()
     achieved = kernel_bytes[dom] / (kernel_ms[dom] / 1e3) / 1e9 if kernel_ms[dom] > 0 else 0.0
     traffic = ncu_traffic(args.workload, args.precision, dom)
-    # link pass + voxel pass; collision: the displacement check, the cooperative list
-    # rebuild kernel (it returns at once unless a rebuild is due), the global grid's list
-    # kernel (the same) and the contact evaluation
-    kernels_per_step = 2 + ((4 if global_grid else 3) if ns_coll else 0)
+    # link pass + voxel pass; collision: the cooperative list rebuild kernel (it returns at once
+    # unless a rebuild is due), the global grid's list kernel (the same) and the contact evaluation;
+    # the displacement check is a kernel of its own in FP64, and in mixed precision in the first step
+    # of a graph (the voxel pass does it after that)
+    checks = 0 if not ns_coll else (C // G + (1 if 0 < C < G else 0)) if prec else C
+    launches_per_call = (2 + ((3 if global_grid else 2) if ns_coll else 0)) * C + checks
+    # mixed-precision workloads without collisions: up to 256 steps in one launch (counted once,
+    # although robots of further cluster sizes have launches of their own beside it)
+    resident = bool(prec) and not ns_coll
+    if resident:
+        launches_per_call = -(-C // 256)
     shapes = [int(x) for x in b.launch_shapes()]
     b.close()
 
@@ -550,7 +557,7 @@ def main():
                      "whole_step_algorithmic_gbs": (ab["links"] + ab["voxels"] + ab["collision"]) * C * K
                      / (total_ms / 1e3) / 1e9},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        "gpu_launches": kernels_per_step * C * K,
+        "gpu_launches": launches_per_call * K,
         "clocks": clk.summary(),
         "robot_status_nonzero": int(np.count_nonzero(status)),
     }

@@ -286,8 +286,8 @@ __device__ __forceinline__ double4 load_state(const Dev &d, const double4 *a, in
 // Threads per block of an FP64 pass over n elements.  An SM issues one FP64 warp instruction
 // about every 16-20 cycles, whichever of its warps it comes from, so these passes are bound by
 // the busiest SM's count of warps, not by occupancy: blocks of one warp spread a small batch over
-// all 152 SMs (a 10^3 block's link pass, 2,700 links: 31.2 us in 11 blocks of 256 threads, 7.4 us
-// in 85 of 32).  Once every SM has eight blocks, larger ones cost nothing and launch faster.
+// all 152 SMs (100 steps of a 10^3 block, 2,700 links: 5.08 ms in blocks of 256 threads, 2.79 ms in
+// blocks of 32).  Once every SM has eight blocks, larger ones cost nothing and launch faster.
 inline int fp64_threads(int n, int most) {
     int t = 32;
     while (t < most && (n + t - 1) / t > 152 * 8) t *= 2;
