@@ -1080,6 +1080,29 @@ __device__ __forceinline__ void coll_list_robots(const Dev &d, unsigned char *ls
                 if (slot < n) srt[slot] = (unsigned short)i;  // bucket h: srt[beg[h] .. cur[h])
             }
             __syncthreads();
+            // Other CTAs bin the robot for its other chunks, and the atomics order a bucket differently in
+            // each: a bucket that lies across a chunk boundary goes in index order, so that all agree which
+            // voxel is in which chunk (else one is in none, and its list stays as it was).  The others keep
+            // theirs: a list does not depend on it.  (cand is free until the lists are made.)
+            if (n > kLocalListChunk) {  // uniform
+                auto across = [&](int i, int *b, int *e) {
+                    const int h = local_bucket(local_cell(P[i], g), g);
+                    *b = beg[h], *e = min(cur[h], n);
+                    return *b / kLocalListChunk != (*e - 1) / kLocalListChunk;
+                };
+                for (int i = tid; i < n; i += T) {
+                    int b, e, rank = 0;
+                    if (!across(i, &b, &e)) continue;
+                    for (int k = b; k < e; k++) rank += srt[k] < i ? 1 : 0;
+                    cand[b + rank] = (unsigned short)i;
+                }
+                __syncthreads();
+                for (int k = tid; k < n; k += T) {
+                    int b, e;
+                    if (across(srt[k], &b, &e)) srt[k] = cand[k];
+                }
+                __syncthreads();
+            }
             built = r;
         }
         // three threads per voxel (a trio), thread q of the trio scanning the plane
