@@ -100,3 +100,11 @@ def test_a_robot_that_diverges_stops_alone():
 
     out = _same(robots, [90], before=tear)
     assert list(out["status"] != 0) == [False, False, True, False, True]
+
+
+# either side of the rule that takes such a batch to the one launch: robots of a whole SM per CTA, as many
+# as run at once, and twice that (a second wave, slower than the passes)
+@pytest.mark.parametrize("count,dims", [(8, (16, 16, 16)), (30, (13, 13, 13))])
+def test_large_robots(count, dims):
+    rng = np.random.default_rng(count)
+    _same([_body(rng, dims, fill=1.0) for _ in range(count)], [3, 40])

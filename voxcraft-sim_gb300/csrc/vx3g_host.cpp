@@ -365,6 +365,35 @@ int check_math_program(const vx3g_math_token *t, int *len, bool *reads_pos, std:
     return VX3G_ERR_INVALID;
 }
 
+// Microseconds of a step by k_steps_mixed and by the two passes.  Fitted to 226 batches of 1 to 800
+// robots of 6^3 to 18^3 cells, filled or to 70%, one size or mixed, each timed both ways: the resident
+// kernel is 0.70 to 3 times as fast as the passes (geometric mean 1.31), slowest where a few more
+// clusters than run at once make a second wave of large CTAs (64 robots of 13^3: 29.3 us against
+// 20.6; one of 16^3, held by 8 of 152 SMs, 7.3 against 6.3).  Chosen by these, with 8% to spare, it is
+// taken in no batch where it was more than 0.4% slower, and the mean is 1.32 (1.33 with the better one
+// each time).  A CTA's step grows with its links; two CTAs share an SM's issue slots (half the slope
+// while they do not); one cluster size goes in whole waves, several sizes fill each other's gaps.
+struct ResLoad {
+    double waves, links;  // bundles by those that run at once; links of a CTA
+    bool whole;           // a CTA has an SM for itself
+};
+double resident_us(const std::vector<ResLoad> &load) {
+    double x = 0, sum = 0, most = 0;
+    for (const ResLoad &l : load) x += l.waves;
+    for (const ResLoad &l : load) {
+        const double t = 3.8 + (l.whole ? 0.0028 : x <= 0.5 ? 0.0025 : 0.0045) * l.links;
+        sum += l.waves * t;
+        most = std::max(most, t);
+    }
+    const double mean = sum / x;
+    if (load.size() == 1) return mean * (x < 6 ? std::ceil(x - 1e-9) : x + 0.5);
+    return x > 0.9 ? std::max(most, mean * (0.75 * x + 1.1)) : most;
+}
+double passes_us(double nv, double nl) {  // launches, then the L2's rate, then that of HBM
+    const double u = nv + nl / 15;
+    return 6.1 + 8.1e-5 * std::min(u, 1.75e5) + 1.73e-4 * std::max(u - 1.75e5, 0.0);
+}
+
 // Whether and how k_steps_mixed steps the batch: mixed precision, whole robots in shared memory.
 // Batches with collisions, force fields, cilia, boundary conditions, signals or a changing link
 // table keep the passes, as does a batch with a robot beyond eight CTAs (about 4,500 voxels).
@@ -374,6 +403,7 @@ int check_math_program(const vx3g_math_token *t, int *len, bool *reads_pos, std:
 // leaves SMs idle: down to 96 voxels per CTA (864 voxels: 3.8 us a step in eight CTAs, 5.4 in four;
 // below 96 the cluster barriers cost more than the shorter phases save: 104 voxels 3.0 us in one
 // CTA, 3.4 in two).  Small robots are bundled up to the same measure.
+// The plan is kept where its estimated step is shorter than the passes' (resident_us, passes_us).
 // lmoff, vmoff: the first link and voxel material of each robot
 int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<int> &vmoff) {
     const Dev &d = c->d;
@@ -432,15 +462,31 @@ int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<
         r = e;
     }
     CU(init_steps_mixed());
+    auto threads = [&](const Plan &p) {
+        int lc = 0;
+        for (const ResBundle &b : p.b) lc = std::max(lc, b.lc);
+        return std::min(std::max(up(lc, 64), 64), p.smem <= kHalf ? kHalfThreads : kResThreads);
+    };
+    std::vector<ResLoad> load;
+    for (int K = kMost; K >= 1; K--) {
+        const Plan &p = by[K - 1];
+        if (p.b.empty()) continue;
+        int act = 0;
+        CU(steps_mixed_active(K, threads(p), p.smem, &act));
+        if (act < 1) return VX3G_OK;
+        double lc = 0;
+        for (const ResBundle &b : p.b) lc += b.lc;
+        load.push_back(ResLoad{(double)p.b.size() / act, lc / p.b.size(), p.smem > kHalf});
+    }
+    if (load.empty() || resident_us(load) > 0.92 * passes_us(d.nv, d.nl)) return VX3G_OK;
     for (int K = kMost; K >= 1; K--) {
         Plan &p = by[K - 1];
         if (p.b.empty()) continue;
         // the longest first: the SMs take the rest as they come free
         std::stable_sort(p.b.begin(), p.b.end(), [](const ResBundle &a, const ResBundle &b) { return a.nl > b.nl; });
         std::vector<int2> ctas, links;
-        int lc = 0, at = 0;
+        int at = 0;
         for (const ResBundle &b : p.b) {
-            lc = std::max(lc, b.lc);
             for (int j = 0; j < K; j++) {
                 const int a = std::min(b.v0 + j * b.q, b.v0 + b.nv), z = std::min(a + b.q, b.v0 + b.nv);
                 const int l0 = link_at(b, a), l1 = link_at(b, z);
@@ -459,8 +505,7 @@ int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<
             return rc;
         CU(launch_res_order(d, pl, pc, (int)ctas.size(), po, c->stream));
         CU(cudaStreamSynchronize(c->stream));  // the host vectors end here
-        const int t = std::min(std::max(up(lc, 64), 64), p.smem <= kHalf ? kHalfThreads : kResThreads);
-        c->res.push_back(ResClass{K, t, (int)p.b.size(), p.smem, pb, pc, po});
+        c->res.push_back(ResClass{K, threads(p), (int)p.b.size(), p.smem, pb, pc, po});
     }
     // the cluster sizes run side by side, the first on the context's own stream
     if (c->res.size() > 1) {

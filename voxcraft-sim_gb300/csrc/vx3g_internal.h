@@ -330,6 +330,8 @@ constexpr int kResSteps = 256;         // most steps of one launch (about 20 ms 
 constexpr int kResSmem = 227 * 1024;   // a CTA's shared memory
 size_t steps_mixed_bytes(int q, int lc);
 cudaError_t init_steps_mixed();
+// clusters of K CTAs that run at once
+cudaError_t steps_mixed_active(int K, int threads, size_t smem, int *n);
 // ResClass::order from each CTA's links (first, end) and its entries
 cudaError_t launch_res_order(const Dev &d, const int2 *links, const int2 *ctas, int n, int *order, cudaStream_t s);
 cudaError_t launch_steps_mixed(const Dev &d, int parity, int n, const ResClass &c, cudaStream_t s);

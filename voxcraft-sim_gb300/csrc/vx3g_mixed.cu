@@ -759,6 +759,21 @@ cudaError_t init_steps_mixed() {
     return e;
 }
 
+cudaError_t steps_mixed_active(int K, int threads, size_t smem, int *n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)K);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)K;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return K > 1 ? cudaOccupancyMaxActiveClusters(n, k_steps_mixed<true>, &cfg)
+                 : cudaOccupancyMaxActiveClusters(n, k_steps_mixed<false>, &cfg);
+}
+
 cudaError_t launch_steps_mixed(const Dev &d, int parity, int n, const ResClass &c, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(c.count * c.K));
