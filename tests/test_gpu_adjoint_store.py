@@ -4,10 +4,7 @@ a next run of the same lengths.  Any interval gives the same gradient: the store
 bits, and an interval of one step has no joined launch at all.  Contraction in the two compiled forms
 may round differently: 1e-16 of each of some 100 terms per step, 60 steps, with cancellations of up to
 1e3 in a sum: 1e-9 of the largest entry.  A second run on the same context repeats the same launches
-from the same states: equal bits.
-
-Without collisions: the order of a voxel's contact candidates, and with it the rounding of its contact
-force, differs between two equal runs, forward ones too, so no two of those need agree to rounding."""
+from the same states: equal bits."""
 
 import numpy as np
 import pytest
@@ -18,23 +15,23 @@ from vx3g import workloads as wl
 pytestmark = pytest.mark.gpu
 
 
-def _robots():
+def _robots(collide):
     out = []
     for i, dims in enumerate([(1, 1, 1), (5, 4, 3), (9, 7, 6)]):  # one voxel, under and over one warp's links
         rng = np.random.default_rng(i)
         mats = [wl.Material(E=2e5, nu=0.35, cte=0.01),
                 wl.Material(E=1e6, nu=0.0, cte=0.01, fail_stress=1e5)]  # some links fail
         out.append(wl.bernoulli_body(rng, dims, 0.85, mats, random_phase=True, temp_vary=True, temp_amplitude=39.0,
-                                     enable_collision=False, enable_expansion=1))
+                                     enable_collision=collide, enable_expansion=1))
     return out
 
 
 W = np.array([[-1.0, 0.5, 0.25]] * 3)
 
 
-@pytest.mark.parametrize("n", [1, 20, 60])
-def test_intervals_and_repeated_runs(n):
-    robots = _robots()
+@pytest.mark.parametrize("n,collide", [(1, False), (20, False), (60, False), (20, True), (60, True)])
+def test_intervals_and_repeated_runs(n, collide):
+    robots = _robots(collide)
 
     def run(b, k):
         b.record(n, k)
