@@ -1139,6 +1139,10 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     // all go out at once (256 colliding robots 161.2 -> 157.5 us a step, a 64^3 body 45.4 -> 44.5,
     // against (256, 1) for both; with (64, 14) for voxels 158.7 and 45.3)
     c->shape_links = 1;
+    // ... except on a state well beyond the L2 without collisions, where the voxel pass wants more blocks
+    // in flight: a step of 270,000 voxels 48.1 us with (256, 1) and 45.7 with (64, 14), of 405,000 80.3 and
+    // 77.2, of 823,000 156.0 and 157.0; of 216,000 31.9 and 32.7, below that now one and now the other
+    if (!d.ns && d.nv >= 240000) c->shape_voxels = 4;
 
     // (c->ends holds the lattice's links alone here: no attachment)
     if (d.mixed && !d.ns && !d.any_dyn && !c->any_ff && !c->any_cilia && !c->any_bcs && !c->any_signals && (rc = plan_resident(c, lmoff, vmoff)))
