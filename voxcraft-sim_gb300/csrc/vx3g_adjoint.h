@@ -16,7 +16,8 @@ struct Snap {
     float2 *strain;
     uint2 *linfo;
     double *T;        // 2*NR
-    int *status;      // NR
+    int *status;      // NR; in the recompute store: at the end of the step, so that a step in which a
+                      // robot stopped passes its gradient through
     // recompute store (NULL elsewhere): per voxel the link force, the link moment and, with
     // collisions, the contact force of the step from this state, kept instead of computed again
     // (six or nine component-major arrays)

@@ -1008,6 +1008,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     d.act = nullptr;
     d.actv = nullptr;
     d.fsum = nullptr;
+    d.fstat = nullptr;
     d.nlm = (int)lmats.size();
     d.nvm = (int)vmats.size();
     float4 *lrow = nullptr, *vrow = nullptr;
@@ -1959,8 +1960,10 @@ cudaError_t enqueue_adj_segment(vx3g_ctx *c, const AdjBufs &a0, int len, int p0)
     for (int i = 0; i < len && e == cudaSuccess; i++) {
         launch_snap_copy(c->rec_store[i].s, live, d.nv, d.nl, d.nr, c->stream);
         c->d.fsum = c->rec_store[i].s.fsum;
+        c->d.fstat = c->rec_store[i].s.status;
         e = enqueue_step(c, (p0 + i) & 1);
         c->d.fsum = nullptr;
+        c->d.fstat = nullptr;
     }
     AdjBufs a = a0;
     // per reverse step: the gather of the step after with the voxel adjoint, the link adjoint and,

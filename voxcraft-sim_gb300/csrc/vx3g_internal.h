@@ -188,6 +188,7 @@ struct Dev {
     double4 *act;
     double2 *actv;
     double *fsum;  // where the FP64 voxel pass keeps its sums (Snap::fsum), or NULL
+    int *fstat;    // with fsum: where it marks the robots that stopped in the step (Snap::status)
     // mixed contexts: the rows of the nlm link and nvm voxel materials (vx3g_mixed_math.cuh)
     const float4 *lrow, *vrow;
     int nlm, nvm;

@@ -710,7 +710,12 @@ template <class R> __device__ __forceinline__ void voxel_update(const Dev &d, in
     const float dtf = d.dt[r];
     const double dt = widen(dtf), tn = Tcur + dt;
     if (v == rp.voff) d.T[(size_t)(parity ^ 1) * d.nr + r] = (st == 0) ? tn : Tcur;  // currentTime += dt
-    if (st != 0) return;
+    if (st != 0) {
+        // the backward pass's recompute: a robot that stopped in this step did not take it, and has no
+        // sums here.  The stored state was copied before; from now on it too says that the robot is stopped.
+        if (d.fsum && v == rp.voff) d.fstat[r] = st;
+        return;
+    }
     uint32_t fl = vi.y;
     if (fl & VF_FIXED) return;
     const VMat &m = d.vmat[fl >> 8];
