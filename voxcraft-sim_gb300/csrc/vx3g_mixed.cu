@@ -446,8 +446,13 @@ struct ResRobot {
     float2 tc[2];    // actuation cycles by parity
     double inv_period;
     float dt, cyc_rate, amp;
-    int status, actuated, expansion, floor;
+    int status;  // with kTorn, a link tore in this step: its voxels stay, and at the end of the step it is stopped
+    int actuated, expansion, floor;
 };
+// The link phase takes no notice of kTorn, so that a step in which a robot diverges updates all of its
+// links, as the reference does, whichever warp finds the torn one first; and a status without it
+// changes between the voxel phase's barriers only.
+constexpr int kTorn = 1 << 30;
 // A CTA's arrays, all computed from q (voxels) and lc (links), multiples of 16.  Float4 planes of q:
 // position hi, lo, orientation hi, lo, six force rows; then the link and material rows and the
 // robots; then float2, float and byte planes.
@@ -513,7 +518,7 @@ __device__ __forceinline__ void res_link(const Dev &d, const ResSmem &S, const R
     const int ip = (int)(e >> 16) - vb;
     int in = (int)(e & 0xffffu) - vb, own = rank;
     ResRobot &R = S.rob(S.rb(ip));
-    if (R.status != 0) return;
+    if (R.status & ~kTorn) return;
     if (CLUSTER && in < 0) {  // the negative end is in a CTA of lower rank
         own = (int)(e & 0xffffu) / q;
         in = (int)(e & 0xffffu) - own * q;
@@ -546,9 +551,9 @@ __device__ __forceinline__ void res_link(const Dev &d, const ResSmem &S, const R
     S.SB(2 * axis + 1, ip) = make_float2(f.mP.y, f.mP.z);
     if (diverged) {
         atomicOr(&d.status[B.r0 + S.rb(ip)], 1);
-        if (!CLUSTER) atomicOr(&R.status, 1);
+        if (!CLUSTER) atomicOr(&R.status, kTorn);
         else
-            for (int k = 0; k < K; k++) atomicOr(res_map(&R.status, k), 1);
+            for (int k = 0; k < K; k++) atomicOr(res_map(&R.status, k), kTorn);
     }
 }
 
@@ -669,8 +674,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_steps_mixed(Dev d, int parit
     }
     res_sync<CLUSTER>();
     unsigned stopped = 0;  // robots that were not running when the launch began
-    for (int i = 0; i < B.nr; i++) stopped |= (unsigned)(S.rob(i).status != 0) << i;
-    if (CLUSTER) res_sync<CLUSTER>();  // before any CTA can mark a robot in another's copy
+    for (int i = 0; i < B.nr; i++) stopped |= (unsigned)((S.rob(i).status & ~kTorn) != 0) << i;
     for (int s = 0; s < n; s++, parity ^= 1) {
         for (int i = tid; i < nl; i += T) res_link<CLUSTER>(d, S, B, i, lid + i, rank, K);
         res_sync<CLUSTER>();
@@ -681,6 +685,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_steps_mixed(Dev d, int parit
             const double Tn = R.status == 0 ? R.T[parity] + R.dt : R.T[parity];
             R.T[parity ^ 1] = Tn;
             R.tc[parity ^ 1] = mx::cycles_df(Tn * R.inv_period * kCycle);
+            if (R.status & kTorn) R.status = (R.status & ~kTorn) | 1;
         }
         res_sync<CLUSTER>();
     }
