@@ -1301,7 +1301,10 @@ cudaError_t init_collision(Dev &d) {
     d.cgrid = 0;
     if (!d.ns) return cudaSuccess;
     const size_t sm = coll_prepare_smem(d);
-    cudaError_t e = cudaFuncSetAttribute(k_coll_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    // the most any context asks for: the limit belongs to the process, and a context made later must not
+    // lower it for those before
+    cudaError_t e = cudaFuncSetAttribute(k_coll_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)local_list_smem(kLocalListMax));
     if (e != cudaSuccess) return e;
     int dev = 0, nsm = 0, occ = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
