@@ -239,7 +239,7 @@ struct vx3g_ctx {
     std::vector<int> vmat_local, surface;
     std::vector<unsigned char> vfixed;
     int64_t steps = 0;
-    int shape_links = 0, shape_voxels = 0;  // launch shapes of the mixed passes (vx3g_autotune)
+    int shape_links = kDefaultShape, shape_voxels = kDefaultShape;  // launch shapes of the mixed passes (vx3g_autotune)
     bool ff_pos = false;  // some robot's force field reads the voxel position
     bool any_ff = false;  // some robot has a force field
     bool any_cilia = false;  // some robot has cilia
@@ -1136,15 +1136,6 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         // body rarely does (a folded 64^3 body 54.4 us a step against 55.8 so)
         c->fork_early = d.nhash == 0 ? 1 : 0;
     }
-    // launch shapes until vx3g_autotune is called: (256, 4) for links, (256, 1) for voxels, whose loads
-    // all go out at once (256 colliding robots 161.2 -> 157.5 us a step, a 64^3 body 45.4 -> 44.5,
-    // against (256, 1) for both; with (64, 14) for voxels 158.7 and 45.3)
-    c->shape_links = 1;
-    // ... except on a state well beyond the L2 without collisions, where the voxel pass wants more blocks
-    // in flight: a step of 270,000 voxels 48.1 us with (256, 1) and 45.7 with (64, 14), of 405,000 80.3 and
-    // 77.2, of 823,000 156.0 and 157.0; of 216,000 31.9 and 32.7, below that now one and now the other
-    if (!d.ns && d.nv >= 240000) c->shape_voxels = 4;
-
     // (c->ends holds the lattice's links alone here: no attachment)
     if (d.mixed && !d.ns && !d.any_dyn && !c->any_ff && !c->any_cilia && !c->any_bcs && !c->any_signals && (rc = plan_resident(c, lmoff, vmoff)))
         return rc;
@@ -1733,7 +1724,7 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
     CU(cudaSetDevice(c->device));
     cudaDeviceProp prop;
     CU(cudaGetDeviceProperties(&prop, c->device));
-    const std::string key = std::string(prop.name) + "|mixed|" + std::to_string(c->d.nv) + "|" +
+    const std::string key = std::string(prop.name) + "|mixed " + std::to_string(kMixedShapes) + "|" + std::to_string(c->d.nv) + "|" +
                             std::to_string(c->d.nl) + "|" + std::to_string(c->d.ns);
     std::string cache;
     if (cache_json) {
@@ -1761,7 +1752,7 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
     }
     // time the passes of real steps, cycling through the shapes (results do not depend on them),
     // then whole steps alternating the fork point of the overlapped step
-    const int warm = 2 * kMixedShapes;
+    const int warm = kMixedShapes;
     if (n_steps < warm + 2 * kMixedShapes) return vx3g_step(c, n_steps);
     const int n_fork = c->overlap && n_steps >= 2 * (warm + 2 * kMixedShapes) ? std::min(n_steps / 2, 64) : 0;
     const int n_shape = n_steps - n_fork;

@@ -304,7 +304,7 @@ void launch_fp64_tables(const Dev &d, LMatD *lmatd, const int *lrob, int n, cuda
 void launch_actuation(const Dev &d, int parity, cudaStream_t s);
 // launch shapes of the mixed-precision passes (vx3g_mixed.cu), chosen by vx3g_autotune
 struct LaunchShape { int threads, min_blocks; };
-constexpr int kMixedShapes = 6;
+constexpr int kMixedShapes = 8, kDefaultShape = 6;
 extern const LaunchShape kLinkShapes[kMixedShapes], kVoxelShapes[kMixedShapes];
 // pdl = false when the kernel before it wrote link info (removal): no early start
 void launch_links_mixed(const Dev &d, cudaStream_t s, int shape = 0, bool pdl = true);

@@ -142,19 +142,42 @@ __device__ __forceinline__ void pdl_wait_then_release() {
 }
 
 // ------------------------------------------------------------- link pass
-__device__ __forceinline__ void links_mixed_body(const Dev &d, int l) {
+struct LinkOut {  // where the link pass leaves a link's update (mx::link_step)
+    const Dev &d;
+    int l, axis, r;
+    int2 e;
+    uint32_t fl;
+    __device__ __forceinline__ void local(V3<float> pos2, V3<float> a1v, V3<float> a2v, bool small) {
+        mixed_lstate_a(d)[l] = make_float4(pos2.x, pos2.y, pos2.z, a2v.x);
+        mixed_lstate_b(d)[l] = make_float2(a2v.y, a2v.z);
+        if (!(small && (fl & LF_SMALL))) {
+            float *C = mixed_lstate_c(d);
+            const size_t NL = (size_t)d.nl;
+            C[l] = a1v.x, C[NL + l] = a1v.y, C[2 * NL + l] = a1v.z;
+        }
+    }
+    __device__ __forceinline__ void strain(float2 s, bool torn) {
+        d.strain[l] = s;
+        if (torn) atomicOr(&d.status[r], 1);
+    }
+    __device__ __forceinline__ void neg(V3<float> f, V3<float> m) { store_slot_mx(d, 2 * axis, e.x, f, m); }
+    __device__ __forceinline__ void pos(V3<float> f, V3<float> m) { store_slot_mx(d, 2 * axis + 1, e.y, f, m); }
+    __device__ __forceinline__ void flags(uint32_t nfl, bool failed) {
+        if ((fl & LF_RUNTIME) && !failed) new_link_scale_mx(d, l, 2 * axis, e.x, e.y);
+        if (nfl != fl) d.linfo[l].y = nfl;
+    }
+};
+template <bool HELD> __device__ __forceinline__ void links_mixed_body(const Dev &d, int l) {
     // every load that depends only on l is issued before the first branch, then the
     // endpoint state: two dependent load levels instead of four (latency-bound kernel)
     const uint2 li = d.linfo[l];
     const int2 e = d.ends[l];
     // link state (mixed precision): a 16-byte row {pos2, angle2v.x} and an 8-byte row
     // {angle2v.y, angle2v.z} per link, then angle1v component-major (mixed_lstate_*)
-    float4 *lsA = mixed_lstate_a(d);
-    float2 *lsB = mixed_lstate_b(d);
-    float *lsC = mixed_lstate_c(d);
+    const float *lsC = mixed_lstate_c(d);
     const size_t NL = (size_t)d.nl;
-    const float4 sa = lsA[l];
-    const float2 sb = lsB[l];
+    const float4 sa = mixed_lstate_a(d)[l];
+    const float2 sb = mixed_lstate_b(d)[l];
     // angle1v is zero while a link is in the small-angle branch (the flag it entered
     // this step with says so); it is read and written only for large-angle links and
     // zeroed once when a link returns to the small branch
@@ -170,21 +193,8 @@ __device__ __forceinline__ void links_mixed_body(const Dev &d, int l) {
     if (d.status[r] != 0) return;
     const uint32_t fl = li.y;
     if (fl & (LF_BOTH_FIXED | LF_GONE)) return;
-    const int axis = fl & LF_AXIS;
-    mx::LinkForces f;
-    bool diverged;
-    mx::link_step(d, mx::link_rows(d.lrow, d.nlm, (int)(fl >> 8)), l, en, ep, s, f, diverged);
-    lsA[l] = make_float4(s.pos2.x, s.pos2.y, s.pos2.z, s.a2v.x);
-    lsB[l] = make_float2(s.a2v.y, s.a2v.z);
-    if (!((s.fl & LF_SMALL) && wasSmall)) {
-        lsC[l] = s.a1v.x; lsC[NL + l] = s.a1v.y; lsC[2 * NL + l] = s.a1v.z;
-    }
-    d.strain[l] = s.strain;
-    if (diverged) atomicOr(&d.status[r], 1);
-    store_slot_mx(d, 2 * axis, e.x, f.fN, f.mN);
-    store_slot_mx(d, 2 * axis + 1, e.y, f.fP, f.mP);
-    if ((fl & LF_RUNTIME) && (s.fl & LF_LVV)) new_link_scale_mx(d, l, 2 * axis, e.x, e.y);
-    if (s.fl != fl) d.linfo[l].y = s.fl;
+    LinkOut out{d, l, (int)(fl & LF_AXIS), r, e, fl};
+    mx::link_step(d, mx::link_rows<HELD>(d.lrow, d.nlm, (int)(fl >> 8)), l, en, ep, s, out);
 }
 
 __global__ void k_init_temperature_mixed(Dev d) {
@@ -197,7 +207,7 @@ __global__ void k_init_temperature_mixed(Dev d) {
     if (rp.vary_temp && rp.temp_period > 0 && !(m.thermal_on_after > 0.0) && !m.fixed)
         te = mx::temperature(make_float2(0.0f, 0.0f), d.phc[v], 0.0f, rp.cyc_rate, rp.amp_f, rp.expansion != 0);
     float4 *P = reinterpret_cast<float4 *>(d.pos);
-    mx::base_size(mx::vox_consts_mx(m), te, P[2 * v].w, P[2 * v + 1].w);
+    mx::base_size(mx::vox_row_c(m), te, P[2 * v].w, P[2 * v + 1].w);
     d.tempe[v] = te;
     d.tempe[d.nv + v] = te;
 }
@@ -228,7 +238,8 @@ __device__ __forceinline__ void set_df(float &hi, float &lo, double x) {
 // compiles without the external code).  BC = true: the voxels with one (Dev::xbc), after
 // the main pass, with the external force and moment, the fixed DOFs and the fixed-all
 // pose (VX3_Voxel.cu:167-173, 222-257, 363-364, 393-394).
-template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &d, int v, int parity) {
+// EARLY: with registers for every load at once (the launch shapes of 96 registers and more)
+template <bool BC, bool EARLY> __device__ __forceinline__ void voxels_mixed_body(const Dev &d, int v, int parity) {
     // the voxel's own state is loaded together with its info word, before any branch
     // (latency-bound kernel: one dependent level fewer)
     const uint2 vi = d.vinfo[v];
@@ -238,19 +249,35 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
     float4 *AM = reinterpret_cast<float4 *>(d.angmom);
     mx::VoxelState s{P[2 * v], P[2 * v + 1], Qa[2 * v], Qa[2 * v + 1], LM[2 * v], LM[2 * v + 1], AM[2 * v], AM[2 * v + 1]};
     pdl_wait_then_release();  // the link pass (or the contact evaluation) of this step is done
-    // what depends on the voxel's number alone, beside the robot's and the materials' loads
     float *tcur = d.tempe + (size_t)parity * d.nv, *tnext = d.tempe + (size_t)(parity ^ 1) * d.nv;
-    float te = tcur[v];
-    const float2 ph = d.phc[v];
-    const float4 ct = d.ns ? reinterpret_cast<const float4 *>(d.contact)[v] : make_float4(0, 0, 0, 0);
-    const int si = d.vsurf ? d.vsurf[v] : -1;
+    float te = 0;
+    float2 ph = make_float2(0, 0);
+    float4 ct = make_float4(0, 0, 0, 0);
+    int si = -1;
+    if (EARLY) {  // what depends on the voxel's number alone, beside the robot's and the materials' loads
+        te = tcur[v];
+        ph = d.phc[v];
+        if (d.ns) ct = reinterpret_cast<const float4 *>(d.contact)[v];
+        if (d.vsurf) si = d.vsurf[v];
+    }
     const int r = (int)vi.x;
     const RobotP &rp = d.rp[r];
     const int st = d.status[r];
     const float dtf = d.dt[r];
     if (!BC && v == rp.voff) advance_time(d, rp, r, parity, dtf, st);
-    if (st != 0) return;
     uint32_t fl = vi.y;
+    // the forces at its faces, with the loads that the checks below wait for
+    V3<float> Fs{0, 0, 0}, Ms{0, 0, 0};
+#pragma unroll
+    for (int dir = 0; dir < 6; dir++) {
+        if (fl & (1u << dir)) {
+            V3<float> sf, sm;
+            load_slot_mx(d, dir, v, &sf, &sm);
+            Fs = add(Fs, sf);
+            Ms = add(Ms, sm);
+        }
+    }
+    if (st != 0) return;
     if (fl & VF_FIXED) return;
     if (!BC && rp.bcs && d.vext[v] >= 0) return;  // stepped by the BC pass
     const mx::VoxC m = mx::vox_rows(d.vrow, d.nvm, (int)(fl >> 8));
@@ -276,16 +303,6 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
         AM[2 * v] = z4;
         AM[2 * v + 1] = z4;
     } else if (dtf != 0.0f) {
-        V3<float> Fs{0, 0, 0}, Ms{0, 0, 0};
-#pragma unroll
-        for (int dir = 0; dir < 6; dir++) {
-            if (fl & (1u << dir)) {
-                V3<float> sf, sm;
-                load_slot_mx(d, dir, v, &sf, &sm);
-                Fs = add(Fs, sf);
-                Ms = add(Ms, sm);
-            }
-        }
         bool stat = (fl & VF_STATIC) != 0;
         const bool floorOn = rp.floor != 0;
         const Q4<float> o{s.qH.x, s.qH.y, s.qH.z, s.qH.w};
@@ -293,8 +310,11 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
         if (BC) F = add(F, V3<float>{d.ext[xi].f[0], d.ext[xi].f[1], d.ext[xi].f[2]});  // external force
         const V3<float> vel = mx::velocity(s.lH, s.lL, m.a.x);
         F = mx::fma3(-m.a.z, vel, F);
-        F.z = mx::plus(F.z, m.b.y);
-        if (rp.collision) F = mx::diff(F, V3<float>{ct.x, ct.y, ct.z});
+        F.z = mx::plus(F.z, m.c.x);
+        if (rp.collision) {
+            if (!EARLY && d.ns) ct = reinterpret_cast<const float4 *>(d.contact)[v];
+            F = mx::diff(F, V3<float>{ct.x, ct.y, ct.z});
+        }
         if (rp.cilia) {  // CiliaForce * Cilia (VX3_Voxel.cu:376), evaluated in FP64 by k_extra_forces
             const double4 c = d.cfv[v];
             F = add(F, V3<float>{(float)c.x, (float)c.y, (float)c.z});
@@ -345,9 +365,10 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
         AM[2 * v + 1] = s.aL;
     }
     if (actuated) {  // next step's temperature and base size
+        if (!EARLY) te = tcur[v], ph = d.phc[v];
         if (m.a.y > 0.0f || thermal_on(d, d.vmat[fl >> 8].thermal_on_after, r, parity, dtf))
             te = mx::temperature(d.tcyc[(size_t)parity * d.nr + r], ph, dtf, rp.cyc_rate, rp.amp_f, rp.expansion != 0);
-        mx::base_size(m, te, s.pH.w, s.pL.w);
+        mx::base_size(m.c, te, s.pH.w, s.pL.w);
         tnext[v] = te;
     }
     P[2 * v] = s.pH;
@@ -355,11 +376,13 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
     // the next step's displacement check (k_coll_check), while the voxel is at hand: 64 bytes written
     // instead of a kernel that reads 80 and writes 64 (2.3 us of a 64^3 body's step, 9 us of 256
     // colliding robots')
+    if (!EARLY && d.vsurf) si = d.vsurf[v];
     if (si >= 0) {
         const float4 q = d.cref[si];
         const float px = mx::plus(s.pH.x, s.pL.x), py = mx::plus(s.pH.y, s.pL.y), pz = mx::plus(s.pH.z, s.pL.z);
         d.cposf[si] = make_float4(px, py, pz, mx::plus(s.pH.w, s.pL.w));
-        contact_record(d, v, s.pH, s.pL, s.lH, m.a.x, m.b.z, m.b.x);
+        const float4 mb = m.b();
+        contact_record(d, v, s.pH, s.pL, s.lH, m.a.x, mb.z, mb.x);
         const float ex = mx::minus(px, q.x), ey = mx::minus(py, q.y), ez = mx::minus(pz, q.z);
         if (fmaf(ez, ez, mx::dot_a(ex, ex, ey, ey)) > q.w) flag_robot(d, r);
     }
@@ -368,28 +391,34 @@ template <bool BC> __device__ __forceinline__ void voxels_mixed_body(const Dev &
 // the voxels with a boundary-condition external, after the main voxel pass
 __global__ void __launch_bounds__(128) k_voxels_bc_mixed(Dev d, int parity) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < d.nxbc) voxels_mixed_body<true>(d, d.xbc[i], parity);
+    if (i < d.nxbc) voxels_mixed_body<true, false>(d, d.xbc[i], parity);
 }
 
 void launch_voxels_bc_mixed(const Dev &d, int parity, cudaStream_t s) {
     if (d.nxbc) k_voxels_bc_mixed<<<(d.nxbc + 127) / 128, 128, 0, s>>>(d, parity);
 }
 
-// Launch-shape variants (threads per block, minimum resident blocks): the same body,
-// so every variant computes bit-identical results; they trade registers for
-// occupancy (both passes are latency-bound gathers).  vx3g_autotune picks one per
-// context by timing real steps.
-template <int TPB, int MINB> __global__ void __launch_bounds__(TPB, MINB) k_links_mixed(Dev d) {
+// Launch-shape variants (threads per block, minimum resident blocks): the same body, so every variant
+// computes bit-identical results; they trade registers for occupancy (both passes are latency-bound
+// gathers), and vx3g_autotune picks one of each per context by timing real steps.  HELD: a link's material
+// rows are loaded with its ends and kept; EARLY: see voxels_mixed_body.
+// Shape 6 of each is the default: small blocks, so that an SM's places are refilled a few warps at a time,
+// and every load of a thread out at once.  Steps of 822,751 voxels / 410,307 / 262,144 / 32,768 / 13,824 without
+// collisions, in us: shapes (6, 6) 143.8, 73.9, 45.6, 8.3, 5.8; (1, 0), in blocks of 256, 145.8, 76.5, 47.9, 10.0,
+// 7.6; (1, 4), the voxel's loads held back until they are used to fit 72 registers, 151.5, 78.6, 46.0, 10.2, 9.3.
+// A link's material rows held or not: 143.8 and 141.6, 73.9 and 74.0, 45.6 and 46.3, 8.3 and 8.7, 5.8 and 6.3.
+// With collisions: a 64^3 body 41.1 us a step early in a run with (6, 6), 43.0 with (1, 0); 256 robots 136.7, 146.2.
+template <int TPB, int MINB, bool HELD> __global__ void __launch_bounds__(TPB, MINB) k_links_mixed(Dev d) {
     const int l = blockIdx.x * TPB + threadIdx.x;
-    if (l < d.nl) links_mixed_body(d, l);
+    if (l < d.nl) links_mixed_body<HELD>(d, l);
 }
-template <int TPB, int MINB> __global__ void __launch_bounds__(TPB, MINB) k_voxels_mixed(Dev d, int parity) {
+template <int TPB, int MINB, bool EARLY> __global__ void __launch_bounds__(TPB, MINB) k_voxels_mixed(Dev d, int parity) {
     const int v = blockIdx.x * TPB + threadIdx.x;
-    if (v < d.nv) voxels_mixed_body<false>(d, v, parity);
+    if (v < d.nv) voxels_mixed_body<false, EARLY>(d, v, parity);
 }
 
-const LaunchShape kLinkShapes[kMixedShapes] = {{256, 1}, {256, 4}, {128, 9}, {128, 10}, {64, 20}, {256, 5}};
-const LaunchShape kVoxelShapes[kMixedShapes] = {{256, 1}, {256, 3}, {128, 7}, {128, 8}, {64, 14}, {64, 16}};
+const LaunchShape kLinkShapes[kMixedShapes] = {{256, 1}, {256, 4}, {128, 9}, {128, 10}, {64, 20}, {256, 5}, {128, 8}, {128, 8}};
+const LaunchShape kVoxelShapes[kMixedShapes] = {{256, 1}, {256, 3}, {128, 7}, {128, 8}, {64, 14}, {64, 16}, {64, 8}, {64, 10}};
 
 // launch with programmatic stream serialization (see pdl_wait_then_release)
 template <typename... KArgs, typename... Args>
@@ -409,23 +438,27 @@ static void launch_pdl(void (*kernel)(KArgs...), int n, int threads, cudaStream_
 void launch_links_mixed(const Dev &d, cudaStream_t s, int shape, bool pdl) {
     if (!d.nl) return;
     switch (shape) {
-        case 1: launch_pdl(k_links_mixed<256, 4>, d.nl, 256, s, pdl, d); break;
-        case 2: launch_pdl(k_links_mixed<128, 9>, d.nl, 128, s, pdl, d); break;
-        case 3: launch_pdl(k_links_mixed<128, 10>, d.nl, 128, s, pdl, d); break;
-        case 4: launch_pdl(k_links_mixed<64, 20>, d.nl, 64, s, pdl, d); break;
-        case 5: launch_pdl(k_links_mixed<256, 5>, d.nl, 256, s, pdl, d); break;
-        default: launch_pdl(k_links_mixed<256, 1>, d.nl, 256, s, pdl, d); break;
+        case 0: launch_pdl(k_links_mixed<256, 1, true>, d.nl, 256, s, pdl, d); break;
+        case 1: launch_pdl(k_links_mixed<256, 4, false>, d.nl, 256, s, pdl, d); break;
+        case 2: launch_pdl(k_links_mixed<128, 9, false>, d.nl, 128, s, pdl, d); break;
+        case 3: launch_pdl(k_links_mixed<128, 10, false>, d.nl, 128, s, pdl, d); break;
+        case 4: launch_pdl(k_links_mixed<64, 20, false>, d.nl, 64, s, pdl, d); break;
+        case 5: launch_pdl(k_links_mixed<256, 5, false>, d.nl, 256, s, pdl, d); break;
+        case 6: launch_pdl(k_links_mixed<128, 8, true>, d.nl, 128, s, pdl, d); break;
+        default: launch_pdl(k_links_mixed<128, 8, false>, d.nl, 128, s, pdl, d); break;
     }
 }
 void launch_voxels_mixed(const Dev &d, int parity, cudaStream_t s, int shape, bool pdl) {
     if (!d.nv) return;
     switch (shape) {
-        case 1: launch_pdl(k_voxels_mixed<256, 3>, d.nv, 256, s, pdl, d, parity); break;
-        case 2: launch_pdl(k_voxels_mixed<128, 7>, d.nv, 128, s, pdl, d, parity); break;
-        case 3: launch_pdl(k_voxels_mixed<128, 8>, d.nv, 128, s, pdl, d, parity); break;
-        case 4: launch_pdl(k_voxels_mixed<64, 14>, d.nv, 64, s, pdl, d, parity); break;
-        case 5: launch_pdl(k_voxels_mixed<64, 16>, d.nv, 64, s, pdl, d, parity); break;
-        default: launch_pdl(k_voxels_mixed<256, 1>, d.nv, 256, s, pdl, d, parity); break;
+        case 0: launch_pdl(k_voxels_mixed<256, 1, true>, d.nv, 256, s, pdl, d, parity); break;
+        case 1: launch_pdl(k_voxels_mixed<256, 3, false>, d.nv, 256, s, pdl, d, parity); break;
+        case 2: launch_pdl(k_voxels_mixed<128, 7, false>, d.nv, 128, s, pdl, d, parity); break;
+        case 3: launch_pdl(k_voxels_mixed<128, 8, false>, d.nv, 128, s, pdl, d, parity); break;
+        case 4: launch_pdl(k_voxels_mixed<64, 14, false>, d.nv, 64, s, pdl, d, parity); break;
+        case 5: launch_pdl(k_voxels_mixed<64, 16, false>, d.nv, 64, s, pdl, d, parity); break;
+        case 6: launch_pdl(k_voxels_mixed<64, 8, true>, d.nv, 64, s, pdl, d, parity); break;
+        default: launch_pdl(k_voxels_mixed<64, 10, true>, d.nv, 64, s, pdl, d, parity); break;
     }
 }
 // ------------------------------------------------------------ many steps in one launch
@@ -509,6 +542,39 @@ template <class T> __device__ __forceinline__ T *res_map(T *p, int k) {
     return q;
 }
 
+template <bool CLUSTER> struct ResLinkOut {  // where k_steps_mixed leaves a link's update (mx::link_step)
+    const Dev &d;
+    const ResSmem &S;
+    int i, axis, in, ip, own, rank, K, r0;
+    uint32_t fl;
+    __device__ __forceinline__ void local(V3<float> pos2, V3<float> a1v, V3<float> a2v, bool small) {
+        S.LA(i) = make_float4(pos2.x, pos2.y, pos2.z, a2v.x);
+        S.LB(i) = make_float2(a2v.y, a2v.z);
+        if (!(small && (fl & LF_SMALL))) S.LC(0, i) = a1v.x, S.LC(1, i) = a1v.y, S.LC(2, i) = a1v.z;
+    }
+    __device__ __forceinline__ void strain(float2 s, bool torn) {
+        S.ST(i) = s;
+        if (!torn) return;
+        const int k = S.rb(ip);
+        atomicOr(&d.status[r0 + k], 1);
+        if (!CLUSTER) atomicOr(&S.rob(k).status, kTorn);
+        else
+            for (int c = 0; c < K; c++) atomicOr(res_map(&S.rob(k).status, c), kTorn);
+    }
+    __device__ __forceinline__ void neg(V3<float> f, V3<float> m) {
+        float4 *a = &S.SA(2 * axis, in);
+        float2 *b = &S.SB(2 * axis, in);
+        if (CLUSTER && own != rank) a = res_map(a, own), b = res_map(b, own);
+        *a = make_float4(f.x, f.y, f.z, m.x);
+        *b = make_float2(m.y, m.z);
+    }
+    __device__ __forceinline__ void pos(V3<float> f, V3<float> m) {
+        S.SA(2 * axis + 1, ip) = make_float4(f.x, f.y, f.z, m.x);
+        S.SB(2 * axis + 1, ip) = make_float2(m.y, m.z);
+    }
+    __device__ __forceinline__ void flags(uint32_t nfl, bool) { S.fl(i) = nfl; }
+};
+
 template <bool CLUSTER>
 __device__ __forceinline__ void res_link(const Dev &d, const ResSmem &S, const ResBundle &B, int i, const int *lid, int rank, int K) {
     const uint32_t fl = S.fl(i);
@@ -517,8 +583,7 @@ __device__ __forceinline__ void res_link(const Dev &d, const ResSmem &S, const R
     const uint32_t e = S.le(i);
     const int ip = (int)(e >> 16) - vb;
     int in = (int)(e & 0xffffu) - vb, own = rank;
-    ResRobot &R = S.rob(S.rb(ip));
-    if (R.status & ~kTorn) return;
+    if (S.rob(S.rb(ip)).status & ~kTorn) return;
     if (CLUSTER && in < 0) {  // the negative end is in a CTA of lower rank
         own = (int)(e & 0xffffu) / q;
         in = (int)(e & 0xffffu) - own * q;
@@ -530,31 +595,11 @@ __device__ __forceinline__ void res_link(const Dev &d, const ResSmem &S, const R
     const mx::Ends ep{S.PH(ip), S.PL(ip), S.QH(ip), S.QL(ip)};
     const float4 sa = S.LA(i);
     const float2 sb = S.LB(i);
-    const bool wasSmall = (fl & LF_SMALL) != 0;
     mx::LinkState st{{sa.x, sa.y, sa.z}, {0, 0, 0}, {sa.w, sb.x, sb.y}, S.ST(i), fl};
-    if (!wasSmall) st.a1v = V3<float>{S.LC(0, i), S.LC(1, i), S.LC(2, i)};
-    mx::LinkForces f;
-    bool diverged;
+    if (!(fl & LF_SMALL)) st.a1v = V3<float>{S.LC(0, i), S.LC(1, i), S.LC(2, i)};
     const int lm = (int)(fl >> 8);
-    mx::link_step(d, B.nlm ? mx::link_rows(&S.lrow(0), B.nlm, lm - B.lm0) : mx::link_rows(d.lrow, d.nlm, lm), *lid, en, ep, st, f,
-                  diverged);
-    S.LA(i) = make_float4(st.pos2.x, st.pos2.y, st.pos2.z, st.a2v.x);
-    S.LB(i) = make_float2(st.a2v.y, st.a2v.z);
-    if (!((st.fl & LF_SMALL) && wasSmall)) S.LC(0, i) = st.a1v.x, S.LC(1, i) = st.a1v.y, S.LC(2, i) = st.a1v.z;
-    S.ST(i) = st.strain;
-    S.fl(i) = st.fl;
-    const float4 na = make_float4(f.fN.x, f.fN.y, f.fN.z, f.mN.x);
-    const float2 nb = make_float2(f.mN.y, f.mN.z);
-    if (CLUSTER && own != rank) *res_map(&S.SA(2 * axis, in), own) = na, *res_map(&S.SB(2 * axis, in), own) = nb;
-    else S.SA(2 * axis, in) = na, S.SB(2 * axis, in) = nb;
-    S.SA(2 * axis + 1, ip) = make_float4(f.fP.x, f.fP.y, f.fP.z, f.mP.x);
-    S.SB(2 * axis + 1, ip) = make_float2(f.mP.y, f.mP.z);
-    if (diverged) {
-        atomicOr(&d.status[B.r0 + S.rb(ip)], 1);
-        if (!CLUSTER) atomicOr(&R.status, kTorn);
-        else
-            for (int k = 0; k < K; k++) atomicOr(res_map(&R.status, k), kTorn);
-    }
+    ResLinkOut<CLUSTER> out{d, S, i, axis, in, ip, own, rank, K, B.r0, fl};
+    mx::link_step(d, B.nlm ? mx::link_rows<true>(&S.lrow(0), B.nlm, lm - B.lm0) : mx::link_rows<true>(d.lrow, d.nlm, lm), *lid, en, ep, st, out);
 }
 
 __device__ __forceinline__ void res_voxel(const Dev &d, const ResSmem &S, const ResBundle &B, int i, int v, int parity, bool last) {
@@ -562,7 +607,8 @@ __device__ __forceinline__ void res_voxel(const Dev &d, const ResSmem &S, const 
     const ResRobot &R = S.rob(S.rb(i));
     if (R.status != 0 || (fl & VF_FIXED)) return;
     const float dtf = R.dt;
-    const mx::VoxC m = B.nvm ? mx::vox_rows(&S.vrow(0), B.nvm, (int)(fl >> 8) - B.vm0) : mx::vox_rows(d.vrow, d.nvm, (int)(fl >> 8));
+    const mx::VoxC m = B.nvm ? mx::vox_rows(&S.vrow(0), B.nvm, (int)(fl >> 8) - B.vm0)
+                             : mx::vox_rows(d.vrow, d.nvm, (int)(fl >> 8));
     mx::VoxelState s;
     s.pH = S.PH(i), s.pL = S.PL(i);
     if (dtf != 0.0f) {
@@ -584,7 +630,7 @@ __device__ __forceinline__ void res_voxel(const Dev &d, const ResSmem &S, const 
         const Q4<float> o{s.qH.x, s.qH.y, s.qH.z, s.qH.w};
         const V3<float> vel = mx::velocity(s.lH, s.lL, m.a.x);
         V3<float> F = mx::fma3(-m.a.z, vel, mx::rotate_voxel(o, Fs));
-        F.z = mx::plus(F.z, m.b.y);
+        F.z = mx::plus(F.z, m.c.x);
         mx::move(s, m, F, vel, R.floor != 0, dtf, stat);
         mx::turn(s, m, mx::fma3(-m.a.w, mx::velocity(s.aH, s.aL, fabsf(m.a.y)), mx::rotate_voxel(o, Ms)), dtf);
         if (R.floor && mx::penetration(s, m) >= 0 && stat) s.aH = s.aL = make_float4(0, 0, 0, 0);
@@ -600,7 +646,7 @@ __device__ __forceinline__ void res_voxel(const Dev &d, const ResSmem &S, const 
         if (last) d.tempe[(size_t)parity * d.nv + v] = te;  // the temperature the last step used
         if (m.a.y > 0.0f || !(d.vmat[fl >> 8].thermal_on_after > R.T[parity] + dtf))
             te = mx::temperature(R.tc[parity], S.ph(i), dtf, R.cyc_rate, R.amp, R.expansion != 0);
-        mx::base_size(m, te, s.pH.w, s.pL.w);
+        mx::base_size(m.c, te, s.pH.w, s.pL.w);
         S.te(i) = te;
     }
     S.PH(i) = s.pH, S.PL(i) = s.pL;
@@ -799,11 +845,11 @@ __global__ void k_rows_mixed(Dev d, float4 *lrow, float4 *vrow, const int *lrob)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < d.nlm) {
         const mx::LinkC c = mx::link_consts_mx(d.lmat[i], d.dt[lrob[i]]);
-        lrow[i] = c.a, lrow[d.nlm + i] = c.b, lrow[2 * (size_t)d.nlm + i] = c.c, lrow[3 * (size_t)d.nlm + i] = c.e;
+        lrow[i] = c.ra, lrow[d.nlm + i] = c.rb, lrow[2 * (size_t)d.nlm + i] = c.rc, lrow[3 * (size_t)d.nlm + i] = c.re;
     }
     if (i < d.nvm) {
-        const mx::VoxC c = mx::vox_consts_mx(d.vmat[i]);
-        vrow[i] = c.a, vrow[d.nvm + i] = c.b, vrow[2 * (size_t)d.nvm + i] = c.c;
+        const VMat &m = d.vmat[i];
+        vrow[i] = mx::vox_row_a(m), vrow[d.nvm + i] = mx::vox_row_b(m), vrow[2 * (size_t)d.nvm + i] = mx::vox_row_c(m);
     }
 }
 void launch_rows_mixed(const Dev &d, float4 *lrow, float4 *vrow, const int *lrob, cudaStream_t s) {

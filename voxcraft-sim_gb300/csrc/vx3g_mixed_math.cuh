@@ -149,35 +149,54 @@ __device__ __forceinline__ Q product_x0(Q a, Q f) {  // a.x = 0
 // material i at [k * count + i]): a warp's lanes pick among a few materials, so a row costs one or
 // two cache lines where the fields of an array of structs cost a line per material and field.
 struct LinkC {
-    float4 a;  // b1, b2, b3, a2
-    float4 b;  // sqA1, sqA2xIp, sqB1, sqB2xFMp
-    float4 c;  // sqB3xIp, the ends' damping multipliers / dt, transverse area (negative: non-linear model)
-    float4 e;  // stress = e.x * (e.y * strain + e.z) of a linear model; failure strain (-1: none)
+    float4 ra;  // b1, b2, b3, a2
+    float4 rb;  // sqA1, sqA2xIp, sqB1, sqB2xFMp
+    float4 rc;  // sqB3xIp, the ends' damping multipliers / dt, transverse area (negative: non-linear model)
+    float4 re;  // stress = e.x * (e.y * strain + e.z) of a linear model; failure strain (-1: none)
+    __device__ __forceinline__ float4 a() const { return ra; }
+    __device__ __forceinline__ float4 b() const { return rb; }
+    __device__ __forceinline__ float4 c() const { return rc; }
+    __device__ __forceinline__ float4 e() const { return re; }
 };
 struct VoxC {
     float4 a;  // 1/mass, 1/inertia (negative: expansion turns on later), global damping of translation, rotation
-    float4 b;  // collision damping, weight, penetration stiffness, static friction
-    float4 c;  // kinetic friction, CTE, nominal size hi, lo
+    float4 c;  // weight, CTE, nominal size hi, lo
+    const float4 *rb;  // collision damping, kinetic friction, penetration stiffness, static friction: read in contact only
+    __device__ __forceinline__ float4 b() const { return *rb; }
 };
 __device__ __forceinline__ LinkC link_consts_mx(const LMat &m, float dt) {
     // dampingMultiplier / dt, infinite for a Fixed end (its numerator over a zero time step)
     const float idt = __fdividef(1.0f, dt);
     LinkC c;
-    c.a = make_float4(m.b1, m.b2, m.b3, m.a2);
-    c.b = make_float4(m.sqA1, m.sqA2xIp, m.sqB1, m.sqB2xFMp);
-    c.c = make_float4(m.sqB3xIp, mul(m.dmcN, m.fixN ? CUDART_INF_F : idt), mul(m.dmcP, m.fixP ? CUDART_INF_F : idt),
+    c.ra = make_float4(m.b1, m.b2, m.b3, m.a2);
+    c.rb = make_float4(m.sqA1, m.sqA2xIp, m.sqB1, m.sqB2xFMp);
+    c.rc = make_float4(m.sqB3xIp, mul(m.dmcN, m.fixN ? CUDART_INF_F : idt), mul(m.dmcP, m.fixP ? CUDART_INF_F : idt),
                       m.lin ? m.area : -m.area);
-    c.e = m.nu == 0.0f ? make_float4(m.E, 1.0f, 0.0f, m.eps_fail)
+    c.re = m.nu == 0.0f ? make_float4(m.E, 1.0f, 0.0f, m.eps_fail)
                        : make_float4(m.eHat, minus(1.0f, m.nu), mul(m.nu, m.tss), m.eps_fail);
     return c;
 }
-__device__ __forceinline__ VoxC vox_consts_mx(const VMat &m) {
-    return VoxC{make_float4(m.mass_inv, m.toa_pos ? -m.mom_inv : m.mom_inv, m.c_glob, m.c_glob_rot),
-                make_float4(m.c_col, m.grav_force, m.pstiff, m.mu_s), make_float4(m.mu_k, m.cte, m.nom_hi, m.nom_lo)};
+__device__ __forceinline__ float4 vox_row_a(const VMat &m) {
+    return make_float4(m.mass_inv, m.toa_pos ? -m.mom_inv : m.mom_inv, m.c_glob, m.c_glob_rot);
 }
-// rows i of a table of n materials
-__device__ __forceinline__ LinkC link_rows(const float4 *t, int n, int i) { return LinkC{t[i], t[n + i], t[2 * n + i], t[3 * n + i]}; }
-__device__ __forceinline__ VoxC vox_rows(const float4 *t, int n, int i) { return VoxC{t[i], t[n + i], t[2 * n + i]}; }
+__device__ __forceinline__ float4 vox_row_b(const VMat &m) { return make_float4(m.c_col, m.mu_k, m.pstiff, m.mu_s); }
+__device__ __forceinline__ float4 vox_row_c(const VMat &m) { return make_float4(m.grav_force, m.cte, m.nom_hi, m.nom_lo); }
+// rows i of a table of n materials; a link's either held in registers from the start (LinkC) or read where
+// they are used (LinkRows)
+struct LinkRows {
+    const float4 *t;
+    int n;
+    __device__ __forceinline__ float4 a() const { return t[0]; }
+    __device__ __forceinline__ float4 b() const { return t[n]; }
+    __device__ __forceinline__ float4 c() const { return t[2 * n]; }
+    __device__ __forceinline__ float4 e() const { return t[3 * n]; }
+};
+template <bool HELD> __device__ __forceinline__ auto link_rows(const float4 *t, int n, int i) {
+    const LinkRows r{t + i, n};
+    if constexpr (HELD) return LinkC{r.a(), r.b(), r.c(), r.e()};
+    else return r;
+}
+__device__ __forceinline__ VoxC vox_rows(const float4 *t, int n, int i) { return VoxC{t[i], t[2 * n + i], t + n + i}; }
 
 // ------------------------------------------------------------- link
 struct Ends {  // a voxel's position and orientation pairs, hi and lo; pos.w the base size
@@ -188,18 +207,15 @@ struct LinkState {
     float2 strain;  // {strain, maxStrain}
     uint32_t fl;
 };
-struct LinkForces {  // in the lattice frame
-    V fN, mN, fP, mP;
-};
-
-// one link's update from its ends; l is read for non-linear materials only (their curve and the
-// plastic offset).  *diverged: axial strain above 100 (VX3_VoxelyzeKernel.cu:271-281).  AXIS: the
-// link's axis where a warp's links share one (no selects), -1 to read it from the flags
-template <int AXIS = -1>
-__device__ __forceinline__ void link_step(const Dev &d, const LinkC &m, int l, const Ends &en, const Ends &ep,
-                                          LinkState &s, LinkForces &f, bool &diverged) {
+// One link's update from its ends; l is read for non-linear materials only (their curve and the plastic
+// offset).  What it leaves is handed to `out` as soon as it is known, so that it does not sit in registers
+// until the end: the local state, the strain (torn: above 100, VX3_VoxelyzeKernel.cu:271-281), the flags,
+// and force and moment of the negative and the positive end in the lattice frame.
+template <class Rows, class Out>
+__device__ __forceinline__ void link_step(const Dev &d, const Rows &m, int l, const Ends &en, const Ends &ep,
+                                          const LinkState &s, Out &out) {
     const uint32_t fl = s.fl;
-    const int axis = AXIS >= 0 ? AXIS : (int)(fl & LF_AXIS);
+    const int axis = (int)(fl & LF_AXIS);
     // rest length L = 0.5*(bsNeg + bsPos) as a hi/lo pair (VX3_Link::updateRestLength)
     float Lh, Ll;
     two_sum(en.pH.w, ep.pH.w, Lh, Ll);
@@ -250,61 +266,61 @@ __device__ __forceinline__ void link_step(const Dev &d, const LinkC &m, int l, c
     }
     const V a2v = rotvec(angle2.w, V{angle2.x, angle2.y, angle2.z});
     const V dP = scale(diff(pos2, s.pos2), 0.5f), d1 = scale(diff(a1v, s.a1v), 0.5f), d2 = scale(diff(a2v, s.a2v), 0.5f);
-    s.pos2 = pos2;
-    s.a1v = a1v;
-    s.a2v = a2v;
+    out.local(pos2, a1v, a2v, small);
     // FP32 quotients in the hot paths use the hardware reciprocal (__fdividef: within 2 ulp)
     const float axialStrain = __fdividef(pos2.x, L);
-    s.strain.x = axialStrain;
+    float2 strain = make_float2(axialStrain, s.strain.y);
     float stress;  // updateStrain (VX3_Link.cu:220-260)
-    if (m.c.w > 0.0f) {
-        if (axialStrain > s.strain.y) s.strain.y = axialStrain;
-        stress = m.e.w != -1.0f && axialStrain > m.e.w ? 0.0f : mul(m.e.x, fmaf(m.e.y, axialStrain, m.e.z));
+    const float4 mc = m.c(), me = m.e();
+    if (mc.w > 0.0f) {
+        if (axialStrain > strain.y) strain.y = axialStrain;
+        stress = me.w != -1.0f && axialStrain > me.w ? 0.0f : mul(me.x, fmaf(me.y, axialStrain, me.z));
     } else {
-        stress = link_stress(d, d.lmat[fl >> 8], l, axialStrain, &s.strain.y);
+        stress = link_stress(d, d.lmat[fl >> 8], l, axialStrain, &strain.y);
     }
-    diverged = axialStrain > 100;
+    out.strain(strain, axialStrain > 100);
     const uint32_t nfl = (fl & ~(LF_SMALL | LF_LVV)) | (small ? LF_SMALL : 0u);
-    if (m.e.w != -1.0f && s.strain.y > m.e.w) {  // isFailed: forces zero
+    if (me.w != -1.0f && strain.y > me.w) {  // isFailed: forces zero
         const V z{0, 0, 0};
-        f = LinkForces{z, z, z, z};
-        s.fl = nfl | (lvv ? LF_LVV : 0u);
+        out.neg(z, z);
+        out.pos(z, z);
+        out.flags(nfl | (lvv ? LF_LVV : 0u), true);
         return;
     }
-    s.fl = nfl | LF_LVV;
-    const float b1 = m.a.x, b2 = m.a.y, b3 = m.a.z, a2 = m.a.w;
-    f.fN = V{mul(stress, fabsf(m.c.w)), dot_a(b1, pos2.y, -b2, plus(a1v.z, a2v.z)), dot_a(b1, pos2.z, b2, plus(a1v.y, a2v.y))};
-    f.fP = neg(f.fN);
-    f.mN = V{mul(a2, minus(a2v.x, a1v.x)), dot_b(-b2, pos2.z, -b3, fmaf(2.0f, a1v.y, a2v.y)),
+    const float4 ma = m.a();
+    const float b1 = ma.x, b2 = ma.y, b3 = ma.z, a2 = ma.w;
+    V fN = V{mul(stress, fabsf(mc.w)), dot_a(b1, pos2.y, -b2, plus(a1v.z, a2v.z)), dot_a(b1, pos2.z, b2, plus(a1v.y, a2v.y))};
+    V fP = neg(fN);
+    V mN = V{mul(a2, minus(a2v.x, a1v.x)), dot_b(-b2, pos2.z, -b3, fmaf(2.0f, a1v.y, a2v.y)),
              dot_b(b2, pos2.y, -b3, fmaf(2.0f, a1v.z, a2v.z))};
-    f.mP = V{mul(a2, minus(a1v.x, a2v.x)), dot_b(-b2, pos2.z, -b3, fmaf(2.0f, a2v.y, a1v.y)),
+    V mP = V{mul(a2, minus(a1v.x, a2v.x)), dot_b(-b2, pos2.z, -b3, fmaf(2.0f, a2v.y, a1v.y)),
              dot_b(b2, pos2.y, -b3, fmaf(2.0f, a2v.z, a1v.z))};
     if (lvv) {
-        const float sB1 = m.b.z, sB2 = m.b.w, sB3 = m.c.x, dmN = m.c.y, dmP = m.c.z;
-        const V pc{mul(m.b.x, dP.x), dot_a(sB1, dP.y, -sB2, plus(d1.z, d2.z)), dot_b(sB1, dP.z, sB2, plus(d1.y, d2.y))};
-        const float tw = mul(m.b.y, minus(d2.x, d1.x));
-        f.fN = fma3(dmN, pc, f.fN);
-        f.fP = fma3(-dmP, pc, f.fP);
-        f.mN = fma3(mul(-0.5f, dmN), V{-tw, dot_a(sB2, dP.z, sB3, fmaf(2.0f, d1.y, d2.y)), dot_b(-sB2, dP.y, sB3, fmaf(2.0f, d1.z, d2.z))}, f.mN);
-        f.mP = fma3(mul(-0.5f, dmP), V{tw, dot_a(sB2, dP.z, sB3, fmaf(2.0f, d2.y, d1.y)), dot_b(-sB2, dP.y, sB3, fmaf(2.0f, d2.z, d1.z))}, f.mP);
+        const float4 mb = m.b();
+        const float sB1 = mb.z, sB2 = mb.w, sB3 = mc.x, dmN = mc.y, dmP = mc.z;
+        const V pc{mul(mb.x, dP.x), dot_a(sB1, dP.y, -sB2, plus(d1.z, d2.z)), dot_b(sB1, dP.z, sB2, plus(d1.y, d2.y))};
+        const float tw = mul(mb.y, minus(d2.x, d1.x));
+        fN = fma3(dmN, pc, fN);
+        fP = fma3(-dmP, pc, fP);
+        mN = fma3(mul(-0.5f, dmN), V{-tw, dot_a(sB2, dP.z, sB3, fmaf(2.0f, d1.y, d2.y)), dot_b(-sB2, dP.y, sB3, fmaf(2.0f, d1.z, d2.z))}, mN);
+        mP = fma3(mul(-0.5f, dmP), V{tw, dot_a(sB2, dP.z, sB3, fmaf(2.0f, d2.y, d1.y)), dot_b(-sB2, dP.y, sB3, fmaf(2.0f, d2.z, d1.z))}, mP);
     }
     if (!small) {
-        f.fN = rotate_inv_x0(angle1, f.fN);
-        f.mN = rotate_inv_x0(angle1, f.mN);
+        fN = rotate_inv_x0(angle1, fN);
+        mN = rotate_inv_x0(angle1, mN);
     }
-    f.fP = rotate_inv(angle2, f.fP);
-    f.mP = rotate_inv(angle2, f.mP);
-    f.fN = to_axis_original(axis, f.fN);
-    f.mN = to_axis_original(axis, f.mN);
-    f.fP = to_axis_original(axis, f.fP);
-    f.mP = to_axis_original(axis, f.mP);
+    out.neg(to_axis_original(axis, fN), to_axis_original(axis, mN));
+    fP = rotate_inv(angle2, fP);
+    mP = rotate_inv(angle2, mP);
+    out.pos(to_axis_original(axis, fP), to_axis_original(axis, mP));
+    out.flags(nfl | LF_LVV, false);
 }
 
 // base size nomSize*(1 + T*cte) as a hi/lo pair
-__device__ __forceinline__ void base_size(const VoxC &m, float te, float &hi, float &lo) {
-    const float f = fmaf(te, m.c.y, 1.0f);
-    const float p = mul(m.c.z, f);
-    quick_two_sum(p, fmaf(m.c.w, f, fmaf(m.c.z, f, -p)), hi, lo);
+__device__ __forceinline__ void base_size(float4 mc, float te, float &hi, float &lo) {  // row c of the material
+    const float f = fmaf(te, mc.y, 1.0f);
+    const float p = mul(mc.z, f);
+    quick_two_sum(p, fmaf(mc.w, f, fmaf(mc.z, f, -p)), hi, lo);
 }
 
 // temperature at the end of a step (gpu_update_temperature, VX3_VoxelyzeKernel.cu:625-650)
@@ -348,16 +364,17 @@ __device__ __forceinline__ void move(VoxelState &s, const VoxC &m, V F, V vel, b
     V fric = F;
     if (floorOn) {
         if (pen >= 0) {
-            const float normal = mul(m.b.z, pen);
-            F.z = plus(F.z, fmaf(-m.b.x, vel.z, normal));
+            const float4 mb = m.b();
+            const float normal = mul(mb.z, pen);
+            F.z = plus(F.z, fmaf(-mb.x, vel.z, normal));
             if (stat) {
-                const float lim = mul(m.b.w, normal);
+                const float lim = mul(mb.w, normal);
                 if (dot_a(F.x, F.x, F.y, F.y) > mul(lim, lim)) stat = false;
             } else {
                 // the horizontal velocity's direction (normalized(): unchanged when zero)
                 const float h2 = dot_a(vel.x, vel.x, vel.y, vel.y);
                 const float k = h2 > 0.0f ? rsqrtf(h2) : 1.0f;
-                const float mk = mul(m.c.x, normal);
+                const float mk = mul(mb.y, normal);
                 F.x = fmaf(-mk, mul(vel.x, k), F.x);
                 F.y = fmaf(-mk, mul(vel.y, k), F.y);
             }
