@@ -325,9 +325,22 @@ int vx3g_recommended_dt_noalloc(vx3g_ctx *ctx, double *rdt);
  *   from / appended to a flat JSON object keyed by GPU name and batch size; a
  *   cached choice is applied without timing.  FP64 contexts just step.
  * vx3g_launch_shapes: the shapes in use: {link threads, link min blocks, voxel
- *   threads, voxel min blocks}. */
+ *   threads, voxel min blocks}.
+ * vx3g_step_plan: how vx3g_step advances the context, decided when it was created.
+ *   plan12[0]: 0 if every step runs the link and voxel passes (and the contact
+ *   kernels); else the fewest steps of a call for which one kernel takes many steps
+ *   at once, robots held in the shared memory of clusters of thread blocks (the
+ *   results are the same bits).  [1]: the most steps of one such launch.  [2]: its
+ *   launches side by side, one per cluster size in use.  [3]: 1 if the contact side
+ *   stream forks before the contact-list rebuild, 0 if after.  [4] to [11]: clusters
+ *   of 1 to 8 thread blocks.  ([1], [2], [4] to [11] are 0 where [0] is.)
+ * vx3g_choose_steps: from now on vx3g_step goes the way decided at creation (0), by
+ *   the passes (1) or by the many-step kernel (2; VX3G_ERR_UNSUPPORTED where the batch
+ *   does not allow it), for comparing the two. */
 int vx3g_autotune(vx3g_ctx *ctx, int n_steps, const char *cache_json);
 int vx3g_launch_shapes(vx3g_ctx *ctx, int32_t *shapes4);
+int vx3g_step_plan(vx3g_ctx *ctx, int32_t *plan12);
+int vx3g_choose_steps(vx3g_ctx *ctx, int way);
 
 /* ---- measurement helpers (no counterpart in the reference) ---------------
  * vx3g_time_steps: runs vx3g_step(ctx, n_steps) between two CUDA events on the

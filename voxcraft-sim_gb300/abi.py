@@ -25,7 +25,7 @@ EXPORTS = [
     "vx3g_counts", "vx3g_offsets", "vx3g_get_state", "vx3g_set_state", "vx3g_get_voxel_aux", "vx3g_get_links",
     "vx3g_get_topology", "vx3g_get_surface", "vx3g_com", "vx3g_dt", "vx3g_time", "vx3g_status",
     "vx3g_steps_taken", "vx3g_time_steps", "vx3g_flush_l2", "vx3g_time_passes", "vx3g_stop_robot",
-    "vx3g_record", "vx3g_backward", "vx3g_recommended_dt_noalloc", "vx3g_autotune", "vx3g_launch_shapes",
+    "vx3g_record", "vx3g_backward", "vx3g_recommended_dt_noalloc", "vx3g_autotune", "vx3g_launch_shapes", "vx3g_step_plan", "vx3g_choose_steps",
     "vx3g_debug_barrier", "vx3g_prepare_graphs", "vx3g_get_signals",
 ]
 
@@ -124,6 +124,8 @@ def load(path: str = LIB_PATH):
     lib.vx3g_recommended_dt_noalloc.argtypes = [vp, dp]
     lib.vx3g_autotune.argtypes = [vp, ip, ctypes.c_char_p]
     lib.vx3g_launch_shapes.argtypes = [vp, vp]
+    lib.vx3g_step_plan.argtypes = [vp, vp]
+    lib.vx3g_choose_steps.argtypes = [vp, ip]
     lib.vx3g_backward.argtypes = [vp, dp, dp, dp]
     lib.vx3g_debug_barrier.argtypes = [vp, ctypes.c_uint32, ctypes.c_uint32]
     lib.vx3g_prepare_graphs.argtypes = [vp]
@@ -371,6 +373,20 @@ class Batch:
         out = np.zeros(4, np.int32)
         _check(self.lib.vx3g_launch_shapes(self.h, _P(out)), "vx3g_launch_shapes")
         return out
+
+    def step_plan(self):
+        """How step() advances the batch (vx3g_step_plan): `many_from`, the fewest steps of a call that one
+        kernel takes at once (0: the passes always), `most`, the most steps of one such launch, `launches`
+        side by side, `fork` of the contact side stream, and `clusters`, {thread blocks: clusters}."""
+        p = np.zeros(12, np.int32)
+        _check(self.lib.vx3g_step_plan(self.h, _P(p)), "vx3g_step_plan")
+        return dict(many_from=int(p[0]), most=int(p[1]), launches=int(p[2]), fork=int(p[3]),
+                    clusters={k + 1: int(n) for k, n in enumerate(p[4:]) if n})
+
+    def choose_steps(self, way: str):
+        """step() goes the way decided at creation ("rule"), by the passes ("passes") or by the many-step
+        kernel ("many"; an error where the batch does not allow it)."""
+        _check(self.lib.vx3g_choose_steps(self.h, ("rule", "passes", "many").index(way)), "vx3g_choose_steps")
 
     def recommended_dt_noalloc(self):
         out = np.zeros(self.n_robots)

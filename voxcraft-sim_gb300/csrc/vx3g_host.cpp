@@ -266,7 +266,10 @@ struct vx3g_ctx {
     void *flush = nullptr;
     size_t flush_bytes = 0;
     double *stage = nullptr;  // 4 doubles per voxel: host state exchange
-    std::vector<ResClass> res;  // launches of k_steps_mixed that together step the batch (empty: the passes)
+    std::vector<ResClass> res;  // launches of k_steps_mixed that together step the batch (empty: no plan made)
+    bool res_on = false;        // vx3g_step takes them, not the passes
+    bool res_chosen = false;    // ... as decided at creation
+    std::vector<int> lmoff, vmoff;  // each robot's first link and voxel material
     std::vector<cudaStream_t> res_stream;
     cudaEvent_t res_fork = nullptr;
     std::vector<cudaEvent_t> res_join;
@@ -404,9 +407,12 @@ double passes_us(double nv, double nl) {  // launches, then the L2's rate, then 
 // below 96 the cluster barriers cost more than the shorter phases save: 104 voxels 3.0 us in one
 // CTA, 3.4 in two).  Small robots are bundled up to the same measure.
 // The plan is kept where its estimated step is shorter than the passes' (resident_us, passes_us).
-// lmoff, vmoff: the first link and voxel material of each robot
-int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<int> &vmoff) {
+// any: the plan is kept whatever the estimate says
+int plan_resident(vx3g_ctx *c, bool any) {
     const Dev &d = c->d;
+    // (c->ends holds the lattice's links alone here: no attachment)
+    if (!d.mixed || d.ns || d.any_dyn || c->any_ff || c->any_cilia || c->any_bcs || c->any_signals) return VX3G_OK;
+    const std::vector<int> &lmoff = c->lmoff, &vmoff = c->vmoff;
     constexpr int kMost = 8;                 // CTAs of a cluster (portable size)
     constexpr size_t kHalf = 115000;         // shared memory with which two CTAs share an SM
     constexpr int kHalfThreads = kResThreads / 2;
@@ -478,7 +484,7 @@ int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<
         for (const ResBundle &b : p.b) lc += b.lc;
         load.push_back(ResLoad{(double)p.b.size() / act, lc / p.b.size(), p.smem > kHalf});
     }
-    if (load.empty() || resident_us(load) > 0.92 * passes_us(d.nv, d.nl)) return VX3G_OK;
+    if (load.empty() || (!any && resident_us(load) > 0.92 * passes_us(d.nv, d.nl))) return VX3G_OK;
     for (int K = kMost; K >= 1; K--) {
         Plan &p = by[K - 1];
         if (p.b.empty()) continue;
@@ -519,6 +525,7 @@ int plan_resident(vx3g_ctx *c, const std::vector<int> &lmoff, const std::vector<
             c->res_join.push_back(e);
         }
     }
+    c->res_on = true;
     return VX3G_OK;
 }
 
@@ -553,7 +560,8 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     std::vector<VMat> vmats;
     std::vector<LMat> lmats;
     std::vector<int> lrob;  // the robot of each link material
-    std::vector<int> lmoff(c->nr + 1, 0), vmoff(c->nr + 1, 0);  // each robot's first link and voxel material
+    c->lmoff.assign(c->nr + 1, 0);
+    c->vmoff.assign(c->nr + 1, 0);
     bool any_actuated = false;
     std::vector<RobotP> rps(c->nr);
     std::vector<double4> pos, quat;
@@ -911,8 +919,8 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
             }
         }
         lrob.resize(lmats.size(), r);
-        lmoff[r + 1] = (int)lmats.size();
-        vmoff[r + 1] = (int)vmats.size();
+        c->lmoff[r + 1] = (int)lmats.size();
+        c->vmoff[r + 1] = (int)vmats.size();
         // lists in shared memory when the robot fits (lattice coordinates below 512, packed in 10 bits each)
         int cmax = 0;
         for (int k = 0; k < nvr; k++) {
@@ -1136,9 +1144,8 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         // body rarely does (a folded 64^3 body 54.4 us a step against 55.8 so)
         c->fork_early = d.nhash == 0 ? 1 : 0;
     }
-    // (c->ends holds the lattice's links alone here: no attachment)
-    if (d.mixed && !d.ns && !d.any_dyn && !c->any_ff && !c->any_cilia && !c->any_bcs && !c->any_signals && (rc = plan_resident(c, lmoff, vmoff)))
-        return rc;
+    if ((rc = plan_resident(c, false))) return rc;
+    c->res_chosen = c->res_on;
     launch_init_temperature(d, c->precision == VX3G_PRECISION_MIXED, c->stream);
     launch_dt(d, c->scratch, c->stream);
     if (d.mixed) launch_rows_mixed(d, lrow, vrow, lrob_d, c->stream);
@@ -1251,7 +1258,7 @@ void vx3g_destroy(vx3g_ctx *c) { delete c; }
 int vx3g_step(vx3g_ctx *c, int n) {
     if (!c || n < 0) return fail(VX3G_ERR_INVALID, "bad arguments to vx3g_step");
     CU(cudaSetDevice(c->device));
-    while (n > 0 && !c->res.empty()) {
+    while (n > 0 && c->res_on) {
         const int k = std::min(n, kResSteps);
         if (int rc = step_resident(c, k)) return rc;
         n -= k;
@@ -1277,7 +1284,7 @@ int vx3g_step(vx3g_ctx *c, int n) {
 
 int vx3g_prepare_graphs(vx3g_ctx *c) {
     if (!c) return fail(VX3G_ERR_INVALID, "null context");
-    if (c->chunk == INT32_MAX || !c->res.empty()) return VX3G_OK;  // graphs off, or not used (k_steps_mixed)
+    if (c->chunk == INT32_MAX || c->res_on) return VX3G_OK;  // graphs off, or not used (k_steps_mixed)
     CU(cudaSetDevice(c->device));
     cudaGraphExec_t g;
     for (int parity = 0; parity < 2; parity++)
@@ -1863,6 +1870,29 @@ int vx3g_launch_shapes(vx3g_ctx *c, int32_t *shapes4) {
     shapes4[1] = mx ? kLinkShapes[c->shape_links].min_blocks : 1;
     shapes4[2] = mx ? kVoxelShapes[c->shape_voxels].threads : 256;
     shapes4[3] = mx ? kVoxelShapes[c->shape_voxels].min_blocks : 1;
+    return VX3G_OK;
+}
+
+int vx3g_step_plan(vx3g_ctx *c, int32_t *plan12) {
+    if (!c || !plan12) return fail(VX3G_ERR_INVALID, "bad arguments to vx3g_step_plan");
+    std::fill(plan12, plan12 + 12, 0);
+    plan12[3] = c->fork_early;
+    if (!c->res_on) return VX3G_OK;
+    plan12[0] = 1;
+    plan12[1] = kResSteps;
+    plan12[2] = (int32_t)c->res.size();
+    for (const ResClass &r : c->res) plan12[3 + r.K] = r.count;
+    return VX3G_OK;
+}
+
+int vx3g_choose_steps(vx3g_ctx *c, int way) {
+    if (!c || way < 0 || way > 2) return fail(VX3G_ERR_INVALID, "bad arguments to vx3g_choose_steps");
+    CU(cudaSetDevice(c->device));
+    if (way == 2 && c->res.empty()) {
+        if (int rc = plan_resident(c, true)) return rc;
+        if (c->res.empty()) return fail(VX3G_ERR_UNSUPPORTED, "the many-step kernel does not handle this batch");
+    }
+    c->res_on = way == 0 ? c->res_chosen : way == 2;
     return VX3G_OK;
 }
 
