@@ -29,10 +29,10 @@ SIZES = [((1, 1, 1), 1), ((2, 1, 1), 1), ((31, 1, 1), 1), ((4, 8, 3), 1), ((8, 4
 def test_one_robot(dims, size):
     b = abi.Batch([resident._body(np.random.default_rng(1), dims, fill=1.0)], abi.PRECISION_MIXED)
     if b.nv <= 1000:
-        assert b.step_plan()["many_from"] > 0  # the rule takes it
+        assert 1 <= b.step_plan()["many_from"] < 12  # the rule takes it, for more than a few steps
     b.choose_steps("many")
     p = b.step_plan()
-    assert p["many_from"] > 0 and p["most"] >= 100 and p["launches"] == 1 and p["clusters"] == {size: 1}
+    assert p["many_from"] == 1 and p["most"] >= 100 and p["launches"] == 1 and p["clusters"] == {size: 1}
     b.choose_steps("passes")
     assert b.step_plan()["many_from"] == 0
     b.close()
@@ -44,8 +44,10 @@ CLUSTERS = [{1: 1}, {1: 5}, {1: 300}, {2: 3}, {8: 2}]
 @pytest.mark.parametrize("form", range(len(divergence.FORMS)))
 def test_forms_of_the_divergence_test(form):
     count, dims = divergence.FORMS[form]
-    p = _plan([divergence._robot(i, dims) for i in range(count)])
-    assert p["many_from"] > 0 and p["clusters"] == CLUSTERS[form]
+    b = abi.Batch([divergence._robot(i, dims) for i in range(count)], abi.PRECISION_MIXED)
+    b.choose_steps("many")
+    assert b.step_plan()["clusters"] == CLUSTERS[form]
+    b.close()
 
 
 def _mixed_batch(count, lo, hi):
@@ -76,6 +78,34 @@ def test_both_ways_leave_the_same(count, lo, hi):
     for other in got[1:]:
         for k in got[0]:
             assert np.array_equal(got[0][k], other[k], equal_nan=True), k
+
+
+def test_calls_of_few_and_of_many_steps():
+    """A call goes by the passes up to the plan's number of steps, and in launches of equal length above the
+    most of one; graphs are captured where a chunk of theirs can still come to run."""
+    rng = np.random.default_rng(6)
+    robots = [resident._body(rng, (7, 6, 5)) for _ in range(5)]
+    got = []
+    for chunk in (100, 2, -1):
+        b = abi.Batch(robots, abi.PRECISION_MIXED, graph_chunk=chunk)
+        b.prepare_graphs()
+        k = b.step_plan()["many_from"]
+        assert k > 2
+        for n in (1, k - 1, k, k + 1, 256, 257, 513, 2):
+            b.step(n)
+        got.append(resident._all(b))
+        b.choose_steps("passes")
+        b.prepare_graphs()
+        b.step(5)
+        b.close()
+    b = abi.Batch(robots, abi.PRECISION_MIXED)
+    b.choose_steps("passes")
+    b.step(3 * k + 1029)
+    want = resident._all(b)
+    b.close()
+    for g in got:
+        for name in want:
+            assert np.array_equal(g[name], want[name], equal_nan=True), name
 
 
 def test_batches_that_keep_the_passes():

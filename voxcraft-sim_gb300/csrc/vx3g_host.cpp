@@ -269,6 +269,8 @@ struct vx3g_ctx {
     std::vector<ResClass> res;  // launches of k_steps_mixed that together step the batch (empty: no plan made)
     bool res_on = false;        // vx3g_step takes them, not the passes
     bool res_chosen = false;    // ... as decided at creation
+    int res_from = 1;           // ... in calls of this many steps and more
+    bool res_always = false;    // ... or of any number (vx3g_choose_steps)
     std::vector<int> lmoff, vmoff;  // each robot's first link and voxel material
     std::vector<cudaStream_t> res_stream;
     cudaEvent_t res_fork = nullptr;
@@ -368,33 +370,60 @@ int check_math_program(const vx3g_math_token *t, int *len, bool *reads_pos, std:
     return VX3G_ERR_INVALID;
 }
 
-// Microseconds of a step by k_steps_mixed and by the two passes.  Fitted to 226 batches of 1 to 800
-// robots of 6^3 to 18^3 cells, filled or to 70%, one size or mixed, each timed both ways: the resident
-// kernel is 0.70 to 3 times as fast as the passes (geometric mean 1.31), slowest where a few more
-// clusters than run at once make a second wave of large CTAs (64 robots of 13^3: 29.3 us against
-// 20.6; one of 16^3, held by 8 of 152 SMs, 7.3 against 6.3).  Chosen by these, with 8% to spare, it is
-// taken in no batch where it was more than 0.4% slower, and the mean is 1.32 (1.33 with the better one
-// each time).  A CTA's step grows with its links; two CTAs share an SM's issue slots (half the slope
-// while they do not); one cluster size goes in whole waves, several sizes fill each other's gaps.
+// Microseconds of a step by k_steps_mixed and by the two passes, both measured for 620 batches of 1 to 1600
+// robots of 2^3 to 18^3 cells, filled or to 60%, one size or mixed (half of them drawn after the fit).  A
+// batch of one cluster size is estimated within 8% in nine of ten cases, one of several sizes within 20%, the
+// passes within 10%, hence the margins of 5% and 20% in plan_resident: the kernel is taken in 405 of the
+// batches, for a geometric mean of 1.32 times the passes' speed (1.34 with the better one each time), and is
+// slower than the passes by more than 2% in three (3, 6 and 11%).  It is fast where a step of the passes
+// is latency (a robot of 100 voxels 2.4 us against 5.4) and where the state is beyond the L2 (800,000 voxels of
+// 8^3 robots 81 us against 142); in between, and for robots of a whole SM per thread block, the passes are
+// (40 robots of 13^3: 21 us against 16).
 struct ResLoad {
-    double waves, links;  // bundles by those that run at once; links of a CTA
+    int K;                // CTAs of a cluster
+    double waves;         // bundles by those that run at once
+    double links, most;   // links of a CTA, on average and at most
     bool whole;           // a CTA has an SM for itself
 };
-double resident_us(const std::vector<ResLoad> &load) {
-    double x = 0, sum = 0, most = 0;
-    for (const ResLoad &l : load) x += l.waves;
-    for (const ResLoad &l : load) {
-        const double t = 3.8 + (l.whole ? 0.0028 : x <= 0.5 ? 0.0025 : 0.0045) * l.links;
-        sum += l.waves * t;
-        most = std::max(most, t);
-    }
-    const double mean = sum / x;
-    if (load.size() == 1) return mean * (x < 6 ? std::ceil(x - 1e-9) : x + 0.5);
-    return x > 0.9 ? std::max(most, mean * (0.75 * x + 1.1)) : most;
+// one wave: a CTA's step grows with its links, more slowly while it has an SM to itself (`alone`) than when
+// two share one's issue slots, and by a jump where its threads take the links in two rounds
+double wave_us(int K, double links, bool whole, bool alone) {
+    if (K == 1) return 2.05 + (alone || whole ? 0.0038 : 0.0078) * links;
+    if (whole) return (links <= kResThreads ? 3.8 : 5.0) + 0.0025 * links;
+    if (links <= kResThreads / 2) return alone ? 3.05 + 0.0025 * links : 3.4 + 0.0042 * links;
+    return alone ? 5.4 + 0.0006 * links : 5.0 + 0.005 * links;
 }
-double passes_us(double nv, double nl) {  // launches, then the L2's rate, then that of HBM
-    const double u = nv + nl / 15;
-    return 6.1 + 8.1e-5 * std::min(u, 1.75e5) + 1.73e-4 * std::max(u - 1.75e5, 0.0);
+double resident_us(const std::vector<ResLoad> &load) {
+    constexpr double kAlone = 0.43;  // waves up to which every CTA finds an SM for itself
+    if (load.size() == 1) {
+        const ResLoad &l = load[0];
+        if (l.waves <= 1.0) return wave_us(l.K, l.most, l.whole, l.waves <= kAlone);
+        const double full = std::floor(l.waves + 1e-9), rest = l.waves - full;
+        return full * wave_us(l.K, l.links, l.whole, false) +
+               (rest < 1e-3 ? 0.0 : wave_us(l.K, l.links, l.whole, !l.whole && rest <= kAlone));
+    }
+    // several sizes fill each other's gaps
+    double waves = 0, sum = 0, alone = 0, shared = 0;
+    for (const ResLoad &l : load) {
+        waves += l.waves;
+        sum += l.waves * wave_us(l.K, l.links, l.whole, false);
+        alone = std::max(alone, wave_us(l.K, l.most, l.whole, true));
+        shared = std::max(shared, wave_us(l.K, l.most, l.whole, false));
+    }
+    return waves <= kAlone ? alone : std::max(shared, 0.95 * sum + 0.6 * shared);
+}
+double passes_us(double nv, double nl, double nr) {  // latency, then the L2's rate, then that of HBM
+    const double u = nv + nl / 6;
+    return 4.9 + 0.18 * std::min(std::log2(nr), 6.0) + 4.5e-5 * std::min(u, 2.5e4) + 8.2e-5 * std::min(std::max(u - 2.5e4, 0.0), 2.1e5) +
+           1.44e-4 * std::max(u - 2.35e5, 0.0);
+}
+// The fewest steps of a call for which one launch is faster: it loads and stores the state (one robot of 8
+// voxels: 11.1 us for one step, 55 for 20, against 9.4 and 116 by the passes; 203 robots of 12^3 cells 127 us
+// for one step against 64, of 43 and 68 a step).  Passes launched one by one start every 5.6 us at best.
+// Over those batches and calls of 1 to 20 steps the way taken is 1% slower than the better one on average.
+int resident_from(double many, double passes, double nv, bool several) {
+    const double once = 5.7 + 1.344 * many + 2.977e-5 * nv + (several ? 4.9 : 0.0) - 6.0;
+    return std::max(1, (int)std::ceil(once / std::max(std::max(passes, 5.6) - many, 0.05)));
 }
 
 // Whether and how k_steps_mixed steps the batch: mixed precision, whole robots in shared memory.
@@ -406,7 +435,8 @@ double passes_us(double nv, double nl) {  // launches, then the L2's rate, then 
 // leaves SMs idle: down to 96 voxels per CTA (864 voxels: 3.8 us a step in eight CTAs, 5.4 in four;
 // below 96 the cluster barriers cost more than the shorter phases save: 104 voxels 3.0 us in one
 // CTA, 3.4 in two).  Small robots are bundled up to the same measure.
-// The plan is kept where its estimated step is shorter than the passes' (resident_us, passes_us).
+// The plan is kept where its estimated step is shorter than the passes', and calls of few steps go by
+// the passes all the same.
 // any: the plan is kept whatever the estimate says
 int plan_resident(vx3g_ctx *c, bool any) {
     const Dev &d = c->d;
@@ -480,11 +510,15 @@ int plan_resident(vx3g_ctx *c, bool any) {
         int act = 0;
         CU(steps_mixed_active(K, threads(p), p.smem, &act));
         if (act < 1) return VX3G_OK;
-        double lc = 0;
-        for (const ResBundle &b : p.b) lc += b.lc;
-        load.push_back(ResLoad{(double)p.b.size() / act, lc / p.b.size(), p.smem > kHalf});
+        double lc = 0, most = 0;
+        for (const ResBundle &b : p.b) lc += b.lc, most = std::max<double>(most, b.lc);
+        load.push_back(ResLoad{K, (double)p.b.size() / act, lc / p.b.size(), most, p.smem > kHalf});
     }
-    if (load.empty() || (!any && resident_us(load) > 0.92 * passes_us(d.nv, d.nl))) return VX3G_OK;
+    if (load.empty()) return VX3G_OK;
+    const bool several = load.size() > 1;
+    const double many = resident_us(load), passes = passes_us(d.nv, d.nl, c->nr);
+    if (!any && many > (several ? 0.8 : 0.95) * passes) return VX3G_OK;
+    c->res_from = resident_from(many, passes, d.nv, several);
     for (int K = kMost; K >= 1; K--) {
         Plan &p = by[K - 1];
         if (p.b.empty()) continue;
@@ -1258,11 +1292,12 @@ void vx3g_destroy(vx3g_ctx *c) { delete c; }
 int vx3g_step(vx3g_ctx *c, int n) {
     if (!c || n < 0) return fail(VX3G_ERR_INVALID, "bad arguments to vx3g_step");
     CU(cudaSetDevice(c->device));
-    while (n > 0 && c->res_on) {
-        const int k = std::min(n, kResSteps);
-        if (int rc = step_resident(c, k)) return rc;
-        n -= k;
-    }
+    if (c->res_on && (n >= c->res_from || c->res_always))
+        for (int left = (n + kResSteps - 1) / kResSteps; left > 0; left--) {  // launches of equal length
+            const int k = (n + left - 1) / left;
+            if (int rc = step_resident(c, k)) return rc;
+            n -= k;
+        }
     for (bool first = true; n > 0; first = false) {
         const int parity = (int)(c->steps & 1);
         if (n >= c->chunk) {
@@ -1284,7 +1319,8 @@ int vx3g_step(vx3g_ctx *c, int n) {
 
 int vx3g_prepare_graphs(vx3g_ctx *c) {
     if (!c) return fail(VX3G_ERR_INVALID, "null context");
-    if (c->chunk == INT32_MAX || c->res_on) return VX3G_OK;  // graphs off, or not used (k_steps_mixed)
+    // graphs off, or not used: k_steps_mixed takes calls of this many steps
+    if (c->chunk == INT32_MAX || (c->res_on && (c->res_always || c->chunk >= c->res_from))) return VX3G_OK;
     CU(cudaSetDevice(c->device));
     cudaGraphExec_t g;
     for (int parity = 0; parity < 2; parity++)
@@ -1878,7 +1914,7 @@ int vx3g_step_plan(vx3g_ctx *c, int32_t *plan12) {
     std::fill(plan12, plan12 + 12, 0);
     plan12[3] = c->fork_early;
     if (!c->res_on) return VX3G_OK;
-    plan12[0] = 1;
+    plan12[0] = c->res_always ? 1 : c->res_from;
     plan12[1] = kResSteps;
     plan12[2] = (int32_t)c->res.size();
     for (const ResClass &r : c->res) plan12[3 + r.K] = r.count;
@@ -1893,6 +1929,7 @@ int vx3g_choose_steps(vx3g_ctx *c, int way) {
         if (c->res.empty()) return fail(VX3G_ERR_UNSUPPORTED, "the many-step kernel does not handle this batch");
     }
     c->res_on = way == 0 ? c->res_chosen : way == 2;
+    c->res_always = way == 2;
     return VX3G_OK;
 }
 
