@@ -30,11 +30,11 @@ __global__ void k_actuation(Dev d, int parity) {
     actuation_phase(d, r, parity, d.T[(size_t)parity * d.nr + r] + (double)d.dt[r]);
 }
 
-__global__ void k_fp64_tables(Dev d, LMatD *out, const int *lrob, int n) {
+__global__ void k_fp64_tables(Dev d, LMatD *out, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const LMat &m = d.lmat[i];
-        out[i] = make_lmatd(m, m.dmcN, m.dmcP, m.fixN, m.fixP, d.dt[lrob[i]]);
+        out[i] = make_lmatd(m, m.dmcN, m.dmcP, m.fixN, m.fixP, d.dt[m.robot]);
     }
     if (d.actv && i < d.nv) d.actv[i] = actuation_voxel(d.phase[i]);
 }
@@ -50,9 +50,9 @@ void launch_voxels_fp64(const Dev &d, int parity, cudaStream_t s) {
 void launch_actuation(const Dev &d, int parity, cudaStream_t s) {
     if (d.act) k_actuation<<<(d.nr + 31) / 32, 32, 0, s>>>(d, parity);
 }
-void launch_fp64_tables(const Dev &d, LMatD *lmatd, const int *lrob, int n, cudaStream_t s) {
+void launch_fp64_tables(const Dev &d, LMatD *lmatd, int n, cudaStream_t s) {
     const int k = d.nv > n ? d.nv : n;
-    if (k) k_fp64_tables<<<(k + 255) / 256, 256, 0, s>>>(d, lmatd, lrob, n);
+    if (k) k_fp64_tables<<<(k + 255) / 256, 256, 0, s>>>(d, lmatd, n);
     launch_actuation(d, 0, s);
 }
 

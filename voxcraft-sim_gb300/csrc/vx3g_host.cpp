@@ -271,6 +271,7 @@ struct vx3g_ctx {
     bool res_chosen = false;    // ... as decided at creation
     int res_from = 1;           // ... in calls of this many steps and more
     bool res_always = false;    // ... or of any number (vx3g_choose_steps)
+    std::vector<int2> res_tables;   // their tables on the host, until the copy is done
     std::vector<int> lmoff, vmoff;  // each robot's first link and voxel material
     std::vector<cudaStream_t> res_stream;
     cudaEvent_t res_fork = nullptr;
@@ -447,10 +448,18 @@ int plan_resident(vx3g_ctx *c, bool any) {
     constexpr size_t kHalf = 115000;         // shared memory with which two CTAs share an SM
     constexpr int kHalfThreads = kResThreads / 2;
     const int goal = std::max(96, d.nv / (2 * 152));  // voxels per CTA that fill the 152 SMs twice
+    struct Cta {
+        int l0, l1, entries;  // its links; their entries axis by axis, each axis up to whole warps
+    };
+    struct Bundle {
+        ResBundle b;
+        size_t ctas;  // its first in ctas
+    };
     struct Plan {
-        std::vector<ResBundle> b;
+        std::vector<Bundle> b;
         size_t smem = 0;
     };
+    std::vector<Cta> ctas;
     Plan by[kMost];
     auto up = [](int x, int m) { return (x + m - 1) / m * m; };
     // the first link whose positive end is voxel v or a later one
@@ -458,19 +467,18 @@ int plan_resident(vx3g_ctx *c, bool any) {
         const auto f = c->ends.begin();
         return (int)(std::lower_bound(f + b.l0, f + b.l0 + b.nl, v, [](const int2 &e, int x) { return e.y < x; }) - f);
     };
-    // links l0 to l1 - 1 by axis (two sums that vectorise; a counter per axis waits on its own stores)
-    auto axes = [&](int l0, int l1) {
-        int n1 = 0, n2 = 0;
-        for (int l = l0; l < l1; l++) n1 += c->laxis[l] == 1, n2 += c->laxis[l] == 2;
-        return std::array<int, 3>{l1 - l0 - n1 - n2, n1, n2};
-    };
-    // most entries a CTA's links take axis by axis, with K CTAs
-    auto entries = [&](const ResBundle &b, int K) {
+    // the CTAs of K; the most entries of one
+    auto split = [&](const ResBundle &b, int K, size_t at) {
         int most = 0;
-        for (int j = 0; j < K; j++) {
-            const int a = std::min(b.v0 + j * b.q, b.v0 + b.nv), z = std::min(a + b.q, b.v0 + b.nv);
-            const auto n = axes(link_at(b, a), link_at(b, z));
-            most = std::max(most, up(n[0], 32) + up(n[1], 32) + up(n[2], 32));
+        ctas.resize(at);
+        for (int j = 0, l0 = b.l0; j < K; j++) {
+            const int l1 = link_at(b, std::min(b.v0 + (j + 1) * b.q, b.v0 + b.nv));
+            // links by axis (two sums that vectorise; a counter per axis waits on its own stores)
+            int n1 = 0, n2 = 0;
+            for (int l = l0; l < l1; l++) n1 += c->laxis[l] == 1, n2 += c->laxis[l] == 2;
+            ctas.push_back({l0, l1, up(l1 - l0 - n1 - n2, 32) + up(n1, 32) + up(n2, 32)});
+            most = std::max(most, ctas.back().entries);
+            l0 = l1;
         }
         return most;
     };
@@ -484,23 +492,22 @@ int plan_resident(vx3g_ctx *c, bool any) {
         if (b.nlm > kResMats || b.nvm > kResMats) b.nlm = b.nvm = 0;
         if (b.nv > 65535) return VX3G_OK;  // voxels are numbered in 16 bits
         int K = 1;
-        bool fits = false;
+        const size_t at = ctas.size();
         for (; K <= kMost; K++) {
             b.q = up((b.nv + K - 1) / K, 16);
-            if (b.q > 4096) continue;  // far beyond any CTA
-            b.lc = up(entries(b, K), 16);
-            fits = steps_mixed_bytes(b.q, b.lc) <= (K == 1 || K == kMost ? (size_t)kResSmem : kHalf);
-            if (fits && (b.q <= goal * 4 / 3 || K == kMost)) break;
+            if (b.q > (K < kMost ? goal * 4 / 3 : 4096)) continue;
+            b.lc = up(split(b, K, at), 16);
+            if (steps_mixed_bytes(b.q, b.lc) <= (K == 1 || K == kMost ? (size_t)kResSmem : kHalf)) break;
         }
-        if (!fits) return VX3G_OK;
-        by[K - 1].b.push_back(b);
+        if (K > kMost) return VX3G_OK;
+        by[K - 1].b.push_back({b, at});
         by[K - 1].smem = std::max(by[K - 1].smem, steps_mixed_bytes(b.q, b.lc));
         r = e;
     }
     CU(init_steps_mixed());
     auto threads = [&](const Plan &p) {
         int lc = 0;
-        for (const ResBundle &b : p.b) lc = std::max(lc, b.lc);
+        for (const Bundle &x : p.b) lc = std::max(lc, x.b.lc);
         return std::min(std::max(up(lc, 64), 64), p.smem <= kHalf ? kHalfThreads : kResThreads);
     };
     std::vector<ResLoad> load;
@@ -511,7 +518,7 @@ int plan_resident(vx3g_ctx *c, bool any) {
         CU(steps_mixed_active(K, threads(p), p.smem, &act));
         if (act < 1) return VX3G_OK;
         double lc = 0, most = 0;
-        for (const ResBundle &b : p.b) lc += b.lc, most = std::max<double>(most, b.lc);
+        for (const Bundle &x : p.b) lc += x.b.lc, most = std::max<double>(most, x.b.lc);
         load.push_back(ResLoad{K, (double)p.b.size() / act, lc / p.b.size(), most, p.smem > kHalf});
     }
     if (load.empty()) return VX3G_OK;
@@ -519,33 +526,45 @@ int plan_resident(vx3g_ctx *c, bool any) {
     const double many = resident_us(load), passes = passes_us(d.nv, d.nl, c->nr);
     if (!any && many > (several ? 0.8 : 0.95) * passes) return VX3G_OK;
     c->res_from = resident_from(many, passes, d.nv, several);
+    // all tables in one allocation and one copy: per size its bundles, then (entries, links) of each CTA
+    std::vector<int2> &tab = c->res_tables;
+    constexpr size_t kPer = sizeof(ResBundle) / sizeof(int2);
+    static_assert(sizeof(ResBundle) % sizeof(int2) == 0, "bundles are copied as pairs");
+    tab.clear();
+    struct At {
+        int K;
+        size_t bundles, ctas, links, n;
+        int order;
+    };
+    std::vector<At> at;
+    int entry = 0;
     for (int K = kMost; K >= 1; K--) {
         Plan &p = by[K - 1];
         if (p.b.empty()) continue;
         // the longest first: the SMs take the rest as they come free
-        std::stable_sort(p.b.begin(), p.b.end(), [](const ResBundle &a, const ResBundle &b) { return a.nl > b.nl; });
-        std::vector<int2> ctas, links;
-        int at = 0;
-        for (const ResBundle &b : p.b) {
+        std::stable_sort(p.b.begin(), p.b.end(), [](const Bundle &a, const Bundle &b) { return a.b.nl > b.b.nl; });
+        const size_t nb = p.b.size(), n = nb * K;
+        At x{K, tab.size(), tab.size() + kPer * nb, tab.size() + kPer * nb + n, n, entry};
+        tab.resize(x.links + n);
+        for (size_t i = 0; i < nb; i++) {
+            memcpy(&tab[x.bundles + kPer * i], &p.b[i].b, sizeof(ResBundle));
             for (int j = 0; j < K; j++) {
-                const int a = std::min(b.v0 + j * b.q, b.v0 + b.nv), z = std::min(a + b.q, b.v0 + b.nv);
-                const int l0 = link_at(b, a), l1 = link_at(b, z);
-                const auto n = axes(l0, l1);
-                const int len = up(n[0], 32) + up(n[1], 32) + up(n[2], 32);
-                links.push_back(make_int2(l0, l1));
-                ctas.push_back(make_int2(at, len));
-                at += len;
+                const Cta &t = ctas[p.b[i].ctas + j];
+                tab[x.ctas + i * K + j] = make_int2(entry - x.order, t.entries);
+                tab[x.links + i * K + j] = make_int2(t.l0, t.l1);
+                entry += t.entries;
             }
         }
-        ResBundle *pb;
-        int2 *pc, *pl;
-        int *po, rc;
-        if ((rc = c->upload(&pb, p.b)) || (rc = c->upload(&pc, ctas)) || (rc = c->upload(&pl, links)) ||
-            (rc = c->alloc(&po, at)))
-            return rc;
-        CU(launch_res_order(d, pl, pc, (int)ctas.size(), po, c->stream));
-        CU(cudaStreamSynchronize(c->stream));  // the host vectors end here
-        c->res.push_back(ResClass{K, threads(p), (int)p.b.size(), p.smem, pb, pc, po});
+        at.push_back(x);
+    }
+    int2 *mem;
+    if (int rc = c->alloc(&mem, tab.size() + ((size_t)entry + 1) / 2)) return rc;
+    CU(cudaMemcpyAsync(mem, tab.data(), tab.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
+    for (const At &x : at) {
+        const Plan &p = by[x.K - 1];
+        int *order = (int *)(mem + tab.size()) + x.order;
+        CU(launch_res_order(d, mem + x.links, mem + x.ctas, (int)x.n, order, c->stream));
+        c->res.push_back(ResClass{x.K, threads(p), (int)p.b.size(), p.smem, (const ResBundle *)(mem + x.bundles), mem + x.ctas, order});
     }
     // the cluster sizes run side by side, the first on the context's own stream
     if (c->res.size() > 1) {
@@ -593,7 +612,6 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
 
     std::vector<VMat> vmats;
     std::vector<LMat> lmats;
-    std::vector<int> lrob;  // the robot of each link material
     c->lmoff.assign(c->nr + 1, 0);
     c->vmoff.assign(c->nr + 1, 0);
     bool any_actuated = false;
@@ -952,7 +970,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
                 vnb_h[6 * (size_t)c->ends[l].y + 2 * a + 1] = c->ends[l].x;  // positive end: toward -axis
             }
         }
-        lrob.resize(lmats.size(), r);
+        for (size_t i = c->lmoff[r]; i < lmats.size(); i++) lmats[i].robot = r;
         c->lmoff[r + 1] = (int)lmats.size();
         c->vmoff[r + 1] = (int)vmats.size();
         // lists in shared memory when the robot fits (lattice coordinates below 512, packed in 10 bits each)
@@ -1055,11 +1073,10 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     d.nvm = (int)vmats.size();
     float4 *lrow = nullptr, *vrow = nullptr;
     LMatD *lmatd = nullptr;  // FP64: link constants and actuation phases (filled once the time step is known)
-    int *lrob_d = nullptr;
-    if ((rc = c->upload(&lrob_d, lrob))) return rc;
     d.lrow = d.vrow = nullptr;
     if (d.mixed) {
-        if ((rc = c->alloc(&lrow, 4 * lmats.size())) || (rc = c->alloc(&vrow, 3 * vmats.size()))) return rc;
+        if ((rc = c->alloc(&lrow, 4 * lmats.size() + 3 * vmats.size()))) return rc;
+        vrow = lrow + 4 * lmats.size();
         d.lrow = lrow;
         d.vrow = vrow;
     } else {
@@ -1182,10 +1199,11 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
     c->res_chosen = c->res_on;
     launch_init_temperature(d, c->precision == VX3G_PRECISION_MIXED, c->stream);
     launch_dt(d, c->scratch, c->stream);
-    if (d.mixed) launch_rows_mixed(d, lrow, vrow, lrob_d, c->stream);
-    else launch_fp64_tables(d, lmatd, lrob_d, (int)lmats.size(), c->stream);
+    if (d.mixed) launch_rows_mixed(d, lrow, vrow, c->stream);
+    else launch_fp64_tables(d, lmatd, (int)lmats.size(), c->stream);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(c->stream));
+    c->res_tables = {};
     return VX3G_OK;
 }
 
@@ -1926,6 +1944,8 @@ int vx3g_choose_steps(vx3g_ctx *c, int way) {
     CU(cudaSetDevice(c->device));
     if (way == 2 && c->res.empty()) {
         if (int rc = plan_resident(c, true)) return rc;
+        CU(cudaStreamSynchronize(c->stream));
+        c->res_tables = {};
         if (c->res.empty()) return fail(VX3G_ERR_UNSUPPORTED, "the many-step kernel does not handle this batch");
     }
     c->res_on = way == 0 ? c->res_chosen : way == 2;

@@ -75,6 +75,7 @@ struct LMat {  // one link material (global index), oriented: (negative end, pos
     int fixN, fixP;   // the ends' materials are Fixed
     int lin;          // 1: linear model (VX3_Material::linear); 0: data points d.ss[sso .. sso+ssn)
     int ssn, sso;     // stress-strain points of a non-linear model: (0,0), then the model's from (0,0) on
+    int robot;
 };
 
 struct LMatD {  // FP64 contexts: a link material's constants as the FP64 link pass multiplies by them
@@ -298,9 +299,9 @@ inline int fp64_threads(int n, int most) {
 // launchers (defined in the .cu files)
 void launch_links_fp64(const Dev &d, cudaStream_t s);
 void launch_voxels_fp64(const Dev &d, int parity, cudaStream_t s);
-// FP64 contexts: fills lmatd (lrob: the robot of each link material) and actv; and act for the
+// FP64 contexts: fills lmatd and actv; and act for the
 // step of the given parity (again whenever T was written by anything but the voxel pass)
-void launch_fp64_tables(const Dev &d, LMatD *lmatd, const int *lrob, int n, cudaStream_t s);
+void launch_fp64_tables(const Dev &d, LMatD *lmatd, int n, cudaStream_t s);
 void launch_actuation(const Dev &d, int parity, cudaStream_t s);
 // launch shapes of the mixed-precision passes (vx3g_mixed.cu), chosen by vx3g_autotune
 struct LaunchShape { int threads, min_blocks; };
@@ -341,7 +342,7 @@ void launch_init_temperature(const Dev &d, int mixed, cudaStream_t s);
 // the main pass, which skips them)
 void launch_voxels_bc_mixed(const Dev &d, int parity, cudaStream_t s);
 void launch_init_temperature_mixed(const Dev &d, cudaStream_t s);
-void launch_rows_mixed(const Dev &d, float4 *lrow, float4 *vrow, const int *lrob, cudaStream_t s);
+void launch_rows_mixed(const Dev &d, float4 *lrow, float4 *vrow, cudaStream_t s);
 void launch_dt(const Dev &d, double *maxfreq2_scratch, cudaStream_t s);
 // surface-voxel collision of one step: displacement check and list rebuild (one
 // cooperative kernel), then the narrow phase

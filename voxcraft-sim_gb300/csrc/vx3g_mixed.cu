@@ -840,11 +840,11 @@ cudaError_t launch_steps_mixed(const Dev &d, int parity, int n, const ResClass &
     return cudaLaunchKernelEx(&cfg, c.K > 1 ? k_steps_mixed<true> : k_steps_mixed<false>, d, parity, n, c.bundles, c.ctas, c.order);
 }
 
-// the material rows (lrob: the robot of each link material), once the time step is known
-__global__ void k_rows_mixed(Dev d, float4 *lrow, float4 *vrow, const int *lrob) {
+// the material rows, once the time step is known
+__global__ void k_rows_mixed(Dev d, float4 *lrow, float4 *vrow) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < d.nlm) {
-        const mx::LinkC c = mx::link_consts_mx(d.lmat[i], d.dt[lrob[i]]);
+        const mx::LinkC c = mx::link_consts_mx(d.lmat[i], d.dt[d.lmat[i].robot]);
         lrow[i] = c.ra, lrow[d.nlm + i] = c.rb, lrow[2 * (size_t)d.nlm + i] = c.rc, lrow[3 * (size_t)d.nlm + i] = c.re;
     }
     if (i < d.nvm) {
@@ -852,9 +852,9 @@ __global__ void k_rows_mixed(Dev d, float4 *lrow, float4 *vrow, const int *lrob)
         vrow[i] = mx::vox_row_a(m), vrow[d.nvm + i] = mx::vox_row_b(m), vrow[2 * (size_t)d.nvm + i] = mx::vox_row_c(m);
     }
 }
-void launch_rows_mixed(const Dev &d, float4 *lrow, float4 *vrow, const int *lrob, cudaStream_t s) {
+void launch_rows_mixed(const Dev &d, float4 *lrow, float4 *vrow, cudaStream_t s) {
     const int n = d.nlm > d.nvm ? d.nlm : d.nvm;
-    if (n) k_rows_mixed<<<(n + 127) / 128, 128, 0, s>>>(d, lrow, vrow, lrob);
+    if (n) k_rows_mixed<<<(n + 127) / 128, 128, 0, s>>>(d, lrow, vrow);
 }
 void launch_init_temperature_mixed(const Dev &d, cudaStream_t s) {
     if (d.nv) k_init_temperature_mixed<<<(d.nv + 255) / 256, 256, 0, s>>>(d);
