@@ -1796,7 +1796,7 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
             fclose(f);
         }
         const size_t at = cache.find("\"" + key + "\": [");
-        int a = -1, b = -1, fk = 0;
+        int a = -1, b = -1, fk = c->fork_early;  // (an entry without a fork point: it was not timed)
         if (at != std::string::npos &&
             sscanf(cache.c_str() + at + key.size() + 5, "%d, %d, %d", &a, &b, &fk) >= 2 && a >= 0 && a < kMixedShapes &&
             b >= 0 && b < kMixedShapes) {
@@ -1852,7 +1852,7 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
     constexpr int G = 8;
     const int reps = n_fork / (2 * G);
     double tf[2] = {0.0, 0.0};
-    if (reps >= 2) {
+    if (reps >= 2) {  // else it stays as it is
         cudaGraphExec_t gx[2] = {nullptr, nullptr};
         const int p0 = (int)(c->steps & 1);  // G is even: every launch starts at this parity
         for (int m = 0; m < 2; m++) {
@@ -1889,7 +1889,7 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
         cudaGraphExecDestroy(gx[0]);
         cudaGraphExecDestroy(gx[1]);
     }
-    c->fork_early = reps >= 2 && tf[1] < tf[0] ? 1 : 0;
+    if (reps >= 2) c->fork_early = tf[1] < tf[0] ? 1 : 0;
     for (int i = 2 * reps * G; i < n_fork; i++) {  // the rest of the n_steps, at the chosen point
         CU(enqueue_step(c, (int)(c->steps & 1)));
         c->steps++;
@@ -1897,11 +1897,11 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
     for (auto &e : ev) cudaEventDestroy(e);
     for (auto &g : c->graph)
         if (g) cudaGraphExecDestroy(g), g = nullptr;
-    if (cache_json) {  // flat JSON object {"<gpu>|mixed|nv|nl|ns": [link shape, voxel shape, fork point], ...}
+    if (cache_json) {  // flat JSON object {"<gpu>|mixed <shapes>|nv|nl|ns": [link shape, voxel shape, fork point if timed], ...}
         std::string body = cache;
         const size_t close = body.rfind('}');
-        const std::string entry = "\"" + key + "\": [" + std::to_string(bl) + ", " + std::to_string(bv) + ", " +
-                                  std::to_string(c->fork_early) + "]";
+        const std::string entry = "\"" + key + "\": [" + std::to_string(bl) + ", " + std::to_string(bv) +
+                                  (reps >= 2 ? ", " + std::to_string(c->fork_early) : "") + "]";
         if (close == std::string::npos || body.find('"') == std::string::npos) {
             body = "{\n  " + entry + "\n}\n";
         } else {
