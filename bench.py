@@ -76,6 +76,28 @@ def algorithmic_bytes(nv, nl, ns, actuated, contacts=0):
     return dict(links=link, voxels=voxel, collision=coll)
 
 
+def launches_per_call(steps, graph_chunk, plan, mixed, collisions, global_grid):
+    """Kernel launches of one vx3g_step call of `steps` steps (vx3g_step_plan: `plan`).  Passes: link and
+    voxel pass; with collisions the list rebuild kernel (it returns at once unless a rebuild is due), the
+    global grid's list kernel (the same) and the contact evaluation; the displacement check is a kernel of
+    its own in FP64, in mixed precision only in the first step of a graph, or of a call that begins with
+    single steps (the voxel pass does it after that)."""
+    if plan["many_from"] and steps >= plan["many_from"]:  # many steps in one launch, per cluster size
+        return -(-steps // plan["most"]) * plan["launches"]
+    n = 2 * steps
+    if collisions:
+        graphs = steps // graph_chunk if graph_chunk > 0 else 0
+        n += (3 if global_grid else 2) * steps + ((graphs or 1) if mixed else steps)
+    return n
+
+
+def many_step_bytes(nv, nl):
+    """Bytes that one launch of the many-step kernel moves: the state read and written once (positions,
+    orientations, momenta, temperatures, flags; link state, strains, flags), phases, link ends and order
+    read, the forces at the six faces written."""
+    return 432 * nv + 100 * nl
+
+
 class ClockSampler:
     """nvidia-smi sampling of SM clocks and throttle reasons during the timed region."""
 
@@ -471,8 +493,8 @@ def main():
     # kernel with the largest time: the link pass, the voxel pass or the contact evaluation
     passes = b.time_passes(20)
     ab = algorithmic_bytes(nv, nl, ns_coll, actuated)
-    kernel_ms = {"k_links_mixed" if prec else "k_links": passes["links"],
-                 "k_voxels_mixed" if prec else "k_voxels": passes["voxels"]}
+    kernel_ms = {"k_links_mixed" if prec else "k_links_fp64": passes["links"],
+                 "k_voxels_mixed" if prec else "k_voxels_fp64": passes["voxels"]}
     if ns_coll:
         kernel_ms["k_coll_eval_mixed" if prec else "k_coll_eval"] = passes["contact_eval"]
     kernel_bytes = dict(zip(kernel_ms, [ab["links"], ab["voxels"], ab["collision"]]))
@@ -480,17 +502,17 @@ def main():
     peak, peak_kind = peaks()
     achieved = kernel_bytes[dom] / (kernel_ms[dom] / 1e3) / 1e9 if kernel_ms[dom] > 0 else 0.0
     traffic = ncu_traffic(args.workload, args.precision, dom)
-    # link pass + voxel pass; collision: the cooperative list rebuild kernel (it returns at once
-    # unless a rebuild is due), the global grid's list kernel (the same) and the contact evaluation;
-    # the displacement check is a kernel of its own in FP64, and in mixed precision in the first step
-    # of a graph (the voxel pass does it after that)
-    checks = 0 if not ns_coll else (C // G + (1 if 0 < C < G else 0)) if prec else C
-    launches_per_call = (2 + ((3 if global_grid else 2) if ns_coll else 0)) * C + checks
-    # mixed-precision workloads without collisions: up to 256 steps in one launch (counted once,
-    # although robots of further cluster sizes have launches of their own beside it)
-    resident = bool(prec) and not ns_coll
-    if resident:
-        launches_per_call = -(-C // 256)
+    plan = b.step_plan()
+    launches = launches_per_call(C, G, plan, bool(prec), ns_coll > 0, global_grid)
+    resident = bool(plan["many_from"]) and C >= plan["many_from"]
+    moved = (ab["links"] + ab["voxels"] + ab["collision"]) * C  # per bench step
+    if resident:  # the passes timed above are no part of the measured run
+        dom, traffic = "k_steps_mixed", ncu_traffic(args.workload, args.precision, "k_steps_mixed")
+        rounds = launches // plan["launches"]  # its cluster sizes run side by side
+        kernel_ms = {dom: total_ms / (K * rounds)}
+        moved = many_step_bytes(nv, nl) * rounds
+        ab = {dom: many_step_bytes(nv, nl)}
+        achieved = ab[dom] / (kernel_ms[dom] / 1e3) / 1e9
     shapes = [int(x) for x in b.launch_shapes()]
     b.close()
 
@@ -546,18 +568,17 @@ def main():
                    "collision_surface_voxels": ns_coll, "precision": args.precision,
                    "physics_steps_per_bench_step": C, "window": f"physics steps 0-{K * C} of a fresh context "
                    f"(the configuration runs {CONFIG_STEPS[args.workload]})",
-                   "cuda_graphs": not args.no_graphs, "graph_chunk": G,
+                   "cuda_graphs": not args.no_graphs, "graph_chunk": G, "step_plan": plan,
                    "launch_shapes": {"links": shapes[:2], "voxels": shapes[2:]},
                    "l2": "512 MB overwrite before every timed bench step",
                    "parallelism": f"robot shards x{world} of {n_total} robots" if args.shard else f"replicas x{world}"},
-        "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": "issue and barriers" if resident else "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind, "traffic": traffic,
-                     "kernel_ms": kernel_ms, "pass_ms": passes, "algorithmic_bytes_per_launch": ab,
+                     "kernel_ms": kernel_ms, "pass_ms": None if resident else passes, "algorithmic_bytes_per_launch": ab,
                      # this GPU's algorithmic bytes over the job time, against one GPU's peak
-                     "whole_step_algorithmic_gbs": (ab["links"] + ab["voxels"] + ab["collision"]) * C * K
-                     / (total_ms / 1e3) / 1e9},
+                     "whole_step_algorithmic_gbs": moved * K / (total_ms / 1e3) / 1e9},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        "gpu_launches": launches_per_call * K,
+        "gpu_launches": launches * K,
         "clocks": clk.summary(),
         "robot_status_nonzero": int(np.count_nonzero(status)),
     }
