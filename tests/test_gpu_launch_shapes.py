@@ -61,3 +61,11 @@ def test_all_shapes(tmp_path):
         got = _run(path)
         for name in want:
             assert np.array_equal(got[name], want[name], equal_nan=True), (k, name)
+
+
+@pytest.mark.parametrize("cells,threads", [(2, 32), (10, 32), (40, 64), (60, 256)])
+def test_fp64_shapes_follow_the_batch(cells, threads):
+    """Blocks of one warp until each of the 152 SMs has eight: 38,912 voxels, then wider ones."""
+    b = abi.Batch([wl.solid_block(cells)], abi.PRECISION_FP64)
+    assert list(b.launch_shapes())[2:] == [threads, 1]
+    b.close()

@@ -1920,9 +1920,9 @@ int vx3g_autotune(vx3g_ctx *c, int n_steps, const char *cache_json) {
 int vx3g_launch_shapes(vx3g_ctx *c, int32_t *shapes4) {
     if (!c || !shapes4) return fail(VX3G_ERR_INVALID, "bad arguments to vx3g_launch_shapes");
     const bool mx = c->precision == VX3G_PRECISION_MIXED;
-    shapes4[0] = mx ? kLinkShapes[c->shape_links].threads : 256;
+    shapes4[0] = mx ? kLinkShapes[c->shape_links].threads : fp64_threads(c->d.nl, 256);
     shapes4[1] = mx ? kLinkShapes[c->shape_links].min_blocks : 1;
-    shapes4[2] = mx ? kVoxelShapes[c->shape_voxels].threads : 256;
+    shapes4[2] = mx ? kVoxelShapes[c->shape_voxels].threads : fp64_threads(c->d.nv, 256);
     shapes4[3] = mx ? kVoxelShapes[c->shape_voxels].min_blocks : 1;
     return VX3G_OK;
 }
