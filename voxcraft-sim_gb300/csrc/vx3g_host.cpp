@@ -447,7 +447,7 @@ int plan_resident(vx3g_ctx *c, bool any) {
     constexpr int kMost = 8;                 // CTAs of a cluster (portable size)
     constexpr size_t kHalf = 115000;         // shared memory with which two CTAs share an SM
     constexpr int kHalfThreads = kResThreads / 2;
-    const int goal = std::max(96, d.nv / (2 * 152));  // voxels per CTA that fill the 152 SMs twice
+    const int goal = std::max(96, d.nv / (2 * kSMs));  // voxels per CTA that fill the SMs twice
     struct Cta {
         int l0, l1, entries;  // its links; their entries axis by axis, each axis up to whole warps
     };

@@ -290,9 +290,10 @@ __device__ __forceinline__ double4 load_state(const Dev &d, const double4 *a, in
 // the busiest SM's count of warps, not by occupancy: blocks of one warp spread a small batch over
 // all 152 SMs (100 steps of a 10^3 block, 2,700 links: 5.08 ms in blocks of 256 threads, 2.79 ms in
 // blocks of 32).  Once every SM has eight blocks, larger ones cost nothing and launch faster.
+constexpr int kSMs = 152;  // of GB300
 inline int fp64_threads(int n, int most) {
     int t = 32;
-    while (t < most && (n + t - 1) / t > 152 * 8) t *= 2;
+    while (t < most && (n + t - 1) / t > kSMs * 8) t *= 2;
     return t;
 }
 
