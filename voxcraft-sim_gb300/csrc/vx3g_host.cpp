@@ -1195,7 +1195,7 @@ int build(vx3g_ctx *c, const vx3g_batch_desc *desc) {
         // body rarely does (a folded 64^3 body 54.4 us a step against 55.8 so)
         c->fork_early = d.nhash == 0 ? 1 : 0;
     }
-    if ((rc = plan_resident(c, false))) return rc;
+    if (c->chunk != INT32_MAX && (rc = plan_resident(c, false))) return rc;  // (else every step's kernels one by one)
     c->res_chosen = c->res_on;
     launch_init_temperature(d, c->precision == VX3G_PRECISION_MIXED, c->stream);
     launch_dt(d, c->scratch, c->stream);
