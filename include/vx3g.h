@@ -202,7 +202,8 @@ typedef struct vx3g_batch_desc {
     int device;                     /* CUDA device ordinal */
     int graph_chunk;                /* steps captured per CUDA graph launch (0 -> 100; < 0: no
                                        graphs, every step's kernels launched one by one, e.g.
-                                       for a per-kernel profiler) */
+                                       for a per-kernel profiler; the many-step kernel of
+                                       vx3g_step_plan is then not taken) */
 } vx3g_batch_desc;
 
 typedef struct vx3g_ctx vx3g_ctx;
@@ -215,12 +216,15 @@ void vx3g_destroy(vx3g_ctx *ctx);
 const char *vx3g_last_error(void);
 
 /* Advances every robot by n_steps time steps (asynchronous on the context's
- * stream; robots that diverged stay frozen).  Full chunks run as CUDA graphs. */
+ * stream; robots that diverged stay frozen).  Full chunks run as CUDA graphs; where
+ * vx3g_step_plan says so, one kernel takes up to 256 steps instead. */
 int vx3g_step(vx3g_ctx *ctx, int n_steps);
 int vx3g_synchronize(vx3g_ctx *ctx);
 /* Captures and instantiates the CUDA graphs vx3g_step replays (both step parities)
  * without running them, so that the first vx3g_step of a latency-sensitive loop does
- * not pay for the capture.  Optional; no counterpart in the reference. */
+ * not pay for the capture.  Captures nothing where no graph would be replayed (calls of
+ * graph_chunk steps go to the many-step kernel).  Optional; no counterpart in the
+ * reference. */
 int vx3g_prepare_graphs(vx3g_ctx *ctx);
 /* The context's CUDA stream (a cudaStream_t), for event timing by the caller. */
 void *vx3g_stream(vx3g_ctx *ctx);
@@ -321,9 +325,12 @@ int vx3g_recommended_dt_noalloc(vx3g_ctx *ctx, double *rdt);
  * vx3g_autotune: advances n_steps exactly like vx3g_step (results identical),
  *   timing the link and voxel passes of a mixed-precision context under each of
  *   their compiled launch shapes (threads per block x minimum resident blocks),
- *   and keeps the fastest.  With cache_json (a path, or NULL) the choice is read
- *   from / appended to a flat JSON object keyed by GPU name and batch size; a
- *   cached choice is applied without timing.  FP64 contexts just step.
+ *   and keeps the fastest (24 steps and more; from 64 also the fork point of the
+ *   contact side stream).  With cache_json (a path, or NULL) the choice is read
+ *   from / appended to a flat JSON object keyed by GPU name, number of compiled shapes
+ *   and batch size; a cached choice is applied without timing.  FP64 contexts just
+ *   step.  On a context that vx3g_step_plan sends to the many-step kernel these steps
+ *   are by the passes all the same, and the choice serves the calls that go by them.
  * vx3g_launch_shapes: the shapes in use: {link threads, link min blocks, voxel
  *   threads, voxel min blocks}.
  * vx3g_step_plan: how vx3g_step advances the context, decided when it was created.
@@ -349,9 +356,10 @@ int vx3g_choose_steps(vx3g_ctx *ctx, int way);
  *   context's stream (evicts the L2 cache between timed iterations).
  * vx3g_time_passes: runs each per-step pass `iters` times on its own, captured
  *   in one CUDA graph as the step graphs run it, between CUDA events, and
- *   returns the mean device time per pass in milliseconds (ms4[4]) for: [0] link pass, [1] collision passes (all kernels of the
- *   broad and narrow phase together), [2] voxel pass, [3] the contact evaluation
- *   kernel alone.  It advances the state like extra steps would; use it after
+ *   returns the mean device time per pass in milliseconds (ms4[4]) for: [0] link pass,
+ *   [1] collision passes (all kernels of the broad and narrow phase together), [2] voxel
+ *   pass, [3] the contact evaluation kernel alone (also where vx3g_step takes the
+ *   many-step kernel, which runs none of them).  It advances the state like extra steps would; use it after
  *   the measured run. */
 int vx3g_time_steps(vx3g_ctx *ctx, int n_steps, float *ms);
 int vx3g_flush_l2(vx3g_ctx *ctx, size_t bytes);

@@ -470,8 +470,9 @@ void launch_voxels_mixed(const Dev &d, int parity, cudaStream_t s, int shape, bo
 // links whose positive end is among them (links are made in the voxel order of that end); the
 // negative end may be in a CTA of lower rank, reached through distributed shared memory.  Two
 // barriers per step: after the links (forces written to the six rows of each end) and after the
-// voxels.  Bound by instruction issue and the two phases' dependency chains: 62% of the issue
-// slots used, 83 us a step on those 1024 robots; 2.7 us instead of 5.9 on one robot of 104 voxels.
+// voxels.  Bound by those barriers and by instruction issue: 43 to 55% of the issue slots of an SM with
+// work, 3.3 to 5.3 stall cycles of an instruction at the barriers; 83 us a step on those 1024 robots, 2.7
+// instead of 5.9 on one robot of 104 voxels.
 // Two CTAs of 384 threads per SM (113 KB each), so that one's loads overlap the other's
 // arithmetic: 1200-voxel robots 80 us a step against 101 with one CTA of 768 threads.
 struct ResRobot {
