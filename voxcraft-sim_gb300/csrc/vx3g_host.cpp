@@ -371,59 +371,65 @@ int check_math_program(const vx3g_math_token *t, int *len, bool *reads_pos, std:
     return VX3G_ERR_INVALID;
 }
 
-// Microseconds of a step by k_steps_mixed and by the two passes, both measured for 620 batches of 1 to 1600
-// robots of 2^3 to 18^3 cells, filled or to 60%, one size or mixed (half of them drawn after the fit).  A
-// batch of one cluster size is estimated within 8% in nine of ten cases, one of several sizes within 20%, the
-// passes within 10%, hence the margins of 5% and 20% in plan_resident: the kernel is taken in 405 of the
-// batches, for a geometric mean of 1.32 times the passes' speed (1.34 with the better one each time), and is
-// slower than the passes by more than 2% in three (3, 6 and 11%).  It is fast where a step of the passes
-// is latency (a robot of 100 voxels 2.4 us against 5.4) and where the state is beyond the L2 (800,000 voxels of
-// 8^3 robots 81 us against 142); in between, and for robots of a whole SM per thread block, the passes are
-// (40 robots of 13^3: 21 us against 16).
+// Microseconds of a step by k_steps_mixed and by the two passes, both measured for 1247 batches of 1 to 1600
+// robots of 2^3 to 18^3 cells, filled or to 60%, one size or mixed (884 of them drawn).  Of nine in ten a batch
+// of one cluster size is estimated within 8%, one of several sizes within 20% (whose launches now fill one wave
+// and now begin another), the passes within 8%.  Taken where its estimate is below the passes' (plan_resident),
+// the kernel makes the 1247 a geometric mean of 1.368 times as fast, of 1.373 with the better way each time; 33
+// are slower than by the passes by more than 2% (one by 24, the next by 17).  It is the better way where a step
+// of the passes is latency (a robot of 100 voxels 2.4 us against 5.4) and where the state is beyond the L2
+// (800,000 voxels of 8^3 robots 81 us against 142); not in between, nor for robots of a whole SM per thread
+// block (40 robots of 13^3: 21 us against 16).
+constexpr double kAlone = 0.43;  // waves up to which every CTA finds an SM for itself
 struct ResLoad {
-    int K;                // CTAs of a cluster
-    double waves;         // bundles by those that run at once
-    double links, most;   // links of a CTA, on average and at most
-    bool whole;           // a CTA has an SM for itself
+    double waves;           // bundles by those that run at once
+    bool whole;             // a CTA has an SM for itself
+    double alone, shared;   // a bundle's step with an SM for each of its CTAs, and with two on one: mean
+    double alone1, shared1; // ... and the longest
 };
-// one wave: a CTA's step grows with its links, more slowly while it has an SM to itself (`alone`) than when
-// two share one's issue slots, and by a jump where its threads take the links in two rounds
-double wave_us(int K, double links, bool whole, bool alone) {
+// a CTA's step grows with its links, more slowly while it has an SM to itself than when two share one's issue
+// slots, and by a jump where its threads take the links in two rounds
+double bundle_us(int K, double links, bool whole, bool alone) {
     if (K == 1) return 2.05 + (alone || whole ? 0.0038 : 0.0078) * links;
     if (whole) return (links <= kResThreads ? 3.8 : 5.0) + 0.0025 * links;
     if (links <= kResThreads / 2) return alone ? 3.05 + 0.0025 * links : 3.4 + 0.0042 * links;
     return alone ? 5.4 + 0.0006 * links : 5.0 + 0.005 * links;
 }
+double total_waves(const std::vector<ResLoad> &load) {
+    double w = 0;
+    for (const ResLoad &l : load) w += l.waves;
+    return w;
+}
 double resident_us(const std::vector<ResLoad> &load) {
-    constexpr double kAlone = 0.43;  // waves up to which every CTA finds an SM for itself
-    if (load.size() == 1) {
+    if (load.size() == 1) {  // whole waves, and a last one
         const ResLoad &l = load[0];
-        if (l.waves <= 1.0) return wave_us(l.K, l.most, l.whole, l.waves <= kAlone);
+        if (l.waves <= 1.0) return l.waves <= kAlone ? l.alone1 : l.shared1;
         const double full = std::floor(l.waves + 1e-9), rest = l.waves - full;
-        return full * wave_us(l.K, l.links, l.whole, false) +
-               (rest < 1e-3 ? 0.0 : wave_us(l.K, l.links, l.whole, !l.whole && rest <= kAlone));
+        return full * l.shared + (rest < 1e-3 ? 0.0 : !l.whole && rest <= 0.5 ? l.alone : l.shared);
     }
     // several sizes fill each other's gaps
-    double waves = 0, sum = 0, alone = 0, shared = 0;
+    const double waves = total_waves(load);
+    double sum = 0, alone = 0, shared = 0;
     for (const ResLoad &l : load) {
-        waves += l.waves;
-        sum += l.waves * wave_us(l.K, l.links, l.whole, false);
-        alone = std::max(alone, wave_us(l.K, l.most, l.whole, true));
-        shared = std::max(shared, wave_us(l.K, l.most, l.whole, false));
+        sum += l.waves * l.shared;
+        alone = std::max(alone, l.alone1);
+        shared = std::max(shared, l.shared1);
     }
-    return waves <= kAlone ? alone : std::max(shared, 0.95 * sum + 0.6 * shared);
+    if (waves <= 1.0) return waves <= kAlone ? alone : shared;
+    return std::max(shared, 0.95 * sum + 0.55 * shared);
 }
 double passes_us(double nv, double nl, double nr) {  // latency, then the L2's rate, then that of HBM
-    const double u = nv + nl / 6;
-    return 4.9 + 0.18 * std::min(std::log2(nr), 6.0) + 4.5e-5 * std::min(u, 2.5e4) + 8.2e-5 * std::min(std::max(u - 2.5e4, 0.0), 2.1e5) +
-           1.44e-4 * std::max(u - 2.35e5, 0.0);
+    const double u = nv + 0.19 * nl, robots = std::min(std::log2(nr), 6.5);
+    return 5.2 + robots * (0.163 - 0.124 * std::min(u / 2.1e4, 1.0)) + 5.1e-5 * std::min(u, 2.1e4) +
+           7.6e-5 * std::min(std::max(u - 2.1e4, 0.0), 1.3e5) + 6.5e-5 * std::min(std::max(u - 1.51e5, 0.0), 8.4e4) +
+           1.37e-4 * std::max(u - 2.35e5, 0.0);
 }
 // The fewest steps of a call for which one launch is faster: it loads and stores the state (one robot of 8
 // voxels: 11.1 us for one step, 55 for 20, against 9.4 and 116 by the passes; 203 robots of 12^3 cells 127 us
 // for one step against 64, of 43 and 68 a step).  Passes launched one by one start every 5.6 us at best.
-// Over those batches and calls of 1 to 20 steps the way taken is 1% slower than the better one on average.
+// Over those batches and calls of 1 to 20 steps the way taken is 0.6% slower than the better one on average.
 int resident_from(double many, double passes, double nv, bool several) {
-    const double once = 5.7 + 1.344 * many + 2.977e-5 * nv + (several ? 4.9 : 0.0) - 6.0;
+    const double once = 5.7 + 1.344 * many + 2.977e-5 * nv + (several ? 4.9 : 0.0) - 6.5;
     return std::max(1, (int)std::ceil(once / std::max(std::max(passes, 5.6) - many, 0.05)));
 }
 
@@ -517,14 +523,19 @@ int plan_resident(vx3g_ctx *c, bool any) {
         int act = 0;
         CU(steps_mixed_active(K, threads(p), p.smem, &act));
         if (act < 1) return VX3G_OK;
-        double lc = 0, most = 0;
-        for (const Bundle &x : p.b) lc += x.b.lc, most = std::max<double>(most, x.b.lc);
-        load.push_back(ResLoad{K, (double)p.b.size() / act, lc / p.b.size(), most, p.smem > kHalf});
+        ResLoad l{(double)p.b.size() / act, p.smem > kHalf, 0, 0, 0, 0};
+        for (const Bundle &x : p.b) {
+            const double al = bundle_us(K, x.b.lc, l.whole, true), sh = bundle_us(K, x.b.lc, l.whole, false);
+            l.alone += al / p.b.size(), l.alone1 = std::max(l.alone1, al);
+            l.shared += sh / p.b.size(), l.shared1 = std::max(l.shared1, sh);
+        }
+        load.push_back(l);
     }
     if (load.empty()) return VX3G_OK;
     const bool several = load.size() > 1;
     const double many = resident_us(load), passes = passes_us(d.nv, d.nl, c->nr);
-    if (!any && many > (several ? 0.8 : 0.95) * passes) return VX3G_OK;
+    // (an estimate of several sizes in more than a few SMs errs most)
+    if (!any && many > (several && total_waves(load) > kAlone ? 1.0 : 1.03) * passes) return VX3G_OK;
     c->res_from = resident_from(many, passes, d.nv, several);
     // all tables in one allocation and one copy: per size its bundles, then (entries, links) of each CTA
     std::vector<int2> &tab = c->res_tables;
