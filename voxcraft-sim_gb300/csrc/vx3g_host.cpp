@@ -426,11 +426,12 @@ double passes_us(double nv, double nl, double nr) {  // latency, then the L2's r
 }
 // The fewest steps of a call for which one launch is faster: it loads and stores the state (one robot of 8
 // voxels: 11.1 us for one step, 55 for 20, against 9.4 and 116 by the passes; 203 robots of 12^3 cells 127 us
-// for one step against 64, of 43 and 68 a step).  Passes launched one by one start every 5.6 us at best.
-// Over those batches and calls of 1 to 20 steps the way taken is 0.6% slower than the better one on average.
+// for one step against 64, of 43 and 68 a step).  Passes launched one by one take 0.6 us a step more than in a
+// graph.  Over those batches and calls of 1 to 20 steps the way taken is 0.5% slower than the better one on
+// average.
 int resident_from(double many, double passes, double nv, bool several) {
-    const double once = 5.7 + 1.344 * many + 2.977e-5 * nv + (several ? 4.9 : 0.0) - 6.5;
-    return std::max(1, (int)std::ceil(once / std::max(std::max(passes, 5.6) - many, 0.05)));
+    const double once = 0.7 + 1.344 * many + 2.977e-5 * nv + (several ? 4.9 : 0.0);
+    return std::max(1, (int)std::ceil(once / std::max(passes + 0.6 - many, 0.05)));
 }
 
 // Whether and how k_steps_mixed steps the batch: mixed precision, whole robots in shared memory.
